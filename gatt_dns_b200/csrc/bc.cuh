@@ -6,27 +6,34 @@
 // The reference applies its lists strictly in order (Dirichlet U,V,W,E,P; Neumann
 // U,V,W,E,P; corners; null second derivative U,V,W,E,P; disturbances), and later
 // items read values earlier ones wrote.  The host flattens those lists into one
-// program of box operations (BcOp) in that order.  A cluster of CTAs (up to 16 SMs) per batch
-// member executes the program, the points of each op spread over all its threads, with the
-// cluster barrier (release/acquire at cluster scope: every write is visible after it) between
-// dependent ops; where a cluster cannot be launched, one CTA per member with block barriers.
-// Consecutive ops whose boxes and fields do not conflict form one phase without a barrier
-// (the host sets BcOp::sync on the last op of each phase).  Boxes are boundary planes, so the whole program touches a small fraction of
-// the field, but on one SM it cost half of a boundary-layer step.
+// program of box operations (BcOp) in that order and sorts them into levels: an op's level is
+// one more than the highest level of the earlier ops it conflicts with (it reads or writes a
+// field point that they write, or writes one that they read), so the ops of one level are
+// independent whatever their order, and every op finds the values that the reference's order
+// gives it.  The points of a level's ops form one index range spread over all threads; a
+// barrier separates the levels.  One CTA per batch member runs small programs (block barriers),
+// a cluster of up to 16 SMs the larger ones (cluster barriers, release/acquire).
+//
+// What bounds it: the chain of levels, about a microsecond each (a barrier, then dependent
+// loads that miss to L2).  The pressure Neumann items and the corners are therefore one op
+// each (P = R E formed on the fly, not through a scratch field): the 128^2 lid-driven cavity
+// has 3 levels instead of 15 phases of consecutive ops, the 800x300 boundary layer over a
+// cavity 9 instead of 27.
 #pragma once
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include "pointwise.cuh"
+#include "sweep.cuh"
 
 namespace gatt {
 
 enum BcOpCode {
     OP_SET = 0,        // F[var](box) = val
     OP_DIR_P = 1,      // R(box) = val/(gamma-1)/E(box)
-    OP_NEU = 2,        // applyNeumann on F[var] over the extended box (face = first plane)
-    OP_P_LOAD = 3,     // P(box) = R*E (box = extended box)
-    OP_P_NEU = 4,      // applyNeumann on P over the extended box
+    OP_NEU = 2,        // applyNeumann on F[var]: the face `box` from the next len nodes along step
+    OP_P_LOAD = 3,     // P(box) = R*E
+    OP_P_NEU = 4,      // applyNeumann on P
     OP_R_FROM_P = 5,   // R(box) = P/E
     OP_CORNER_E0 = 6,  // E(box) = 0
     OP_P_FROM_E = 7,   // P(box) = E
@@ -37,29 +44,38 @@ enum BcOpCode {
     OP_R_DIV_E = 12,   // R(box) = R/E/aux
     OP_LID = 13,       // lidDrivenMovement on F[var](box), x coordinates at xoff, U0 = val
     OP_SINE = 14,      // periodicSine: F[var](box) += xs[xoff + i - i1] * sin(val * t)
-    OP_HOLD = 15       // holdInlet: aux fields (U, V, W, E, then R) of the box <-> hold + xoff
+    OP_HOLD = 15,      // holdInlet: aux fields (U, V, W, E, then R) of the box <-> hold + xoff
+    // 3..5 and 6..12 in one op, without the scratch field (boxes one node thick along their
+    // directions; the scratch form serves the others, and the adjoint)
+    OP_PNEU = 16,      // R(face) = applyNeumann(R*E)/E
+    OP_CORNER = 17     // adiabatic (var = 1): E = sum of its extrapolations / aux;
+                       // R = sum of the extrapolations of R*E / E / aux; directions step[0..aux)
 };
 
 struct BcOp {
     int code;
     int var;        // 0..4 (U,V,W,R,E)
-    int box[6];     // 1-based inclusive i1 i2 j1 j2 k1 k2
-    int dir;        // 1..6 for Neumann
+    int box[6];     // 1-based inclusive i1 i2 j1 j2 k1 k2 of the points the op runs over
     int len;        // extrapolation length
     int coef;       // 0 = neumannCoeffs, 1 = neumann2Coeffs
     int aux;        // divisor for corner averages
     int xoff;       // offset of the box's x coordinates (OP_LID), of its x factors (OP_SINE), of
                     // its values in the member's hold buffer (OP_HOLD)
-    int sync;       // barrier after this op (the next op depends on this op's phase)
+    unsigned first, count;  // its points in its level's index range
+    FastDiv fd_ni, fd_nij;  // dividers by the box's x extent and x-y extent
+    long long step[3];      // element strides of the extrapolation directions, signed
     double val;
     long long tape; // adjoint tape: offset of this op's recorded base values (-1: none)
 };
 
 static_assert(sizeof(BcOp) % sizeof(long long) == 0, "ops are staged as 8-byte words");
 
+// Levels of a program: ops lev_op[l] .. lev_op[l+1] make level l, lev_pts[l] points in all
+// (lev holds lev_op[0 .. nlev], then lev_pts[0 .. nlev-1]).
 struct BcProgram {
     const BcOp *ops;
-    int nops;
+    const unsigned *lev;
+    int nops, nlev;
     const double *coef1;  // neumannCoeffs
     const double *coef2;  // neumann2Coeffs
     const double *xs;     // disturbance coordinates (OP_LID) and x factors (OP_SINE)
@@ -86,136 +102,146 @@ __device__ __forceinline__ double bc_sine(double u, double fx, double omega, dou
     return __dadd_rn(u, __dmul_rn(fx, sin(omega * t)));
 }
 
+// lidDrivenMovement.F90:15-17 at x node i of an op's box
+__device__ __forceinline__ double bc_lid(const BcProgram &pg, const BcOp &op, int i)
+{
+    const double *x = pg.xs + op.xoff;
+    const double s = 2 * (x[i - op.box[0]] - x[0]) / (x[op.box[1] - op.box[0]] - x[0]) - 1;
+    const double s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s16 = s8 * s8;
+    const double pp = 1 - s16 * s2;
+    return op.val * (pp * pp);
+}
+
 // holdInlet.F90 keeps u, v, w, e (and r with holdDensity): field of the v-th held value
 __device__ __forceinline__ int bc_hold_field(int v) { return v < 3 ? v : (v == 3 ? 4 : 3); }
 
-__device__ __forceinline__ long long bidx(const BcProgram &pg, int i, int j, int k)
+// applyNeumann (nseq.F90:552-599) at one face point: u points to it, st steps into the domain;
+// products and sums rounded one by one as the reference does (no fused multiply-add: chains of
+// boundary items, with divisions by extrapolated E between them, amplify the difference)
+__device__ __forceinline__ double bc_extrapolate(const double *u, long long st, int len, const double *c)
 {
-    return (long long)(i - 1) + (long long)pg.nx * ((long long)(j - 1) + (long long)pg.ny * (k - 1));
+    double v = __dmul_rn(c[0], u[st]);
+    for (int m = 2; m <= len; m++) v = __dadd_rn(v, __dmul_rn(c[m - 1], u[m * st]));
+    return v;
+}
+// the same of P = R*E
+__device__ __forceinline__ double bc_extrapolate_p(const double *r, const double *e, long long st, int len,
+                                                   const double *c)
+{
+    double v = __dmul_rn(c[0], __dmul_rn(r[st], e[st]));
+    for (int m = 2; m <= len; m++) v = __dadd_rn(v, __dmul_rn(c[m - 1], __dmul_rn(r[m * st], e[m * st])));
+    return v;
 }
 
-// Extrapolate the face of box b along dir from the next len nodes (applyNeumann,
-// nseq.F90:552-599).  Thread tid of nthr strides over the face points.
-__device__ void neumann_face(const BcProgram &pg, double *u, const int *b, int dir, int len, const double *c,
-                             int tid, int nthr)
+// Largest program whose ops and levels are staged in shared memory (48 KB, no opt-in needed);
+// longer programs read them from global memory.
+constexpr int kBcStagedBytes = 48 * 1024;
+__host__ __device__ __forceinline__ size_t bc_stage_bytes(int nops, int nlev)
 {
-    int n1, n2;  // the two extents that span the face
-    int a0, a1, c0, c1;
-    if (dir <= 2) { a0 = b[2]; a1 = b[3]; c0 = b[4]; c1 = b[5]; }
-    else if (dir <= 4) { a0 = b[0]; a1 = b[1]; c0 = b[4]; c1 = b[5]; }
-    else { a0 = b[0]; a1 = b[1]; c0 = b[2]; c1 = b[3]; }
-    n1 = a1 - a0 + 1; n2 = c1 - c0 + 1;
-    const long long total = (long long)n1 * n2;
-    for (long long q = tid; q < total; q += nthr) {
-        const int a = a0 + (int)(q % n1), cc = c0 + (int)(q / n1);
-        int i, j, k, di = 0, dj = 0, dk = 0;
-        const bool lo = (dir & 1);               // odd dirs extrapolate at the low end
-        const int s = lo ? 1 : -1;
-        int face;
-        if (dir <= 2) { face = lo ? b[0] : b[0] + len; di = s; j = a; k = cc; i = face; }
-        else if (dir <= 4) { face = lo ? b[2] : b[2] + len; dj = s; i = a; k = cc; j = face; }
-        else { face = lo ? b[4] : b[4] + len; dk = s; i = a; j = cc; k = face; }
-        double v = c[0] * u[bidx(pg, i + di, j + dj, k + dk)];
-        for (int m = 2; m <= len; m++) v = v + c[m - 1] * u[bidx(pg, i + m * di, j + m * dj, k + m * dk)];
-        u[bidx(pg, i, j, k)] = v;
+    return (size_t)nops * sizeof(BcOp) + ((size_t)(2 * nlev + 1) * sizeof(unsigned) + 7) / 8 * 8;
+}
+
+// Copy ops and levels to shared memory (when they fit) and point pg there; every thread of the
+// CTA calls it.  The host pads the level table to whole 8-byte words.
+__device__ __forceinline__ void bc_stage(BcProgram &pg, long long *sh)
+{
+    if (bc_stage_bytes(pg.nops, pg.nlev) > (size_t)kBcStagedBytes) return;
+    const int n = pg.nops * (int)(sizeof(BcOp) / sizeof(long long)), m = (2 * pg.nlev + 2) / 2;
+    const long long *g = reinterpret_cast<const long long *>(pg.ops), *gl = reinterpret_cast<const long long *>(pg.lev);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) sh[i] = g[i];
+    for (int i = threadIdx.x; i < m; i += blockDim.x) sh[n + i] = gl[i];
+    __syncthreads();
+    pg.ops = reinterpret_cast<const BcOp *>(sh);
+    pg.lev = reinterpret_cast<const unsigned *>(sh + n);
+}
+
+// fn(op, r, i, p) for every point of every level, thread tid of nthr: r the point's index in
+// the op's box (x fastest), i its x node, p its element offset; sync() (a barrier over all nthr
+// threads that orders their memory accesses) between levels.  REV: last level first.
+template <bool REV = false, typename Sync, typename Fn>
+__device__ __forceinline__ void bc_levels(const BcProgram &pg, int tid, int nthr, Sync sync, Fn fn)
+{
+    for (int l = 0; l < pg.nlev; l++) {
+        if (l) sync();
+        const int lv = REV ? pg.nlev - 1 - l : l;
+        const unsigned total = pg.lev[pg.nlev + 1 + lv];
+        const BcOp *op = pg.ops + pg.lev[lv];
+        for (unsigned q = tid; q < total; q += nthr) {
+            while (q >= op->first + op->count) op++;
+            const unsigned r = q - op->first;
+            const unsigned kq = fdiv((int)r, op->fd_nij), rr = r - kq * op->fd_nij.d, jq = fdiv((int)rr, op->fd_ni);
+            const int i = op->box[0] + (int)(rr - jq * op->fd_ni.d);
+            const long long p = (long long)(i - 1) +
+                                (long long)pg.nx * ((op->box[2] - 1 + (int)jq) + (long long)pg.ny * (op->box[4] - 1 + (int)kq));
+            fn(*op, r, i, p);
+        }
     }
 }
 
-// Largest program whose ops are staged in shared memory (48 KB, no opt-in needed); longer
-// programs read their ops from global memory.
-constexpr int kBcStagedOps = 48 * 1024 / (int)sizeof(BcOp);
-
-// The program on one member: F the five state arrays (U,V,W,R,E), P a scratch field, thread
-// tid of nthr; sync() is a barrier over all nthr threads that orders their memory accesses.
-// sops: the ops copied to this CTA's shared memory (nullptr: read them from pg.ops).
+// The program on one member: F the five state arrays (U,V,W,R,E), P a scratch field.
 template <typename Sync>
-__device__ __forceinline__ void bc_run(const BcProgram &pg, const BcOp *sops, double *const *F, double *P, double *H,
-                                       int tid, int nthr, Sync sync)
+__device__ __forceinline__ void bc_run(const BcProgram &pg, double *const *F, double *P, double *H, int tid, int nthr,
+                                       Sync sync)
 {
     double *Rr = F[3], *Ee = F[4];
-    const BcOp *ops = sops ? sops : pg.ops;
     const double tnow = bc_time(pg);
-    for (int o = 0; o < pg.nops; o++) {
-        const BcOp op = ops[o];
-        if (op.code == OP_NEU || op.code == OP_P_NEU) {
-            double *u = (op.code == OP_NEU) ? F[op.var] : P;
-            neumann_face(pg, u, op.box, op.dir, op.len, op.coef ? pg.coef2 : pg.coef1, tid, nthr);
-            if (op.sync) sync();
-            continue;
-        }
-        // 32-bit index arithmetic: a box holds fewer than 2^31 points (the grid does)
-        const unsigned ni = op.box[1] - op.box[0] + 1, nj = op.box[3] - op.box[2] + 1, nk = op.box[5] - op.box[4] + 1;
-        const unsigned nij = ni * nj, total = nij * nk;
-        for (unsigned q2 = tid; q2 < total; q2 += nthr) {
-            const unsigned kq = q2 / nij, r = q2 - kq * nij, jq = r / ni;
-            const int i = op.box[0] + (int)(r - jq * ni);
-            const int j = op.box[2] + (int)jq;
-            const int k = op.box[4] + (int)kq;
-            const long long p = bidx(pg, i, j, k);
-            switch (op.code) {
-            case OP_SET: F[op.var][p] = op.val; break;
-            case OP_DIR_P: Rr[p] = op.val / (pg.gamma - 1.0) / Ee[p]; break;
-            case OP_P_LOAD: P[p] = Rr[p] * Ee[p]; break;
-            case OP_R_FROM_P: Rr[p] = P[p] / Ee[p]; break;
-            case OP_CORNER_E0: Ee[p] = 0.0; break;
-            case OP_P_FROM_E: P[p] = Ee[p]; break;
-            case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; break;
-            case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; break;
-            case OP_R0: Rr[p] = 0.0; break;
-            case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; break;
-            case OP_R_DIV_E: Rr[p] = Rr[p] / Ee[p] / (double)op.aux; break;
-            case OP_LID: {
-                // lidDrivenMovement.F90:15-17
-                const double *x = pg.xs + op.xoff;
-                const double s = 2 * (x[i - op.box[0]] - x[0]) / (x[ni - 1] - x[0]) - 1;
-                const double s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s16 = s8 * s8;
-                const double pp = 1 - s16 * s2;
-                F[op.var][p] = op.val * (pp * pp);
-                break;
+    bc_levels(pg, tid, nthr, sync, [&](const BcOp &op, unsigned r, int i, long long p) {
+        const double *cf = op.coef ? pg.coef2 : pg.coef1;
+        switch (op.code) {
+        case OP_SET: F[op.var][p] = op.val; break;
+        case OP_DIR_P: Rr[p] = op.val / (pg.gamma - 1.0) / Ee[p]; break;
+        case OP_NEU: F[op.var][p] = bc_extrapolate(F[op.var] + p, op.step[0], op.len, cf); break;
+        case OP_PNEU: Rr[p] = bc_extrapolate_p(Rr + p, Ee + p, op.step[0], op.len, cf) / Ee[p]; break;
+        case OP_CORNER: {
+            if (op.var) {
+                double e = 0.0;
+                for (int d = 0; d < op.aux; d++) e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
+                Ee[p] = e / (double)op.aux;
             }
-            case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
-            case OP_HOLD:
-                for (int v = 0; v < op.aux; v++) {
-                    double *h = H + op.xoff + (long long)v * total + q2;
-                    if (pg.hold_save) *h = F[bc_hold_field(v)][p];
-                    else F[bc_hold_field(v)][p] = *h;
-                }
-                break;
-            default: break;
-            }
+            double v = 0.0;
+            for (int d = 0; d < op.aux; d++) v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
+            Rr[p] = v / Ee[p] / (double)op.aux;
+            break;
         }
-        // the next op reads or writes what this phase wrote (or writes what it read)
-        if (op.sync) sync();
-    }
+        case OP_P_LOAD: P[p] = Rr[p] * Ee[p]; break;
+        case OP_P_NEU: P[p] = bc_extrapolate(P + p, op.step[0], op.len, cf); break;
+        case OP_R_FROM_P: Rr[p] = P[p] / Ee[p]; break;
+        case OP_CORNER_E0: Ee[p] = 0.0; break;
+        case OP_P_FROM_E: P[p] = Ee[p]; break;
+        case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; break;
+        case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; break;
+        case OP_R0: Rr[p] = 0.0; break;
+        case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; break;
+        case OP_R_DIV_E: Rr[p] = Rr[p] / Ee[p] / (double)op.aux; break;
+        case OP_LID: F[op.var][p] = bc_lid(pg, op, i); break;
+        case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
+        case OP_HOLD:
+            for (int v = 0; v < op.aux; v++) {
+                double *h = H + op.xoff + (long long)v * op.count + r;
+                if (pg.hold_save) *h = F[bc_hold_field(v)][p];
+                else F[bc_hold_field(v)][p] = *h;
+            }
+            break;
+        default: break;
+        }
+    });
 }
 
-// Copy the ops to shared memory (when they fit); every thread of the CTA calls it.
-__device__ __forceinline__ const BcOp *bc_stage_ops(const BcProgram &pg, BcOp *sops)
+// One CTA per batch member (block barriers); dynamic shared memory: the staged program.
+__global__ void __launch_bounds__(512) k_bc(BcProgram pg, StateSet q, double *Pbase, long long pstride)
 {
-    if (pg.nops > kBcStagedOps) return nullptr;
-    const int n = pg.nops * (int)(sizeof(BcOp) / sizeof(long long));
-    const long long *g = reinterpret_cast<const long long *>(pg.ops);
-    long long *d = reinterpret_cast<long long *>(sops);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = g[i];
-    __syncthreads();
-    return sops;
-}
-
-// One CTA per batch member (block barriers); dynamic shared memory: the staged ops.
-__global__ void k_bc(BcProgram pg, StateSet q, double *Pbase, long long pstride)
-{
-    extern __shared__ BcOp bc_sops[];
+    extern __shared__ long long bc_sh[];
     const int b = blockIdx.x;
     double *F[5];
 #pragma unroll
     for (int f = 0; f < 5; f++) F[f] = q.v[f] + b * q.bstride;
-    const BcOp *sops = bc_stage_ops(pg, bc_sops);
+    bc_stage(pg, bc_sh);
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
-    bc_run(pg, sops, F, Pbase + b * pstride, H, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+    bc_run(pg, F, Pbase + b * pstride, H, threadIdx.x, blockDim.x, [] { __syncthreads(); });
 }
 
 // One cluster of CTAs per batch member (cluster barriers); launched with a cluster dimension.
-__global__ void k_bc_cluster(BcProgram pg, StateSet q, double *Pbase, long long pstride)
+__global__ void __launch_bounds__(512) k_bc_cluster(BcProgram pg, StateSet q, double *Pbase, long long pstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -223,12 +249,11 @@ __global__ void k_bc_cluster(BcProgram pg, StateSet q, double *Pbase, long long 
     double *F[5];
 #pragma unroll
     for (int f = 0; f < 5; f++) F[f] = q.v[f] + b * q.bstride;
-    extern __shared__ BcOp bc_sops[];
-    const int nthr = (int)cl.num_threads();
-    const int tid = (int)cl.block_rank() * blockDim.x + threadIdx.x;
-    const BcOp *sops = bc_stage_ops(pg, bc_sops);
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
-    bc_run(pg, sops, F, Pbase + b * pstride, H, tid, nthr, [&] { cl.sync(); });
+    bc_run(pg, F, Pbase + b * pstride, H, (int)cl.block_rank() * blockDim.x + threadIdx.x, (int)cl.num_threads(),
+           [&] { cl.sync(); });
 }
 
 // ---- tangent-linear and adjoint of the program (no counterpart in the reference) -------
@@ -245,35 +270,11 @@ __host__ __device__ __forceinline__ int bc_tape_width(int code)
     return code == OP_DIR_P ? 1 : (code == OP_P_LOAD || code == OP_R_FROM_P || code == OP_R_DIV_E) ? 2 : 0;
 }
 
-// Face point q of a Neumann op: the face node and the unit step into the domain.
-__device__ __forceinline__ void neumann_geom(const int *b, int dir, int len, long long q, int n1, int &i, int &j,
-                                             int &k, int &di, int &dj, int &dk)
-{
-    int a0, c0;
-    if (dir <= 2) { a0 = b[2]; c0 = b[4]; }
-    else if (dir <= 4) { a0 = b[0]; c0 = b[4]; }
-    else { a0 = b[0]; c0 = b[2]; }
-    const int a = a0 + (int)(q % n1), cc = c0 + (int)(q / n1);
-    const bool lo = (dir & 1);
-    const int s = lo ? 1 : -1;
-    di = dj = dk = 0;
-    if (dir <= 2) { i = lo ? b[0] : b[0] + len; di = s; j = a; k = cc; }
-    else if (dir <= 4) { j = lo ? b[2] : b[2] + len; dj = s; i = a; k = cc; }
-    else { k = lo ? b[4] : b[4] + len; dk = s; i = a; j = cc; }
-}
-
-__device__ __forceinline__ void neumann_extent(const int *b, int dir, int &n1, int &n2)
-{
-    if (dir <= 2) { n1 = b[3] - b[2] + 1; n2 = b[5] - b[4] + 1; }
-    else if (dir <= 4) { n1 = b[1] - b[0] + 1; n2 = b[5] - b[4] + 1; }
-    else { n1 = b[1] - b[0] + 1; n2 = b[3] - b[2] + 1; }
-}
-
-// the forward program on the base, recording the tape (same arithmetic as k_bc)
+// The forward program (scratch form) on the base, recording the tape: member b, thread tid of
+// nthr, sync() a barrier over the nthr threads.
 template <typename Sync>
-// member b, thread tid of nthr, sync(): a barrier over the nthr threads
-__device__ __forceinline__ void k_bc_rec_run(int b, int tid, int nthr, Sync sync,
-    BcProgram pg, StateSet q, double *Pbase, long long pstride, double *tape, long long tstride)
+__device__ __forceinline__ void k_bc_rec_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, StateSet q,
+                                             double *Pbase, long long pstride, double *tape, long long tstride)
 {
     double *F[5];
 #pragma unroll
@@ -283,74 +284,66 @@ __device__ __forceinline__ void k_bc_rec_run(int b, int tid, int nthr, Sync sync
     double *tp = tape + b * tstride;
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
     const double tnow = bc_time(pg);
-    for (int o = 0; o < pg.nops; o++) {
-        const BcOp op = pg.ops[o];
-        if (op.code == OP_NEU || op.code == OP_P_NEU) {
-            double *u = (op.code == OP_NEU) ? F[op.var] : P;
-            neumann_face(pg, u, op.box, op.dir, op.len, op.coef ? pg.coef2 : pg.coef1, tid, nthr);
-            sync();
-            continue;
+    bc_levels(pg, tid, nthr, sync, [&](const BcOp &op, unsigned r, int i, long long p) {
+        const double *cf = op.coef ? pg.coef2 : pg.coef1;
+        double *t = tp + op.tape + (long long)bc_tape_width(op.code) * r;
+        switch (op.code) {
+        case OP_SET: F[op.var][p] = op.val; break;
+        case OP_DIR_P: t[0] = Ee[p]; Rr[p] = op.val / (pg.gamma - 1.0) / Ee[p]; break;
+        case OP_NEU: F[op.var][p] = bc_extrapolate(F[op.var] + p, op.step[0], op.len, cf); break;
+        case OP_P_LOAD: t[0] = Rr[p]; t[1] = Ee[p]; P[p] = Rr[p] * Ee[p]; break;
+        case OP_P_NEU: P[p] = bc_extrapolate(P + p, op.step[0], op.len, cf); break;
+        case OP_R_FROM_P: t[0] = P[p]; t[1] = Ee[p]; Rr[p] = P[p] / Ee[p]; break;
+        case OP_CORNER_E0: Ee[p] = 0.0; break;
+        case OP_P_FROM_E: P[p] = Ee[p]; break;
+        case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; break;
+        case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; break;
+        case OP_R0: Rr[p] = 0.0; break;
+        case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; break;
+        case OP_R_DIV_E: t[0] = Rr[p]; t[1] = Ee[p]; Rr[p] = Rr[p] / Ee[p] / (double)op.aux; break;
+        case OP_LID: F[op.var][p] = bc_lid(pg, op, i); break;
+        case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
+        case OP_HOLD:  // the fields put back (the tangent and adjoint never run a first call)
+            for (int v = 0; v < op.aux; v++) F[bc_hold_field(v)][p] = H[op.xoff + (long long)v * op.count + r];
+            break;
+        default: break;
         }
-        const int ni = op.box[1] - op.box[0] + 1, nj = op.box[3] - op.box[2] + 1, nk = op.box[5] - op.box[4] + 1;
-        const long long total = (long long)ni * nj * nk;
-        const int tw = bc_tape_width(op.code);
-        for (long long q2 = tid; q2 < total; q2 += nthr) {
-            const int i = op.box[0] + (int)(q2 % ni);
-            const int j = op.box[2] + (int)((q2 / ni) % nj);
-            const int k = op.box[4] + (int)(q2 / ((long long)ni * nj));
-            const long long p = bidx(pg, i, j, k);
-            double *t = tp + op.tape + tw * q2;
-            switch (op.code) {
-            case OP_SET: F[op.var][p] = op.val; break;
-            case OP_DIR_P: t[0] = Ee[p]; Rr[p] = op.val / (pg.gamma - 1.0) / Ee[p]; break;
-            case OP_P_LOAD: t[0] = Rr[p]; t[1] = Ee[p]; P[p] = Rr[p] * Ee[p]; break;
-            case OP_R_FROM_P: t[0] = P[p]; t[1] = Ee[p]; Rr[p] = P[p] / Ee[p]; break;
-            case OP_CORNER_E0: Ee[p] = 0.0; break;
-            case OP_P_FROM_E: P[p] = Ee[p]; break;
-            case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; break;
-            case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; break;
-            case OP_R0: Rr[p] = 0.0; break;
-            case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; break;
-            case OP_R_DIV_E: t[0] = Rr[p]; t[1] = Ee[p]; Rr[p] = Rr[p] / Ee[p] / (double)op.aux; break;
-            case OP_LID: {
-                const double *x = pg.xs + op.xoff;
-                const double sx = 2 * (x[i - op.box[0]] - x[0]) / (x[ni - 1] - x[0]) - 1;
-                const double s2 = sx * sx, s4 = s2 * s2, s8 = s4 * s4, s16 = s8 * s8;
-                const double pp = 1 - s16 * s2;
-                F[op.var][p] = op.val * (pp * pp);
-                break;
-            }
-            case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
-            case OP_HOLD:  // the fields put back (the tangent and adjoint never run a first call)
-                for (int v = 0; v < op.aux; v++) F[bc_hold_field(v)][p] = H[op.xoff + (long long)v * total + q2];
-                break;
-            default: break;
-            }
-        }
-        sync();
-    }
+    });
 }
 
-__global__ void k_bc_rec(
-    BcProgram pg, StateSet q, double *Pbase, long long pstride, double *tape, long long tstride)
+__global__ void __launch_bounds__(512) k_bc_rec(BcProgram pg, StateSet q, double *Pbase, long long pstride, double *tape,
+                                                long long tstride)
 {
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
     k_bc_rec_run(blockIdx.x, threadIdx.x, blockDim.x, [] { __syncthreads(); }, pg, q, Pbase, pstride, tape, tstride);
 }
 
-__global__ void k_bc_rec_cluster(
-    BcProgram pg, StateSet q, double *Pbase, long long pstride, double *tape, long long tstride)
+__global__ void __launch_bounds__(512) k_bc_rec_cluster(BcProgram pg, StateSet q, double *Pbase, long long pstride,
+                                                        double *tape, long long tstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-    k_bc_rec_run(blockIdx.x / (int)cl.num_blocks(), (int)cl.block_rank() * blockDim.x + threadIdx.x, (int)cl.num_threads(),
-           [&] { cl.sync(); }, pg, q, Pbase, pstride, tape, tstride);
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
+    k_bc_rec_run(blockIdx.x / (int)cl.num_blocks(), (int)cl.block_rank() * blockDim.x + threadIdx.x,
+                 (int)cl.num_threads(), [&] { cl.sync(); }, pg, q, Pbase, pstride, tape, tstride);
 }
 
-// tangent: base q (updated as k_bc does) and tangent dq (P, dP scratch)
+// tangent of bc_extrapolate_p's sum
+__device__ __forceinline__ double bc_extrapolate_dp(const double *r, const double *e, const double *dr, const double *de,
+                                                    long long st, int len, const double *c)
+{
+    double v = 0.0;
+    for (int m = 1; m <= len; m++) v = v + c[m - 1] * (dr[m * st] * e[m * st] + r[m * st] * de[m * st]);
+    return v;
+}
+
+// tangent: base q (updated as k_bc does) and tangent dq (P, dP scratch); member b, thread tid
+// of nthr, sync() a barrier over the nthr threads
 template <typename Sync>
-// member b, thread tid of nthr, sync(): a barrier over the nthr threads
-__device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync,
-    BcProgram pg, StateSet q, double *Pbase, StateSet dq, double *dPbase, long long pstride)
+__device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, StateSet q,
+                                            double *Pbase, StateSet dq, double *dPbase, long long pstride)
 {
     double *F[5], *dF[5];
 #pragma unroll
@@ -359,110 +352,118 @@ __device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync,
     double *Rr = F[3], *Ee = F[4], *dR = dF[3], *dE = dF[4];
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
     const double tnow = bc_time(pg);
-    for (int o = 0; o < pg.nops; o++) {
-        const BcOp op = pg.ops[o];
-        if (op.code == OP_NEU || op.code == OP_P_NEU) {
-            const double *cf = op.coef ? pg.coef2 : pg.coef1;
-            neumann_face(pg, op.code == OP_NEU ? F[op.var] : P, op.box, op.dir, op.len, cf, tid, nthr);
-            neumann_face(pg, op.code == OP_NEU ? dF[op.var] : dP, op.box, op.dir, op.len, cf, tid, nthr);
-            sync();
-            continue;
+    bc_levels(pg, tid, nthr, sync, [&](const BcOp &op, unsigned r, int i, long long p) {
+        const double *cf = op.coef ? pg.coef2 : pg.coef1;
+        switch (op.code) {
+        case OP_SET: F[op.var][p] = op.val; dF[op.var][p] = 0.0; break;
+        case OP_DIR_P: {
+            const double e = Ee[p], rn = op.val / (pg.gamma - 1.0) / e;
+            dR[p] = -rn / e * dE[p];
+            Rr[p] = rn;
+            break;
         }
-        const int ni = op.box[1] - op.box[0] + 1, nj = op.box[3] - op.box[2] + 1, nk = op.box[5] - op.box[4] + 1;
-        const long long total = (long long)ni * nj * nk;
-        for (long long q2 = tid; q2 < total; q2 += nthr) {
-            const int i = op.box[0] + (int)(q2 % ni);
-            const int j = op.box[2] + (int)((q2 / ni) % nj);
-            const int k = op.box[4] + (int)(q2 / ((long long)ni * nj));
-            const long long p = bidx(pg, i, j, k);
-            switch (op.code) {
-            case OP_SET: F[op.var][p] = op.val; dF[op.var][p] = 0.0; break;
-            case OP_DIR_P: {
-                const double e = Ee[p], rn = op.val / (pg.gamma - 1.0) / e;
-                dR[p] = -rn / e * dE[p];
-                Rr[p] = rn;
-                break;
-            }
-            case OP_P_LOAD: dP[p] = dR[p] * Ee[p] + Rr[p] * dE[p]; P[p] = Rr[p] * Ee[p]; break;
-            case OP_R_FROM_P: {
-                const double e = Ee[p], pv = P[p];
-                dR[p] = dP[p] / e - pv * dE[p] / (e * e);
-                Rr[p] = pv / e;
-                break;
-            }
-            case OP_CORNER_E0: Ee[p] = 0.0; dE[p] = 0.0; break;
-            case OP_P_FROM_E: P[p] = Ee[p]; dP[p] = dE[p]; break;
-            case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; dE[p] = dE[p] + dP[p]; break;
-            case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; dE[p] = dE[p] / (double)op.aux; break;
-            case OP_R0: Rr[p] = 0.0; dR[p] = 0.0; break;
-            case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; dR[p] = dR[p] + dP[p]; break;
-            case OP_R_DIV_E: {
-                const double r = Rr[p], e = Ee[p], aux = (double)op.aux;
-                dR[p] = dR[p] / e / aux - r * dE[p] / (e * e) / aux;
-                Rr[p] = r / e / aux;
-                break;
-            }
-            case OP_LID: {
-                const double *x = pg.xs + op.xoff;
-                const double sx = 2 * (x[i - op.box[0]] - x[0]) / (x[ni - 1] - x[0]) - 1;
-                const double s2 = sx * sx, s4 = s2 * s2, s8 = s4 * s4, s16 = s8 * s8;
-                const double pp = 1 - s16 * s2;
-                F[op.var][p] = op.val * (pp * pp);
-                dF[op.var][p] = 0.0;
-                break;
-            }
-            // an additive forcing in time: the tangent passes through
-            case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
-            case OP_HOLD:  // held fields are constants
-                for (int v = 0; v < op.aux; v++) {
-                    F[bc_hold_field(v)][p] = H[op.xoff + (long long)v * total + q2];
-                    dF[bc_hold_field(v)][p] = 0.0;
+        case OP_NEU:
+            F[op.var][p] = bc_extrapolate(F[op.var] + p, op.step[0], op.len, cf);
+            dF[op.var][p] = bc_extrapolate(dF[op.var] + p, op.step[0], op.len, cf);
+            break;
+        case OP_PNEU: {
+            const double e = Ee[p], pv = bc_extrapolate_p(Rr + p, Ee + p, op.step[0], op.len, cf);
+            const double dp = bc_extrapolate_dp(Rr + p, Ee + p, dR + p, dE + p, op.step[0], op.len, cf);
+            dR[p] = dp / e - pv * dE[p] / (e * e);
+            Rr[p] = pv / e;
+            break;
+        }
+        case OP_CORNER: {
+            const double aux = (double)op.aux;
+            if (op.var) {
+                double e = 0.0, de = 0.0;
+                for (int d = 0; d < op.aux; d++) {
+                    e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
+                    de = de + bc_extrapolate(dE + p, op.step[d], op.len, cf);
                 }
-                break;
-            default: break;
+                Ee[p] = e / aux;
+                dE[p] = de / aux;
             }
+            double v = 0.0, dv = 0.0;
+            for (int d = 0; d < op.aux; d++) {
+                v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
+                dv = dv + bc_extrapolate_dp(Rr + p, Ee + p, dR + p, dE + p, op.step[d], op.len, cf);
+            }
+            const double e = Ee[p];
+            dR[p] = dv / e / aux - v * dE[p] / (e * e) / aux;
+            Rr[p] = v / e / aux;
+            break;
         }
-        sync();
-    }
+        case OP_P_LOAD: dP[p] = dR[p] * Ee[p] + Rr[p] * dE[p]; P[p] = Rr[p] * Ee[p]; break;
+        case OP_P_NEU:
+            P[p] = bc_extrapolate(P + p, op.step[0], op.len, cf);
+            dP[p] = bc_extrapolate(dP + p, op.step[0], op.len, cf);
+            break;
+        case OP_R_FROM_P: {
+            const double e = Ee[p], pv = P[p];
+            dR[p] = dP[p] / e - pv * dE[p] / (e * e);
+            Rr[p] = pv / e;
+            break;
+        }
+        case OP_CORNER_E0: Ee[p] = 0.0; dE[p] = 0.0; break;
+        case OP_P_FROM_E: P[p] = Ee[p]; dP[p] = dE[p]; break;
+        case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; dE[p] = dE[p] + dP[p]; break;
+        case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; dE[p] = dE[p] / (double)op.aux; break;
+        case OP_R0: Rr[p] = 0.0; dR[p] = 0.0; break;
+        case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; dR[p] = dR[p] + dP[p]; break;
+        case OP_R_DIV_E: {
+            const double rr = Rr[p], e = Ee[p], aux = (double)op.aux;
+            dR[p] = dR[p] / e / aux - rr * dE[p] / (e * e) / aux;
+            Rr[p] = rr / e / aux;
+            break;
+        }
+        case OP_LID: F[op.var][p] = bc_lid(pg, op, i); dF[op.var][p] = 0.0; break;
+        // an additive forcing in time: the tangent passes through
+        case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
+        case OP_HOLD:  // held fields are constants
+            for (int v = 0; v < op.aux; v++) {
+                F[bc_hold_field(v)][p] = H[op.xoff + (long long)v * op.count + r];
+                dF[bc_hold_field(v)][p] = 0.0;
+            }
+            break;
+        default: break;
+        }
+    });
 }
 
-__global__ void k_bc_tl(
-    BcProgram pg, StateSet q, double *Pbase, StateSet dq, double *dPbase, long long pstride)
+__global__ void __launch_bounds__(512) k_bc_tl(BcProgram pg, StateSet q, double *Pbase, StateSet dq, double *dPbase,
+                                               long long pstride)
 {
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
     k_bc_tl_run(blockIdx.x, threadIdx.x, blockDim.x, [] { __syncthreads(); }, pg, q, Pbase, dq, dPbase, pstride);
 }
 
-__global__ void k_bc_tl_cluster(
-    BcProgram pg, StateSet q, double *Pbase, StateSet dq, double *dPbase, long long pstride)
+__global__ void __launch_bounds__(512) k_bc_tl_cluster(BcProgram pg, StateSet q, double *Pbase, StateSet dq,
+                                                       double *dPbase, long long pstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
     k_bc_tl_run(blockIdx.x / (int)cl.num_blocks(), (int)cl.block_rank() * blockDim.x + threadIdx.x, (int)cl.num_threads(),
-           [&] { cl.sync(); }, pg, q, Pbase, dq, dPbase, pstride);
+                [&] { cl.sync(); }, pg, q, Pbase, dq, dPbase, pstride);
 }
 
-// adjoint of a Neumann face: g = lam[face]; lam[face] = 0; lam[face + m s] += c_{m-1} g
-__device__ void neumann_face_adj(const BcProgram &pg, double *lam, const int *b, int dir, int len, const double *c,
-                                 int tid, int nthr)
+// adjoint of bc_extrapolate at a face point: g = lam[face]; lam[face] = 0; lam[face + m s] += c_{m-1} g
+__device__ __forceinline__ void bc_extrapolate_adj(double *lam, long long st, int len, const double *c)
 {
-    int n1, n2;
-    neumann_extent(b, dir, n1, n2);
-    const long long total = (long long)n1 * n2;
-    for (long long q = tid; q < total; q += nthr) {
-        int i, j, k, di, dj, dk;
-        neumann_geom(b, dir, len, q, n1, i, j, k, di, dj, dk);
-        const long long pf = bidx(pg, i, j, k);
-        const double g = lam[pf];
-        lam[pf] = 0.0;
-        for (int m = 1; m <= len; m++) lam[bidx(pg, i + m * di, j + m * dj, k + m * dk)] += c[m - 1] * g;
-    }
+    const double g = *lam;
+    *lam = 0.0;
+    for (int m = 1; m <= len; m++) lam[m * st] += c[m - 1] * g;
 }
 
-// adjoint: lam (the five variables) and lP (the scratch's lambda, zero on entry), ops in reverse
+// adjoint: lam (the five variables) and lP (the scratch's lambda, zero on entry), the scratch
+// form's levels in reverse.  Its levels also keep apart ops that only read the same point: their
+// adjoints both add to it.
 template <typename Sync>
-// member b, thread tid of nthr, sync(): a barrier over the nthr threads
-__device__ __forceinline__ void k_bc_adj_run(int b, int tid, int nthr, Sync sync,
-    BcProgram pg, StateSet lam, double *lPbase, long long pstride, const double *tape, long long tstride)
+__device__ __forceinline__ void k_bc_adj_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, StateSet lam,
+                                             double *lPbase, long long pstride, const double *tape, long long tstride)
 {
     double *L[5];
 #pragma unroll
@@ -470,76 +471,66 @@ __device__ __forceinline__ void k_bc_adj_run(int b, int tid, int nthr, Sync sync
     double *lP = lPbase + b * pstride;
     double *lR = L[3], *lE = L[4];
     const double *tp = tape + b * tstride;
-    for (int o = pg.nops - 1; o >= 0; o--) {
-        const BcOp op = pg.ops[o];
-        if (op.code == OP_NEU || op.code == OP_P_NEU) {
-            neumann_face_adj(pg, op.code == OP_NEU ? L[op.var] : lP, op.box, op.dir, op.len,
-                             op.coef ? pg.coef2 : pg.coef1, tid, nthr);
-            sync();
-            continue;
+    bc_levels<true>(pg, tid, nthr, sync, [&](const BcOp &op, unsigned r, int, long long p) {
+        const double *cf = op.coef ? pg.coef2 : pg.coef1;
+        const double *t = tp + op.tape + (long long)bc_tape_width(op.code) * r;
+        switch (op.code) {
+        case OP_SET: L[op.var][p] = 0.0; break;
+        case OP_DIR_P: {
+            const double e = t[0], rn = op.val / (pg.gamma - 1.0) / e;
+            lE[p] += -rn / e * lR[p];
+            lR[p] = 0.0;
+            break;
         }
-        const int ni = op.box[1] - op.box[0] + 1, nj = op.box[3] - op.box[2] + 1, nk = op.box[5] - op.box[4] + 1;
-        const long long total = (long long)ni * nj * nk;
-        const int tw = bc_tape_width(op.code);
-        for (long long q2 = tid; q2 < total; q2 += nthr) {
-            const int i = op.box[0] + (int)(q2 % ni);
-            const int j = op.box[2] + (int)((q2 / ni) % nj);
-            const int k = op.box[4] + (int)(q2 / ((long long)ni * nj));
-            const long long p = bidx(pg, i, j, k);
-            const double *t = tp + op.tape + tw * q2;
-            switch (op.code) {
-            case OP_SET: L[op.var][p] = 0.0; break;
-            case OP_DIR_P: {
-                const double e = t[0], rn = op.val / (pg.gamma - 1.0) / e;
-                lE[p] += -rn / e * lR[p];
-                lR[p] = 0.0;
-                break;
-            }
-            case OP_P_LOAD: lR[p] += t[1] * lP[p]; lE[p] += t[0] * lP[p]; lP[p] = 0.0; break;
-            case OP_R_FROM_P: {
-                const double pv = t[0], e = t[1];
-                lP[p] += lR[p] / e;
-                lE[p] += -pv / (e * e) * lR[p];
-                lR[p] = 0.0;
-                break;
-            }
-            case OP_CORNER_E0: lE[p] = 0.0; break;
-            case OP_P_FROM_E: lE[p] += lP[p]; lP[p] = 0.0; break;
-            case OP_E_ADD_P: lP[p] += lE[p]; break;
-            case OP_E_DIV: lE[p] = lE[p] / (double)op.aux; break;
-            case OP_R0: lR[p] = 0.0; break;
-            case OP_R_ADD_P: lP[p] += lR[p]; break;
-            case OP_R_DIV_E: {
-                const double r = t[0], e = t[1], aux = (double)op.aux;
-                lE[p] += -r / (e * e) / aux * lR[p];
-                lR[p] = lR[p] / e / aux;
-                break;
-            }
-            case OP_LID: L[op.var][p] = 0.0; break;
-            case OP_SINE: break;
-            case OP_HOLD:
-                for (int v = 0; v < op.aux; v++) L[bc_hold_field(v)][p] = 0.0;
-                break;
-            default: break;
-            }
+        case OP_NEU: bc_extrapolate_adj(L[op.var] + p, op.step[0], op.len, cf); break;
+        case OP_P_LOAD: lR[p] += t[1] * lP[p]; lE[p] += t[0] * lP[p]; lP[p] = 0.0; break;
+        case OP_P_NEU: bc_extrapolate_adj(lP + p, op.step[0], op.len, cf); break;
+        case OP_R_FROM_P: {
+            const double pv = t[0], e = t[1];
+            lP[p] += lR[p] / e;
+            lE[p] += -pv / (e * e) * lR[p];
+            lR[p] = 0.0;
+            break;
         }
-        sync();
-    }
+        case OP_CORNER_E0: lE[p] = 0.0; break;
+        case OP_P_FROM_E: lE[p] += lP[p]; lP[p] = 0.0; break;
+        case OP_E_ADD_P: lP[p] += lE[p]; break;
+        case OP_E_DIV: lE[p] = lE[p] / (double)op.aux; break;
+        case OP_R0: lR[p] = 0.0; break;
+        case OP_R_ADD_P: lP[p] += lR[p]; break;
+        case OP_R_DIV_E: {
+            const double rr = t[0], e = t[1], aux = (double)op.aux;
+            lE[p] += -rr / (e * e) / aux * lR[p];
+            lR[p] = lR[p] / e / aux;
+            break;
+        }
+        case OP_LID: L[op.var][p] = 0.0; break;
+        case OP_SINE: break;
+        case OP_HOLD:
+            for (int v = 0; v < op.aux; v++) L[bc_hold_field(v)][p] = 0.0;
+            break;
+        default: break;
+        }
+    });
 }
 
-__global__ void k_bc_adj(
-    BcProgram pg, StateSet lam, double *lPbase, long long pstride, const double *tape, long long tstride)
+__global__ void __launch_bounds__(512) k_bc_adj(BcProgram pg, StateSet lam, double *lPbase, long long pstride,
+                                                const double *tape, long long tstride)
 {
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
     k_bc_adj_run(blockIdx.x, threadIdx.x, blockDim.x, [] { __syncthreads(); }, pg, lam, lPbase, pstride, tape, tstride);
 }
 
-__global__ void k_bc_adj_cluster(
-    BcProgram pg, StateSet lam, double *lPbase, long long pstride, const double *tape, long long tstride)
+__global__ void __launch_bounds__(512) k_bc_adj_cluster(BcProgram pg, StateSet lam, double *lPbase, long long pstride,
+                                                        const double *tape, long long tstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ long long bc_sh[];
+    bc_stage(pg, bc_sh);
     k_bc_adj_run(blockIdx.x / (int)cl.num_blocks(), (int)cl.block_rank() * blockDim.x + threadIdx.x, (int)cl.num_threads(),
-           [&] { cl.sync(); }, pg, lam, lPbase, pstride, tape, tstride);
+                 [&] { cl.sync(); }, pg, lam, lPbase, pstride, tape, tstride);
 }
 
 }  // namespace gatt

@@ -123,7 +123,14 @@ struct gatt_ctx {
     std::vector<double> coef1, coef2;
     std::vector<Dist> dists;
     std::vector<double> distx;
-    BcOp *d_ops = nullptr;
+    // two forms of it (bc.cuh): d_prog[0] for steps and the tangent, d_prog[1] (the scratch-field
+    // ops) for the recorded program and its adjoint
+    struct BcDev {
+        BcOp *ops = nullptr;
+        unsigned *lev = nullptr;
+        int nops = 0, nlev = 0;
+        long long widest = 0;  // points of the largest level
+    } d_prog[2];
     int nops = 0;
     double *d_coef1 = nullptr, *d_coef2 = nullptr, *d_xs = nullptr;
     // holdInlet: the values the first gatt_apply_bc kept, hold_len per member, laid out as the
@@ -206,7 +213,6 @@ struct gatt_ctx {
     bool mc_done = false;   // set when a filter launch ran the max-change epilogue
     int bc_cluster = 0;     // CTAs per member for the boundary program (0: one CTA, k_bc)
     int bc_cluster_rec = 0, bc_cluster_tl = 0, bc_cluster_adj = 0;  // same, tape / tangent / adjoint
-    long long bc_points = 0;  // point updates of one application of the program (sum over ops)
     // per-kernel-class timing (gatt_profile_kernels): events around every launch
     bool profiling = false;
     int prof_cls = -1;
@@ -1056,37 +1062,159 @@ void neumann_box(const int *in, int dir, int len, int *out)
     }
 }
 
+// One op of the boundary program on the host: the op and the points it reads and writes, per
+// field (bits 0..4: U, V, W, R, E; 5: the scratch field P).
+struct HostBcOp {
+    struct Acc {
+        unsigned fields;
+        int box[6];
+    };
+    BcOp op;
+    std::vector<Acc> rd, wr;
+};
+
+bool bc_overlap(const std::vector<HostBcOp::Acc> &x, const std::vector<HostBcOp::Acc> &y)
+{
+    for (const auto &a : x)
+        for (const auto &b : y) {
+            if (!(a.fields & b.fields)) continue;
+            bool apart = false;
+            for (int q = 0; q < 3; q++) apart |= a.box[2 * q + 1] < b.box[2 * q] || b.box[2 * q + 1] < a.box[2 * q];
+            if (!apart) return true;
+        }
+    return false;
+}
+
+// Sort the ops into levels (bc.cuh) and upload them: an op's level is one more than the highest
+// level of the earlier ops it conflicts with.  strict: ops that read the same point conflict too
+// (their adjoints add to it).
+int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict)
+{
+    std::vector<int> level(ops.size(), 0);
+    int top = 0;
+    for (size_t j = 0; j < ops.size(); j++) {
+        for (size_t i = 0; i < j; i++) {
+            if (level[i] < level[j]) continue;
+            const HostBcOp &a = ops[i], &b = ops[j];
+            if (bc_overlap(a.wr, b.rd) || bc_overlap(a.wr, b.wr) || bc_overlap(a.rd, b.wr) ||
+                (strict && bc_overlap(a.rd, b.rd)))
+                level[j] = level[i] + 1;
+        }
+        top = std::max(top, level[j]);
+    }
+    std::vector<BcOp> out;
+    std::vector<unsigned> begin, points;
+    d.widest = 0;
+    for (int l = 0; l <= top && !ops.empty(); l++) {
+        begin.push_back((unsigned)out.size());
+        points.push_back(0);
+        for (size_t j = 0; j < ops.size(); j++) {
+            if (level[j] != l) continue;
+            BcOp o = ops[j].op;
+            const long long ni = o.box[1] - o.box[0] + 1, nj = o.box[3] - o.box[2] + 1, nk = o.box[5] - o.box[4] + 1;
+            if (points.back() && (long long)points.back() + ni * nj * nk > INT_MAX) {  // its index range ends here
+                begin.push_back((unsigned)out.size());
+                points.push_back(0);
+            }
+            o.first = points.back();
+            o.count = (unsigned)(ni * nj * nk);
+            o.fd_ni = make_fastdiv((uint32_t)ni);
+            o.fd_nij = make_fastdiv((uint32_t)(ni * nj));
+            points.back() += o.count;
+            d.widest = std::max(d.widest, (long long)points.back());
+            out.push_back(o);
+        }
+    }
+    cudaFree(d.ops); d.ops = nullptr;
+    cudaFree(d.lev); d.lev = nullptr;
+    d.nops = (int)out.size();
+    d.nlev = (int)begin.size();
+    if (out.empty()) return GATT_OK;
+    std::vector<unsigned> lev(begin);
+    lev.push_back((unsigned)out.size());
+    lev.insert(lev.end(), points.begin(), points.end());
+    lev.push_back(0);  // whole 8-byte words
+    CU(cudaMalloc(&d.ops, out.size() * sizeof(BcOp)));
+    CU(cudaMemcpy(d.ops, out.data(), out.size() * sizeof(BcOp), cudaMemcpyHostToDevice));
+    CU(cudaMalloc(&d.lev, lev.size() * sizeof(unsigned)));
+    CU(cudaMemcpy(d.lev, lev.data(), lev.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+    return GATT_OK;
+}
+
 int build_bc_program(gatt_ctx *c)
 {
-    std::vector<BcOp> ops;
+    constexpr unsigned R = 1u << 3, E = 1u << 4, P = 1u << 5;
+    std::vector<HostBcOp> ops[2];  // with fused pressure items and corners, and in scratch form
     auto mk = [&](int code, int var, const int *box) {
-        BcOp o;
-        memset(&o, 0, sizeof(o));
-        o.code = code; o.var = var;
-        for (int q = 0; q < 6; q++) o.box[q] = box[q];
+        HostBcOp o;
+        memset(&o.op, 0, sizeof(o.op));
+        o.op.code = code; o.op.var = var;
+        for (int q = 0; q < 6; q++) o.op.box[q] = box[q];
         return o;
     };
+    auto acc = [](unsigned fields, const int *box) {
+        HostBcOp::Acc a;
+        a.fields = fields;
+        for (int q = 0; q < 6; q++) a.box[q] = box[q];
+        return a;
+    };
+    // an op that reads rd and writes wr at its own points
+    auto local = [&](int form, HostBcOp o, unsigned rd, unsigned wr) {
+        if (rd) o.rd.push_back(acc(rd, o.op.box));
+        if (wr) o.wr.push_back(acc(wr, o.op.box));
+        ops[form].push_back(o);
+    };
+    auto both = [&](const HostBcOp &o, unsigned rd, unsigned wr) { local(0, o, rd, wr); local(1, o, rd, wr); };
     auto row = [&](const HostBC &h, int i, int *box) {
         for (int q = 0; q < 6; q++) box[q] = h.ind[i + (size_t)h.n * q];
     };
+    const long long stride[3] = {1, c->nx, (long long)c->nx * c->ny};
+    auto step_of = [&](int dir) { return (dir & 1) ? stride[(dir - 1) / 2] : -stride[(dir - 1) / 2]; };
+    auto thin = [](const int *box, int dir) { return box[(dir - 1) / 2 * 2] == box[(dir - 1) / 2 * 2 + 1]; };
+    // the face an extrapolation along dir sets, and the len planes it reads
+    auto face_of = [](const int *box, int dir, int *face) {
+        const int a = (dir - 1) / 2 * 2;
+        for (int q = 0; q < 6; q++) face[q] = box[q];
+        face[a + 1] = face[a];
+    };
+    auto read_of = [&](const int *face, int dir, int len, int *rd) {
+        const int a = (dir - 1) / 2 * 2;
+        for (int q = 0; q < 6; q++) rd[q] = face[q];
+        if (dir & 1) { rd[a] = face[a] + 1; rd[a + 1] = face[a] + len; }
+        else { rd[a] = face[a] - len; rd[a + 1] = face[a] - 1; }
+    };
+    auto extrapolate = [&](int code, int var, const int *box, int dir, int len, int coef) {
+        int face[6];
+        face_of(box, dir, face);
+        HostBcOp o = mk(code, var, face);
+        o.op.len = len; o.op.coef = coef; o.op.step[0] = step_of(dir);
+        return o;
+    };
     const int NL = (int)c->coef1.size(), N2 = (int)c->coef2.size();
     const int order[4] = {GATT_VAR_U, GATT_VAR_V, GATT_VAR_W, GATT_VAR_E};
-    int box[6], ext[6];
+    int box[6], ext[6], rd[6];
     // Dirichlet (nseq.F90:357-373)
     for (int v : order) {
         const HostBC &h = c->bc[GATT_BC_DIRICHLET][v];
         for (int i = 0; i < h.n; i++) {
             row(h, i, box); TRY(check_box(c, box));
-            BcOp o = mk(OP_SET, v, box); o.val = h.val[i]; ops.push_back(o);
+            HostBcOp o = mk(OP_SET, v, box); o.op.val = h.val[i]; both(o, 0, 1u << v);
         }
     }
     {
         const HostBC &h = c->bc[GATT_BC_DIRICHLET][GATT_VAR_R];
         for (int i = 0; i < h.n; i++) {
             row(h, i, box); TRY(check_box(c, box));
-            BcOp o = mk(OP_DIR_P, GATT_VAR_R, box); o.val = h.val[i]; ops.push_back(o);
+            HostBcOp o = mk(OP_DIR_P, GATT_VAR_R, box); o.op.val = h.val[i]; both(o, E, R);
         }
     }
+    // P <- its extrapolation along dir at the face of box (P loaded over ext before)
+    auto p_neumann = [&](int var, const int *bx, int dir, int len, int coef) {
+        HostBcOp o = extrapolate(OP_P_NEU, var, bx, dir, len, coef);
+        read_of(o.op.box, dir, len, rd);
+        o.rd.push_back(acc(P, rd));
+        local(1, o, 0, P);
+    };
     // Neumann (kind 1, nseq.F90:377-400) and null second derivative (kind 2, :491-513)
     auto neumann_lists = [&](int kind, int len, int coefsel) -> int {
         if (len < 1 && (c->bc[kind][0].n || c->bc[kind][1].n || c->bc[kind][2].n || c->bc[kind][3].n ||
@@ -1099,7 +1227,10 @@ int build_bc_program(gatt_ctx *c)
                 const int d = h.dirs[i];
                 if (d < 1 || d > 6) return fail(GATT_ERR_BADARG, "Neumann direction must be 1..6");
                 neumann_box(box, d, len, ext); TRY(check_box(c, ext));
-                BcOp o = mk(OP_NEU, v, ext); o.dir = d; o.len = len; o.coef = coefsel; ops.push_back(o);
+                HostBcOp o = extrapolate(OP_NEU, v, box, d, len, coefsel);
+                read_of(o.op.box, d, len, rd);
+                o.rd.push_back(acc(1u << v, rd));
+                both(o, 0, 1u << v);
             }
         }
         const HostBC &h = c->bc[kind][GATT_VAR_R];
@@ -1108,9 +1239,18 @@ int build_bc_program(gatt_ctx *c)
             const int d = h.dirs[i];
             if (d < 1 || d > 6) return fail(GATT_ERR_BADARG, "Neumann direction must be 1..6");
             neumann_box(box, d, len, ext); TRY(check_box(c, ext)); TRY(check_box(c, box));
-            ops.push_back(mk(OP_P_LOAD, 3, ext));
-            BcOp o = mk(OP_P_NEU, 3, ext); o.dir = d; o.len = len; o.coef = coefsel; ops.push_back(o);
-            ops.push_back(mk(OP_R_FROM_P, 3, box));
+            const size_t n0 = ops[1].size();
+            local(1, mk(OP_P_LOAD, 3, ext), R | E, P);
+            p_neumann(3, box, d, len, coefsel);
+            local(1, mk(OP_R_FROM_P, 3, box), P | E, R);
+            if (thin(box, d)) {
+                HostBcOp o = extrapolate(OP_PNEU, 3, box, d, len, coefsel);
+                read_of(o.op.box, d, len, rd);
+                o.rd.push_back(acc(R | E, rd));
+                local(0, o, E, R);
+            } else {
+                ops[0].insert(ops[0].end(), ops[1].begin() + n0, ops[1].end());
+            }
         }
         return GATT_OK;
     };
@@ -1123,28 +1263,43 @@ int build_bc_program(gatt_ctx *c)
         const int nd = std::abs(cd[0]) + std::abs(cd[1]) + std::abs(cd[2]);
         if (nd == 0) return fail(GATT_ERR_BADARG, "corner without direction");
         if (NL < 1) return fail(GATT_ERR_STATE, "Neumann coefficients not set");
+        const size_t n0 = ops[1].size();
+        HostBcOp one = mk(OP_CORNER, c->cAd[i] == 1, box);
+        one.op.aux = nd; one.op.len = NL;
+        int used = 0;
+        bool fits = true;  // every direction is -1, 0 or 1 and the box one node thick along it
+        for (int a = 0; a < 3; a++) {
+            if (cd[a] == 0) continue;
+            const int d = cd[a] == 1 ? 2 * a + 1 : 2 * a + 2;
+            fits = fits && (cd[a] == 1 || cd[a] == -1) && thin(box, d);
+            one.op.step[used++] = step_of(d);
+            read_of(box, d, NL, rd);
+            one.rd.push_back(acc(R | E, rd));
+        }
         if (c->cAd[i] == 1) {
-            ops.push_back(mk(OP_CORNER_E0, 4, box));
+            local(1, mk(OP_CORNER_E0, 4, box), 0, E);
             for (int a = 0; a < 3; a++) {
                 if (cd[a] != 1 && cd[a] != -1) continue;
                 const int d = cd[a] == 1 ? 2 * a + 1 : 2 * a + 2;
                 neumann_box(box, d, NL, ext); TRY(check_box(c, ext));
-                ops.push_back(mk(OP_P_FROM_E, 4, ext));
-                BcOp o = mk(OP_P_NEU, 4, ext); o.dir = d; o.len = NL; o.coef = 0; ops.push_back(o);
-                ops.push_back(mk(OP_E_ADD_P, 4, box));
+                local(1, mk(OP_P_FROM_E, 4, ext), E, P);
+                p_neumann(4, box, d, NL, 0);
+                local(1, mk(OP_E_ADD_P, 4, box), E | P, E);
             }
-            BcOp o = mk(OP_E_DIV, 4, box); o.aux = nd; ops.push_back(o);
+            HostBcOp o = mk(OP_E_DIV, 4, box); o.op.aux = nd; local(1, o, E, E);
         }
-        ops.push_back(mk(OP_R0, 3, box));
+        local(1, mk(OP_R0, 3, box), 0, R);
         for (int a = 0; a < 3; a++) {
             if (cd[a] != 1 && cd[a] != -1) continue;
             const int d = cd[a] == 1 ? 2 * a + 1 : 2 * a + 2;
             neumann_box(box, d, NL, ext); TRY(check_box(c, ext));
-            ops.push_back(mk(OP_P_LOAD, 3, ext));
-            BcOp o = mk(OP_P_NEU, 3, ext); o.dir = d; o.len = NL; o.coef = 0; ops.push_back(o);
-            ops.push_back(mk(OP_R_ADD_P, 3, box));
+            local(1, mk(OP_P_LOAD, 3, ext), R | E, P);
+            p_neumann(3, box, d, NL, 0);
+            local(1, mk(OP_R_ADD_P, 3, box), R | P, R);
         }
-        BcOp o = mk(OP_R_DIV_E, 3, box); o.aux = nd; ops.push_back(o);
+        HostBcOp o = mk(OP_R_DIV_E, 3, box); o.op.aux = nd; local(1, o, R | E, R);
+        if (fits) local(0, one, E, one.op.var ? R | E : R);
+        else ops[0].insert(ops[0].end(), ops[1].begin() + n0, ops[1].end());
     }
     TRY(neumann_lists(GATT_BC_SECOND, N2, 1));
     // disturbances (runDisturbances.F90)
@@ -1153,92 +1308,38 @@ int build_bc_program(gatt_ctx *c)
     for (const Dist &d : c->dists) {
         TRY(check_box(c, d.ind));
         if (d.type == GATT_DIST_HOLD_INLET) {
-            BcOp o = mk(OP_HOLD, 0, d.ind);
-            o.aux = d.par > 0.5 ? 5 : 4;
+            HostBcOp o = mk(OP_HOLD, 0, d.ind);
+            o.op.aux = d.par > 0.5 ? 5 : 4;
             const long long n = (long long)(d.ind[1] - d.ind[0] + 1) * (d.ind[3] - d.ind[2] + 1) * (d.ind[5] - d.ind[4] + 1);
-            if (hold_len + o.aux * n > INT_MAX) return fail(GATT_ERR_BADARG, "holdInlet boxes too large");
-            o.xoff = (int)hold_len;
-            hold_len += o.aux * n;
+            if (hold_len + o.op.aux * n > INT_MAX) return fail(GATT_ERR_BADARG, "holdInlet boxes too large");
+            o.op.xoff = (int)hold_len;
+            hold_len += o.op.aux * n;
             hold_sig.insert(hold_sig.end(), d.ind, d.ind + 6);
-            hold_sig.push_back(o.aux);
-            ops.push_back(o);
+            hold_sig.push_back(o.op.aux);
+            const unsigned held = 0x17u | (o.op.aux == 5 ? R : 0u);  // U V W E (R)
+            both(o, held, held);
         } else {
-            BcOp o = mk(d.type == GATT_DIST_PERIODIC_SINE ? OP_SINE : OP_LID, d.var, d.ind);
-            o.xoff = d.xoff; o.val = d.par; ops.push_back(o);
+            const bool sine = d.type == GATT_DIST_PERIODIC_SINE;
+            HostBcOp o = mk(sine ? OP_SINE : OP_LID, d.var, d.ind);
+            o.op.xoff = d.xoff; o.op.val = d.par;
+            both(o, sine ? 1u << d.var : 0, 1u << d.var);
         }
-    }
-    // phases: an op joins the running phase unless it reads or writes a field point that an op
-    // of the phase writes, or writes one that it reads (fields U, V, W, R, E and the P scratch;
-    // boxes compared as index ranges, the Neumann ones over their extended box)
-    {
-        auto access = [](const BcOp &o, unsigned &rd, unsigned &wr) {
-            const unsigned U = 1u << o.var, R = 1u << 3, E = 1u << 4, P = 1u << 5;
-            rd = wr = 0;
-            switch (o.code) {
-            case OP_SET: case OP_LID: wr = U; break;
-            case OP_SINE: rd = wr = U; break;
-            case OP_HOLD: rd = wr = 0x17u | (o.aux == 5 ? R : 0u); break;  // U V W E (R)
-            case OP_DIR_P: rd = E; wr = R; break;
-            case OP_NEU: rd = wr = U; break;
-            case OP_P_LOAD: rd = R | E; wr = P; break;
-            case OP_P_NEU: rd = wr = P; break;
-            case OP_R_FROM_P: rd = P | E; wr = R; break;
-            case OP_CORNER_E0: wr = E; break;
-            case OP_P_FROM_E: rd = E; wr = P; break;
-            case OP_E_ADD_P: rd = E | P; wr = E; break;
-            case OP_E_DIV: rd = wr = E; break;
-            case OP_R0: wr = R; break;
-            case OP_R_ADD_P: rd = R | P; wr = R; break;
-            case OP_R_DIV_E: rd = R | E; wr = R; break;
-            default: rd = wr = 0x3f; break;
-            }
-        };
-        auto overlap = [](const BcOp &a, const BcOp &b) {
-            for (int q = 0; q < 3; q++)
-                if (a.box[2 * q + 1] < b.box[2 * q] || b.box[2 * q + 1] < a.box[2 * q]) return false;
-            return true;
-        };
-        size_t start = 0;
-        for (size_t i = 0; i < ops.size(); i++) {
-            unsigned rb, wb;
-            access(ops[i], rb, wb);
-            bool dep = false;
-            for (size_t k = start; k < i && !dep; k++) {
-                unsigned ra, wa;
-                access(ops[k], ra, wa);
-                dep = ((wa & (rb | wb)) || (ra & wb)) && overlap(ops[k], ops[i]);
-            }
-            if (dep) {
-                ops[i - 1].sync = 1;
-                start = i;
-            }
-        }
-        if (!ops.empty()) ops.back().sync = 1;
     }
     // adjoint tape offsets (base values of the nonlinear ops, per box point)
     long long tape = 0;
-    for (BcOp &o : ops) {
-        const int tw = bc_tape_width(o.code);
+    for (HostBcOp &h : ops[1]) {
+        BcOp &o = h.op;
         o.tape = tape;
-        if (o.code != OP_NEU && o.code != OP_P_NEU && tw > 0)
-            tape += (long long)tw * (o.box[1] - o.box[0] + 1) * (o.box[3] - o.box[2] + 1) * (o.box[5] - o.box[4] + 1);
+        tape += (long long)bc_tape_width(o.code) * (o.box[1] - o.box[0] + 1) * (o.box[3] - o.box[2] + 1) *
+                (o.box[5] - o.box[4] + 1);
     }
     c->tape_len = tape;
-    c->bc_points = 0;
-    for (const BcOp &o : ops) {
-        const long long ni = o.box[1] - o.box[0] + 1, nj = o.box[3] - o.box[2] + 1, nk = o.box[5] - o.box[4] + 1;
-        c->bc_points += (o.code == OP_NEU || o.code == OP_P_NEU) ? (o.dir <= 2 ? nj * nk : o.dir <= 4 ? ni * nk : ni * nj)
-                                                                 : ni * nj * nk;
-    }
-    cudaFree(c->d_ops); c->d_ops = nullptr;
+    TRY(upload_bc_levels(c->d_prog[0], ops[0], false));
+    TRY(upload_bc_levels(c->d_prog[1], ops[1], true));
+    c->nops = c->d_prog[0].nops;
     cudaFree(c->d_coef1); c->d_coef1 = nullptr;
     cudaFree(c->d_coef2); c->d_coef2 = nullptr;
     cudaFree(c->d_xs); c->d_xs = nullptr;
-    c->nops = (int)ops.size();
-    if (!ops.empty()) {
-        CU(cudaMalloc(&c->d_ops, ops.size() * sizeof(BcOp)));
-        CU(cudaMemcpy(c->d_ops, ops.data(), ops.size() * sizeof(BcOp), cudaMemcpyHostToDevice));
-    }
     if (!c->coef1.empty()) {
         CU(cudaMalloc(&c->d_coef1, c->coef1.size() * sizeof(double)));
         CU(cudaMemcpy(c->d_coef1, c->coef1.data(), c->coef1.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -1262,11 +1363,13 @@ int build_bc_program(gatt_ctx *c)
     return GATT_OK;
 }
 
-// The program as the kernels take it, at time t + tfac dt of the step parameters on the device
-BcProgram bc_program(const gatt_ctx *c, double tfac)
+// The program (form 0 or 1 of d_prog) as the kernels take it, at time t + tfac dt of the step
+// parameters on the device
+BcProgram bc_program(const gatt_ctx *c, double tfac, int form = 0)
 {
+    const gatt_ctx::BcDev &d = c->d_prog[form];
     BcProgram pg;
-    pg.ops = c->d_ops; pg.nops = c->nops; pg.coef1 = c->d_coef1; pg.coef2 = c->d_coef2; pg.xs = c->d_xs;
+    pg.ops = d.ops; pg.lev = d.lev; pg.nops = d.nops; pg.nlev = d.nlev; pg.coef1 = c->d_coef1; pg.coef2 = c->d_coef2; pg.xs = c->d_xs;
     pg.gamma = c->ph.gamma; pg.nx = c->nx; pg.ny = c->ny; pg.nz = c->nz;
     pg.sp = c->d_params; pg.tfac = tfac; pg.tfix = 0.0;
     pg.hold = c->d_hold; pg.hstride = c->hold_len; pg.hold_save = 0;
@@ -1330,16 +1433,18 @@ int choose_bc_cluster(gatt_ctx *c)
     return GATT_OK;
 }
 
-// Launch a boundary-program kernel for nmem members: the cluster form with cs CTAs per
-// member, cs the largest power of two up to the schedulable size cs_max that keeps the
-// clusters of all members within the SMs and gives every CTA about 2048 point updates (small
-// or many-member programs gain nothing from more CTAs and pay a barrier per op); with cs < 2
-// the one-CTA form.
+// Launch a boundary-program kernel on form `form` of the program for nmem members: the cluster
+// form with cs CTAs per member, cs the largest power of two up to the schedulable size cs_max
+// that keeps the clusters of all members within the SMs and gives every CTA about 2048 points of
+// the largest level (smaller programs gain nothing from more CTAs and pay a dearer barrier per
+// level); with cs < 2 the one-CTA form.
 template <typename... KArgs, typename... Args>
-int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...), int cs_max, int nmem, size_t smem,
+int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...), int cs_max, int nmem, int form,
               Args &&...args)
 {
-    const long long by_work = (c->bc_points + 2047) / 2048;
+    const gatt_ctx::BcDev &d = c->d_prog[form];
+    const size_t need = bc_stage_bytes(d.nops, d.nlev), smem = need <= (size_t)kBcStagedBytes ? need : 0;
+    const long long by_work = (d.widest + 2047) / 2048;
     const long long by_sms = std::max(1, c->nsm / std::max(1, nmem));
     int cs = 1;
     while (cs * 2 <= cs_max && cs * 2 <= by_work && cs * 2 <= by_sms) cs *= 2;
@@ -1376,9 +1481,8 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
     } else if (c->hold_len > 0 && !c->hold_saved) {
         return fail(GATT_ERR_STATE, "holdInlet: call gatt_apply_bc on the initial state before stepping");
     }
-    const size_t smem = c->nops <= kBcStagedOps ? (size_t)c->nops * sizeof(BcOp) : 0;  // staged ops
     TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc, k_bc_cluster, c->bc_cluster, nmem, smem, pg, q, c->P, (long long)c->npts));
+    TRY(launch_bc(c, k_bc, k_bc_cluster, c->bc_cluster, nmem, 0, pg, q, c->P, (long long)c->npts));
     return after_launch(c);
 }
 
@@ -1913,7 +2017,7 @@ int bc_rec(gatt_ctx *c, const StateSet &x, int which, double tfac)
     if (c->nops == 0) return GATT_OK;
     const long long ts = std::max(1LL, c->tape_len);
     TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc_rec, k_bc_rec_cluster, c->bc_cluster_rec, c->nb, 0, bc_program(c, tfac), x, c->P,
+    TRY(launch_bc(c, k_bc_rec, k_bc_rec_cluster, c->bc_cluster_rec, c->nb, 1, bc_program(c, tfac, 1), x, c->P,
                   (long long)c->npts, c->a_tape + which * ts * c->nb, ts));
     return after_launch(c);
 }
@@ -1925,7 +2029,7 @@ int bc_adj(gatt_ctx *c, const StateSet &lam, int which)
     const long long ts = std::max(1LL, c->tape_len);
     CU(cudaMemsetAsync(c->a_lP, 0, sizeof(double) * (size_t)c->npts * c->nb, c->stream));
     TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc_adj, k_bc_adj_cluster, c->bc_cluster_adj, c->nb, 0, bc_program(c, 1.0), lam, c->a_lP,
+    TRY(launch_bc(c, k_bc_adj, k_bc_adj_cluster, c->bc_cluster_adj, c->nb, 1, bc_program(c, 1.0, 1), lam, c->a_lP,
                   (long long)c->npts, (const double *)(c->a_tape + which * ts * c->nb), ts));
     return after_launch(c);
 }
@@ -2513,7 +2617,8 @@ void gatt_destroy(gatt_ctx *c)
                        c->a_lm, c->a_mscr};
     for (double *p : dbufs) cudaFree(p);
     for (double *p : bufs) cudaFree(p);
-    cudaFree(c->d_ops); cudaFree(c->acc); cudaFree(c->d_params);
+    for (gatt_ctx::BcDev &d : c->d_prog) { cudaFree(d.ops); cudaFree(d.lev); }
+    cudaFree(c->acc); cudaFree(c->d_params);
     cudaFree(c->fsum); cudaFree(c->fpart);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_err) cudaFreeHost(c->h_err);
