@@ -18,7 +18,7 @@
 // loads that miss to L2).  The pressure Neumann items and the corners are therefore one op
 // each (P = R E formed on the fly, not through a scratch field): the 128^2 lid-driven cavity
 // has 3 levels instead of 15 phases of consecutive ops, the 800x300 boundary layer over a
-// cavity 9 instead of 27.
+// cavity 7 instead of 27.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -76,6 +76,7 @@ struct BcProgram {
     const BcOp *ops;
     const unsigned *lev;
     int nops, nlev;
+    int n1, n2;           // lengths of the two
     const double *coef1;  // neumannCoeffs
     const double *coef2;  // neumann2Coeffs
     const double *xs;     // disturbance coordinates (OP_LID) and x factors (OP_SINE)
@@ -115,44 +116,70 @@ __device__ __forceinline__ double bc_lid(const BcProgram &pg, const BcOp &op, in
 // holdInlet.F90 keeps u, v, w, e (and r with holdDensity): field of the v-th held value
 __device__ __forceinline__ int bc_hold_field(int v) { return v < 3 ? v : (v == 3 ? 4 : 3); }
 
+// Extrapolation terms whose loads are issued together (the sixth-order Neumann rows have six
+// nodes); one load at a time waits for L2 once per term.
+constexpr int kBcLen = 6;
+
 // applyNeumann (nseq.F90:552-599) at one face point: u points to it, st steps into the domain;
 // products and sums rounded one by one as the reference does (no fused multiply-add: chains of
 // boundary items, with divisions by extrapolated E between them, amplify the difference)
 __device__ __forceinline__ double bc_extrapolate(const double *u, long long st, int len, const double *c)
 {
-    double v = __dmul_rn(c[0], u[st]);
-    for (int m = 2; m <= len; m++) v = __dadd_rn(v, __dmul_rn(c[m - 1], u[m * st]));
+    double x[kBcLen];
+#pragma unroll
+    for (int m = 1; m <= kBcLen; m++) x[m - 1] = m <= len ? u[m * st] : 0.0;
+    double v = __dmul_rn(c[0], x[0]);
+#pragma unroll
+    for (int m = 2; m <= kBcLen; m++)
+        if (m <= len) v = __dadd_rn(v, __dmul_rn(c[m - 1], x[m - 1]));
+    for (int m = kBcLen + 1; m <= len; m++) v = __dadd_rn(v, __dmul_rn(c[m - 1], u[m * st]));
     return v;
 }
 // the same of P = R*E
 __device__ __forceinline__ double bc_extrapolate_p(const double *r, const double *e, long long st, int len,
                                                    const double *c)
 {
-    double v = __dmul_rn(c[0], __dmul_rn(r[st], e[st]));
-    for (int m = 2; m <= len; m++) v = __dadd_rn(v, __dmul_rn(c[m - 1], __dmul_rn(r[m * st], e[m * st])));
+    double x[kBcLen], y[kBcLen];
+#pragma unroll
+    for (int m = 1; m <= kBcLen; m++) {
+        x[m - 1] = m <= len ? r[m * st] : 0.0;
+        y[m - 1] = m <= len ? e[m * st] : 0.0;
+    }
+    double v = __dmul_rn(c[0], __dmul_rn(x[0], y[0]));
+#pragma unroll
+    for (int m = 2; m <= kBcLen; m++)
+        if (m <= len) v = __dadd_rn(v, __dmul_rn(c[m - 1], __dmul_rn(x[m - 1], y[m - 1])));
+    for (int m = kBcLen + 1; m <= len; m++)
+        v = __dadd_rn(v, __dmul_rn(c[m - 1], __dmul_rn(r[m * st], e[m * st])));
     return v;
 }
 
-// Largest program whose ops and levels are staged in shared memory (48 KB, no opt-in needed);
-// longer programs read them from global memory.
+// Largest program that is staged in shared memory (ops, levels, coefficients; 48 KB, no opt-in
+// needed); longer programs read them from global memory.
 constexpr int kBcStagedBytes = 48 * 1024;
-__host__ __device__ __forceinline__ size_t bc_stage_bytes(int nops, int nlev)
+constexpr int kBcThreads = 512;   // threads of a boundary-program CTA
+__host__ __device__ __forceinline__ size_t bc_stage_bytes(const BcProgram &pg)
 {
-    return (size_t)nops * sizeof(BcOp) + ((size_t)(2 * nlev + 1) * sizeof(unsigned) + 7) / 8 * 8;
+    return (size_t)pg.nops * sizeof(BcOp) + (size_t)(pg.nlev + 1) * 8 + (size_t)(pg.n1 + pg.n2) * 8;
 }
 
-// Copy ops and levels to shared memory (when they fit) and point pg there; every thread of the
-// CTA calls it.  The host pads the level table to whole 8-byte words.
+// Copy the program to shared memory (when it fits) and point pg there; every thread of the CTA
+// calls it.  The host pads the level table to whole 8-byte words.
 __device__ __forceinline__ void bc_stage(BcProgram &pg, long long *sh)
 {
-    if (bc_stage_bytes(pg.nops, pg.nlev) > (size_t)kBcStagedBytes) return;
-    const int n = pg.nops * (int)(sizeof(BcOp) / sizeof(long long)), m = (2 * pg.nlev + 2) / 2;
+    if (bc_stage_bytes(pg) > (size_t)kBcStagedBytes) return;
+    const int n = pg.nops * (int)(sizeof(BcOp) / sizeof(long long)), m = pg.nlev + 1;
     const long long *g = reinterpret_cast<const long long *>(pg.ops), *gl = reinterpret_cast<const long long *>(pg.lev);
+    double *c1 = reinterpret_cast<double *>(sh + n + m), *c2 = c1 + pg.n1;
     for (int i = threadIdx.x; i < n; i += blockDim.x) sh[i] = g[i];
     for (int i = threadIdx.x; i < m; i += blockDim.x) sh[n + i] = gl[i];
+    for (int i = threadIdx.x; i < pg.n1; i += blockDim.x) c1[i] = pg.coef1[i];
+    for (int i = threadIdx.x; i < pg.n2; i += blockDim.x) c2[i] = pg.coef2[i];
     __syncthreads();
     pg.ops = reinterpret_cast<const BcOp *>(sh);
     pg.lev = reinterpret_cast<const unsigned *>(sh + n);
+    pg.coef1 = c1;
+    pg.coef2 = c2;
 }
 
 // fn(op, r, i, p) for every point of every level, thread tid of nthr: r the point's index in
@@ -178,9 +205,18 @@ __device__ __forceinline__ void bc_levels(const BcProgram &pg, int tid, int nthr
     }
 }
 
+// A member's state arrays: indexed by the op's variable, straight from the kernel parameters (a
+// local pointer array would live in local memory).
+struct BcFields {
+    const StateSet &s;
+    long long off;
+    __device__ __forceinline__ BcFields(const StateSet &set, int b) : s(set), off(b * set.bstride) {}
+    __device__ __forceinline__ double *operator[](int v) const { return s.v[v] + off; }
+};
+
 // The program on one member: F the five state arrays (U,V,W,R,E), P a scratch field.
 template <typename Sync>
-__device__ __forceinline__ void bc_run(const BcProgram &pg, double *const *F, double *P, double *H, int tid, int nthr,
+__device__ __forceinline__ void bc_run(const BcProgram &pg, const BcFields &F, double *P, double *H, int tid, int nthr,
                                        Sync sync)
 {
     double *Rr = F[3], *Ee = F[4];
@@ -195,11 +231,15 @@ __device__ __forceinline__ void bc_run(const BcProgram &pg, double *const *F, do
         case OP_CORNER: {
             if (op.var) {
                 double e = 0.0;
-                for (int d = 0; d < op.aux; d++) e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
+#pragma unroll
+                for (int d = 0; d < 3; d++)
+                    if (d < op.aux) e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
                 Ee[p] = e / (double)op.aux;
             }
             double v = 0.0;
-            for (int d = 0; d < op.aux; d++) v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                if (d < op.aux) v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
             Rr[p] = v / Ee[p] / (double)op.aux;
             break;
         }
@@ -228,27 +268,25 @@ __device__ __forceinline__ void bc_run(const BcProgram &pg, double *const *F, do
 }
 
 // One CTA per batch member (block barriers); dynamic shared memory: the staged program.
-__global__ void __launch_bounds__(512) k_bc(BcProgram pg, StateSet q, double *Pbase, long long pstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                            long long pstride)
 {
     extern __shared__ long long bc_sh[];
     const int b = blockIdx.x;
-    double *F[5];
-#pragma unroll
-    for (int f = 0; f < 5; f++) F[f] = q.v[f] + b * q.bstride;
+    const BcFields F(q, b);
     bc_stage(pg, bc_sh);
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
     bc_run(pg, F, Pbase + b * pstride, H, threadIdx.x, blockDim.x, [] { __syncthreads(); });
 }
 
 // One cluster of CTAs per batch member (cluster barriers); launched with a cluster dimension.
-__global__ void __launch_bounds__(512) k_bc_cluster(BcProgram pg, StateSet q, double *Pbase, long long pstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_cluster(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                                    long long pstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int b = blockIdx.x / (int)cl.num_blocks();
-    double *F[5];
-#pragma unroll
-    for (int f = 0; f < 5; f++) F[f] = q.v[f] + b * q.bstride;
+    const BcFields F(q, b);
     extern __shared__ long long bc_sh[];
     bc_stage(pg, bc_sh);
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
@@ -273,12 +311,10 @@ __host__ __device__ __forceinline__ int bc_tape_width(int code)
 // The forward program (scratch form) on the base, recording the tape: member b, thread tid of
 // nthr, sync() a barrier over the nthr threads.
 template <typename Sync>
-__device__ __forceinline__ void k_bc_rec_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, StateSet q,
+__device__ __forceinline__ void k_bc_rec_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, const StateSet &q,
                                              double *Pbase, long long pstride, double *tape, long long tstride)
 {
-    double *F[5];
-#pragma unroll
-    for (int f = 0; f < 5; f++) F[f] = q.v[f] + b * q.bstride;
+    const BcFields F(q, b);
     double *P = Pbase + b * pstride;
     double *Rr = F[3], *Ee = F[4];
     double *tp = tape + b * tstride;
@@ -311,16 +347,16 @@ __device__ __forceinline__ void k_bc_rec_run(int b, int tid, int nthr, Sync sync
     });
 }
 
-__global__ void __launch_bounds__(512) k_bc_rec(BcProgram pg, StateSet q, double *Pbase, long long pstride, double *tape,
-                                                long long tstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_rec(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                                long long pstride, double *tape, long long tstride)
 {
     extern __shared__ long long bc_sh[];
     bc_stage(pg, bc_sh);
     k_bc_rec_run(blockIdx.x, threadIdx.x, blockDim.x, [] { __syncthreads(); }, pg, q, Pbase, pstride, tape, tstride);
 }
 
-__global__ void __launch_bounds__(512) k_bc_rec_cluster(BcProgram pg, StateSet q, double *Pbase, long long pstride,
-                                                        double *tape, long long tstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_rec_cluster(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                                        long long pstride, double *tape, long long tstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -342,12 +378,10 @@ __device__ __forceinline__ double bc_extrapolate_dp(const double *r, const doubl
 // tangent: base q (updated as k_bc does) and tangent dq (P, dP scratch); member b, thread tid
 // of nthr, sync() a barrier over the nthr threads
 template <typename Sync>
-__device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, StateSet q,
-                                            double *Pbase, StateSet dq, double *dPbase, long long pstride)
+__device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, const StateSet &q,
+                                            double *Pbase, const StateSet &dq, double *dPbase, long long pstride)
 {
-    double *F[5], *dF[5];
-#pragma unroll
-    for (int f = 0; f < 5; f++) { F[f] = q.v[f] + b * q.bstride; dF[f] = dq.v[f] + b * dq.bstride; }
+    const BcFields F(q, b), dF(dq, b);
     double *P = Pbase + b * pstride, *dP = dPbase + b * pstride;
     double *Rr = F[3], *Ee = F[4], *dR = dF[3], *dE = dF[4];
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
@@ -377,7 +411,9 @@ __device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync,
             const double aux = (double)op.aux;
             if (op.var) {
                 double e = 0.0, de = 0.0;
-                for (int d = 0; d < op.aux; d++) {
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    if (d >= op.aux) continue;
                     e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
                     de = de + bc_extrapolate(dE + p, op.step[d], op.len, cf);
                 }
@@ -385,7 +421,9 @@ __device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync,
                 dE[p] = de / aux;
             }
             double v = 0.0, dv = 0.0;
-            for (int d = 0; d < op.aux; d++) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                if (d >= op.aux) continue;
                 v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
                 dv = dv + bc_extrapolate_dp(Rr + p, Ee + p, dR + p, dE + p, op.step[d], op.len, cf);
             }
@@ -431,16 +469,17 @@ __device__ __forceinline__ void k_bc_tl_run(int b, int tid, int nthr, Sync sync,
     });
 }
 
-__global__ void __launch_bounds__(512) k_bc_tl(BcProgram pg, StateSet q, double *Pbase, StateSet dq, double *dPbase,
-                                               long long pstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_tl(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                               const __grid_constant__ StateSet dq, double *dPbase, long long pstride)
 {
     extern __shared__ long long bc_sh[];
     bc_stage(pg, bc_sh);
     k_bc_tl_run(blockIdx.x, threadIdx.x, blockDim.x, [] { __syncthreads(); }, pg, q, Pbase, dq, dPbase, pstride);
 }
 
-__global__ void __launch_bounds__(512) k_bc_tl_cluster(BcProgram pg, StateSet q, double *Pbase, StateSet dq,
-                                                       double *dPbase, long long pstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_tl_cluster(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                                       const __grid_constant__ StateSet dq, double *dPbase,
+                                                       long long pstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -462,12 +501,10 @@ __device__ __forceinline__ void bc_extrapolate_adj(double *lam, long long st, in
 // form's levels in reverse.  Its levels also keep apart ops that only read the same point: their
 // adjoints both add to it.
 template <typename Sync>
-__device__ __forceinline__ void k_bc_adj_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, StateSet lam,
+__device__ __forceinline__ void k_bc_adj_run(int b, int tid, int nthr, Sync sync, const BcProgram &pg, const StateSet &lam,
                                              double *lPbase, long long pstride, const double *tape, long long tstride)
 {
-    double *L[5];
-#pragma unroll
-    for (int f = 0; f < 5; f++) L[f] = lam.v[f] + b * lam.bstride;
+    const BcFields L(lam, b);
     double *lP = lPbase + b * pstride;
     double *lR = L[3], *lE = L[4];
     const double *tp = tape + b * tstride;
@@ -514,16 +551,16 @@ __device__ __forceinline__ void k_bc_adj_run(int b, int tid, int nthr, Sync sync
     });
 }
 
-__global__ void __launch_bounds__(512) k_bc_adj(BcProgram pg, StateSet lam, double *lPbase, long long pstride,
-                                                const double *tape, long long tstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_adj(BcProgram pg, const __grid_constant__ StateSet lam, double *lPbase,
+                                                long long pstride, const double *tape, long long tstride)
 {
     extern __shared__ long long bc_sh[];
     bc_stage(pg, bc_sh);
     k_bc_adj_run(blockIdx.x, threadIdx.x, blockDim.x, [] { __syncthreads(); }, pg, lam, lPbase, pstride, tape, tstride);
 }
 
-__global__ void __launch_bounds__(512) k_bc_adj_cluster(BcProgram pg, StateSet lam, double *lPbase, long long pstride,
-                                                        const double *tape, long long tstride)
+__global__ void __launch_bounds__(kBcThreads) k_bc_adj_cluster(BcProgram pg, const __grid_constant__ StateSet lam, double *lPbase,
+                                                        long long pstride, const double *tape, long long tstride)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();

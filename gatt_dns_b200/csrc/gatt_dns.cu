@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -22,6 +23,7 @@
 #include "arnoldi.cuh"
 #include "tangent.cuh"
 #include "bc.cuh"
+#include "lsweep.cuh"
 #include "pointwise.cuh"
 #include "pwpipe.cuh"
 #include "rsweep.cuh"
@@ -54,8 +56,9 @@ int fail(int code, const std::string &msg)
     } while (0)
 
 // Line-solve kernel families: shared-memory tile (any N), register-resident rows loaded
-// from global memory, register-resident rows fed by a TMA ring (persistent CTAs).
-enum SweepFamily { FAM_TILE = 0, FAM_REG = 1, FAM_PIPE = 2 };
+// from global memory, register-resident rows fed by a TMA ring (persistent CTAs),
+// register-resident rows of lines of any length (up to 1024 rows) through asynchronous copies.
+enum SweepFamily { FAM_TILE = 0, FAM_REG = 1, FAM_PIPE = 2, FAM_LINE = 3 };
 
 // Matrix kinds per direction: 0 derivative, 1 filter, 2/3 derivative transpose (LHS^T solve,
 // then R^T band), 4/5 filter transpose (same split); see gatt_set_matrices.
@@ -76,6 +79,13 @@ struct DevDir {
     std::vector<double> hA, hB, hC, hD, hR;
     double *Rm = nullptr;  // band coefficients [nTypes][N][Wp]
     double *Q = nullptr;   // row records [nTypes][N][kQ] (see sweep.cuh)
+    int cap = 0;           // rows per type the two arrays have room for
+    // coefficients of the any-length solver (lsweep.cuh: LineArgs), null where it does not apply
+    // (one allocation at lQ)
+    double *lQ = nullptr, *lS = nullptr;
+    int *lB = nullptr;
+    int lP = 0, nspecial = 0;
+    double lband[16] = {};
 };
 
 struct HostBC {
@@ -426,12 +436,13 @@ int resident_ctas(const void *k, int threads, size_t smem)
     return n;
 }
 
-// Line-solve family for new matrices: GATT_SWEEP = tile | reg | pipe (default pipe).
+// Line-solve family for new matrices: GATT_SWEEP = tile | reg | line | pipe (default pipe).
 int choose_family()
 {
     const char *e = getenv("GATT_SWEEP");
     if (e && strcmp(e, "tile") == 0) return FAM_TILE;
     if (e && strcmp(e, "reg") == 0) return FAM_REG;
+    if (e && strcmp(e, "line") == 0) return FAM_LINE;
     return FAM_PIPE;
 }
 
@@ -469,6 +480,14 @@ int choose_rpb(int d, int N, int Np, int nR, int nTypes, int Wp)
     const int maxp = d == 0 ? kMaxPx : (nR == 6 ? kMaxP : kMaxPyz);
     if (!pipe || P > maxp) return 0;
     return psweep_smem_bytes(d == 0, Np, P, nTypes, Wp, 1) <= kMaxSmem ? kRPB : 0;
+}
+
+// Whether k_lsweep takes lines of N rows and band nR, LL lines to a tile.
+bool line_fits(bool xd, int N, int nR, int LL)
+{
+    const int P = (N + kLineRows - 1) / kLineRows;
+    return nR >= 2 && nR <= kMaxNRreg && P * LL <= line_max_threads(nR) &&
+           line_smem_bytes(xd, N, P, LL, 1, 0, 0, false) <= kMaxSmem;
 }
 
 size_t sweep_smem(int N, int P, int nR, int Wp, bool stage = true)
@@ -521,8 +540,117 @@ int set_sweep_attributes()
             CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
             CU(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         }
+    for (int xd = 0; xd < 2; xd++)
+        for (int per = 0; per < 2; per++)
+            for (int LL : {4, 8, 16, 32})
+                for (int nR = 2; nR <= kMaxNRreg; nR++) {
+                    void *k = xd ? line_kernel_x(per != 0, nR, LL) : line_kernel_yz(per != 0, nR, LL);
+                    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+                }
     CU(cudaFuncSetAttribute((const void *)k_assemble3d_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)pw_smem_bytes(kPwStages)));
+    return GATT_OK;
+}
+
+void invalidate_graphs(gatt_ctx *c)
+{
+    if (c->stream && (c->graph[0] || c->graph[1])) cudaStreamSynchronize(c->stream);
+    for (int i = 0; i < 2; i++) {
+        if (c->graph[i]) cudaGraphExecDestroy(c->graph[i]);
+        c->graph[i] = nullptr;
+    }
+}
+
+// Row records (sweep.cuh) of type t for N rows -- rows past the line's are identity rows -- cut
+// into P blocks: the reference's factors in uniform row semantics and the block propagators.
+void type_records(const DevDir &m, int t, int N, int P, double *q)
+{
+    const int N0 = m.N;
+    const bool periodic = m.periodic != 0;
+    const double *tA = &m.hA[(size_t)t * N0], *tB = &m.hB[(size_t)t * N0], *tC = &m.hC[(size_t)t * N0];
+    for (int r = 0; r < N; r++) {
+        double *qr = q + (size_t)r * kQ;
+        if (r >= N0) {  // padding: x = 0 whatever comes before or after
+            qr[kQfB] = 1.0;
+            continue;
+        }
+        if (!periodic) {
+            qr[kQfA] = r > 0 ? tA[r - 1] : 0.0;       // derivs.F90:607
+            qr[kQfB] = tB[r];
+            qr[kQbC] = r < N0 - 1 ? tC[r] : 0.0;      // derivs.F90:610
+        } else {
+            qr[kQfA] = r >= 2 ? tA[r - 1] : 0.0;      // derivs.F90:798
+            qr[kQfB] = r >= 1 ? tB[r - 1] : 0.0;      // derivs.F90:796-798
+            qr[kQbC] = (r >= 1 && r <= N0 - 2) ? tC[r] : 0.0;  // derivs.F90:801
+            qr[kQD] = m.hD[(size_t)t * N0 + r];       // derivs.F90:786-789
+        }
+    }
+    if (periodic) { q[kQcA] = tA[0]; q[kQcC] = tC[0]; }  // derivs.F90:792-793
+    for (int p = 0; p < P; p++) {
+        const int s0 = block_start(p, N, P), e0 = block_start(p + 1, N, P) - 1;
+        const int rs = (periodic && p == 0) ? 1 : s0;
+        long double prod = 1.0L;
+        for (int r = rs; r <= e0; r++) {
+            prod *= -(long double)q[(size_t)r * kQ + kQfA] * (long double)q[(size_t)r * kQ + kQfB];
+            q[(size_t)r * kQ + kQpi] = (double)prod;
+        }
+        prod = 1.0L;
+        for (int r = e0; r >= rs; r--) {
+            prod *= -(long double)q[(size_t)r * kQ + kQbC];
+            q[(size_t)r * kQ + kQrho] = (double)prod;
+        }
+    }
+}
+
+// Coefficients of the any-length solver (lsweep.cuh): compact records of 16-row blocks, the most
+// frequent band as the uniform one, the blocks with other rows apart.
+int upload_line_records(gatt_ctx *c, DevDir &m)
+{
+    const int N = m.N, P = (N + kLineRows - 1) / kLineRows, rows = P * kLineRows, W = m.W;
+    const int td = line_type_doubles(P), bd = line_band_doubles(m.Wp);
+    auto band_of = [&](int t, int r) { return &m.hR[((size_t)t * N + r) * W]; };
+    std::map<std::vector<double>, int> count;
+    std::vector<double> common;
+    int most = 0;
+    for (int t = 0; t < m.nTypes; t++)
+        for (int r = 0; r < N; r++) {
+            const std::vector<double> b(band_of(t, r), band_of(t, r) + W);
+            const int n = ++count[b];
+            if (n > most) { most = n; common = b; }
+        }
+    std::vector<double> hQ((size_t)m.nTypes * td, 0.0), rec((size_t)rows * kQ), hS;
+    std::vector<int> hB((size_t)m.nTypes * P, -1);
+    m.nspecial = 0;
+    for (int t = 0; t < m.nTypes; t++) {
+        std::fill(rec.begin(), rec.end(), 0.0);
+        type_records(m, t, rows, P, rec.data());
+        double *q = &hQ[(size_t)t * td];
+        for (int r = 0; r < rows; r++)
+            for (int k = 0; k < kLineQ; k++) q[r * kLineQ + r / kLineRows * 2 + k] = rec[(size_t)r * kQ + k];
+        q[td - 2] = rec[kQcA];
+        q[td - 1] = rec[kQcC];
+        for (int p = 0; p < P; p++) {
+            bool same = true;
+            for (int r = p * kLineRows; r < std::min(N, (p + 1) * kLineRows); r++)
+                for (int k = 0; k < W; k++) same = same && band_of(t, r)[k] == common[k];
+            if (same) continue;
+            hB[(size_t)t * P + p] = m.nspecial++;
+            hS.resize((size_t)m.nspecial * bd, 0.0);
+            for (int r = p * kLineRows; r < std::min(N, (p + 1) * kLineRows); r++)
+                for (int k = 0; k < W; k++) hS[(size_t)(m.nspecial - 1) * bd + (r - p * kLineRows) * m.Wp + k] = band_of(t, r)[k];
+        }
+    }
+    memset(m.lband, 0, sizeof(m.lband));
+    memcpy(m.lband, common.data(), sizeof(double) * W);
+    m.lP = P;
+    const size_t nQ = hQ.size(), nS = hS.size();
+    hQ.insert(hQ.end(), hS.begin(), hS.end());
+    hQ.resize(nQ + nS + (hB.size() + 1) / 2, 0.0);
+    memcpy(&hQ[nQ + nS], hB.data(), hB.size() * sizeof(int));
+    CU(cudaMalloc(&m.lQ, hQ.size() * sizeof(double)));
+    CU(cudaMemcpy(m.lQ, hQ.data(), hQ.size() * sizeof(double), cudaMemcpyHostToDevice));
+    m.lS = m.lQ + nQ;
+    m.lB = reinterpret_cast<int *>(m.lQ + nQ + nS);
     return GATT_OK;
 }
 
@@ -534,44 +662,11 @@ int upload_records(gatt_ctx *c, DevDir &m, int P, int rows = 0)
     const int N0 = m.N, W = m.W, Wp = m.Wp, nTypes = m.nTypes;
     const int N = rows > 0 ? rows : N0;  // records for N rows: rows past N0 are identity rows
     const bool periodic = m.periodic != 0;
-    if (N != N0 && periodic) return fail(GATT_ERR_STATE, "cyclic lines cannot be padded");
     std::vector<double> hRm((size_t)nTypes * N * Wp, 0.0), hQ((size_t)nTypes * N * kQ, 0.0);
     for (int t = 0; t < nTypes; t++) {
-        const double *tA = &m.hA[(size_t)t * N0], *tB = &m.hB[(size_t)t * N0], *tC = &m.hC[(size_t)t * N0];
-        double *q = &hQ[(size_t)t * N * kQ];
-        for (int r = 0; r < N; r++) {
-            double *qr = q + (size_t)r * kQ;
-            if (r >= N0) {  // padding: x = 0 whatever comes before or after
-                qr[kQfB] = 1.0;
-                continue;
-            }
-            if (!periodic) {
-                qr[kQfA] = r > 0 ? tA[r - 1] : 0.0;       // derivs.F90:607
-                qr[kQfB] = tB[r];
-                qr[kQbC] = r < N0 - 1 ? tC[r] : 0.0;      // derivs.F90:610
-            } else {
-                qr[kQfA] = r >= 2 ? tA[r - 1] : 0.0;      // derivs.F90:798
-                qr[kQfB] = r >= 1 ? tB[r - 1] : 0.0;      // derivs.F90:796-798
-                qr[kQbC] = (r >= 1 && r <= N - 2) ? tC[r] : 0.0;  // derivs.F90:801
-                qr[kQD] = m.hD[(size_t)t * N + r];        // derivs.F90:786-789
-            }
+        type_records(m, t, N, P, &hQ[(size_t)t * N * kQ]);
+        for (int r = 0; r < std::min(N, N0); r++)
             for (int k = 0; k < W; k++) hRm[((size_t)t * N + r) * Wp + k] = m.hR[((size_t)t * N0 + r) * W + k];
-        }
-        if (periodic) { q[kQcA] = tA[0]; q[kQcC] = tC[0]; }  // derivs.F90:792-793
-        for (int p = 0; p < P; p++) {
-            const int s0 = block_start(p, N, P), e0 = block_start(p + 1, N, P) - 1;
-            const int rs = (periodic && p == 0) ? 1 : s0;
-            long double prod = 1.0L;
-            for (int r = rs; r <= e0; r++) {
-                prod *= -(long double)q[(size_t)r * kQ + kQfA] * (long double)q[(size_t)r * kQ + kQfB];
-                q[(size_t)r * kQ + kQpi] = (double)prod;
-            }
-            prod = 1.0L;
-            for (int r = e0; r >= rs; r--) {
-                prod *= -(long double)q[(size_t)r * kQ + kQbC];
-                q[(size_t)r * kQ + kQrho] = (double)prod;
-            }
-        }
     }
     // uniform band: cyclic, one type, every row's band equal to row 0's
     m.uband = periodic && nTypes == 1 && W <= 16 && N == N0;
@@ -585,8 +680,15 @@ int upload_records(gatt_ctx *c, DevDir &m, int P, int rows = 0)
         m.cac[1] = m.hC[0];
     }
     TRY(sync_stream(c));
-    if (!m.Rm) CU(cudaMalloc(&m.Rm, hRm.size() * sizeof(double)));
-    if (!m.Q) CU(cudaMalloc(&m.Q, hQ.size() * sizeof(double)));
+    if (m.cap < N) {
+        cudaFree(m.Rm); m.Rm = nullptr;
+        cudaFree(m.Q); m.Q = nullptr;
+        m.cap = 0;
+        CU(cudaMalloc(&m.Rm, hRm.size() * sizeof(double)));
+        CU(cudaMalloc(&m.Q, hQ.size() * sizeof(double)));
+        m.cap = N;
+        invalidate_graphs(c);  // graphs hold the record pointers
+    }
     CU(cudaMemcpy(m.Rm, hRm.data(), hRm.size() * sizeof(double), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(m.Q, hQ.data(), hQ.size() * sizeof(double), cudaMemcpyHostToDevice));
     m.P = P;
@@ -710,6 +812,104 @@ int launch_psweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nmember
     return after_launch(c);
 }
 
+// Tile width, ring depth and staged coefficients of a k_lsweep launch of nf fields and nmem
+// members.
+struct LinePlan {
+    int LL = 0, nst = 1, per_sm = 0;
+    long long jobs = 0;
+    bool stageS = false;
+    size_t smem = 0;
+    void *kernel = nullptr;
+};
+
+long long line_tiles(const gatt_ctx *c, int d, int LL)
+{
+    return d == 0 ? (nlines(c, 0) + LL - 1) / LL : (long long)((c->nx + LL - 1) / LL) * (d == 1 ? c->nz : c->ny);
+}
+
+constexpr size_t kLineBandBytes = 24 * 1024;  // non-uniform band rows that are staged
+
+// The plan of LL-line tiles with the shortest estimated time over ring depth and staged band
+// rows: rounds of resident CTAs, each a tile's latency (about that of 16 warps' issue) plus the
+// issue of the warps that share an SM.  LL = 0 in the result: does not fit.
+LinePlan line_plan_for(const gatt_ctx *c, const DevDir &m, int d, int nf, int nmem, int LL)
+{
+    const bool xd = d == 0;
+    LinePlan best;
+    if (!line_fits(xd, m.N, m.nR, LL)) return best;
+    double best_cost = 0;
+    LinePlan pl;
+    pl.LL = LL;
+    pl.jobs = line_tiles(c, d, LL) * nf * nmem;
+    pl.kernel = xd ? line_kernel_x(m.periodic != 0, m.nR, LL) : line_kernel_yz(m.periodic != 0, m.nR, LL);
+    const int warps = (m.lP * LL + 31) / 32;
+    const bool S = m.nspecial > 0 && (size_t)m.nspecial * line_band_doubles(m.Wp) * sizeof(double) <= kLineBandBytes;
+    for (int v = S ? 0 : 2; v < 4; v++) {
+        pl.nst = v & 1 ? 1 : 2;
+        pl.stageS = v < 2;
+        pl.smem = line_smem_bytes(xd, m.N, m.lP, LL, pl.nst, m.nspecial, m.Wp, pl.stageS);
+        if (pl.smem > kMaxSmem) continue;
+        pl.per_sm = resident_ctas(pl.kernel, 32 * warps, pl.smem);
+        if (pl.per_sm < 1) continue;
+        const long long at_once = (long long)pl.per_sm * c->nsm;
+        const double rounds = (double)((pl.jobs + at_once - 1) / at_once);
+        const double shared = (double)std::min<long long>(pl.per_sm, (pl.jobs + c->nsm - 1) / c->nsm);
+        const double cost = rounds * (1.0 + (pl.nst == 1 && rounds > 1 ? 0.4 : 0.0) + shared * warps / 16.0) *
+                            (m.nspecial > 0 && !pl.stageS ? 1.05 : 1.0);
+        if (!best.LL || cost < best_cost) { best = pl; best_cost = cost; }
+    }
+    return best;
+}
+
+// Tile width.  Wide tiles read the records at one address a warp instead of 32/LL, narrow ones
+// make more and smaller CTAs: 32 lines where they fill the SMs (y lines of the 90x75x54 box: 15.4
+// us against 18.5 with 16 and 20.8 with 8), fewer for launches that would leave SMs idle, and 8
+// for lines of 20 blocks and more, whose wide CTAs hold an SM alone (400-point x lines of the
+// plate boundary layer: 118 us against 137 with 16).  4 where 8-line tiles just miss one round
+// (800-point x lines, 152 tiles on 148 SMs: 21.7 us against 28.9).
+LinePlan line_plan(const gatt_ctx *c, const DevDir &m, int d, int nf, int nmem)
+{
+    const char *e = getenv("GATT_LINES");  // 4, 8, 16 or 32 lines a tile, where they fit
+    if (e) {
+        const LinePlan pl = line_plan_for(c, m, d, nf, nmem, atoi(e) == 4 || atoi(e) == 16 || atoi(e) == 32 ? atoi(e) : 8);
+        if (pl.LL) return pl;
+    }
+    if (m.lP < 20)
+        for (int LL : {32, 16}) {
+            const LinePlan pl = line_plan_for(c, m, d, nf, nmem, LL);
+            if (pl.LL && pl.jobs >= c->nsm) return pl;
+        }
+    const LinePlan pl = line_plan_for(c, m, d, nf, nmem, 8), half = line_plan_for(c, m, d, nf, nmem, 4);
+    const long long at_once = (long long)pl.per_sm * c->nsm;
+    if (half.LL && (!pl.LL || (pl.jobs > at_once && pl.jobs < 2 * at_once && half.jobs <= (long long)half.per_sm * c->nsm)))
+        return half;
+    return pl;
+}
+
+int launch_lsweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nf, int nmem, int cls)
+{
+    const LinePlan pl = line_plan(c, m, d, nf, nmem);
+    if (!pl.LL || pl.jobs > INT_MAX / 2) return GATT_ERR_STATE;
+    a.P = m.lP;
+    a.nst = pl.nst;
+    a.tiles_per_row = (c->nx + pl.LL - 1) / pl.LL;
+    a.fd_tpr = make_fastdiv(a.tiles_per_row);
+    a.ntiles = (int)line_tiles(c, d, pl.LL);
+    a.njobs = (int)pl.jobs;
+    LineArgs la;
+    memset(&la, 0, sizeof(la));
+    la.Q = m.lQ; la.S = m.lS; la.blk = m.lB;
+    la.nspecial = m.nspecial;
+    la.stageS = pl.stageS;
+    memcpy(la.band, m.lband, sizeof(la.band));
+    la.fd_ntiles = make_fastdiv(a.ntiles); la.fd_nf = make_fastdiv(nf);
+    const int grid = (int)std::min<long long>(pl.jobs, (long long)pl.per_sm * c->nsm);
+    void *args[] = {&a, &la};
+    TRY(before_launch(c, cls));
+    CU(cudaLaunchKernel(pl.kernel, dim3(grid), dim3((m.lP * pl.LL + 31) / 32 * 32), args, pl.smem, c->stream));
+    return after_launch(c);
+}
+
 // Run one compact solve (direction d, coefficient kind) over nf fields.
 // in/out are set bases with per-member strides; slots index fields inside a set.
 // blend_dt: device dt for the filter blend (NULL = use `blend`).
@@ -743,6 +943,13 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
     a.ntypes = m.nTypes;
     if (mc_ref && d > 0) {  // the max-change epilogue: only the pipelined y/z solver has it
         a.mc_acc = c->acc; a.mc_ref = mc_ref->v[0]; a.mc_ref_bstride = mc_ref->bstride;
+    }
+    // lines of many blocks whose 32-line tiles leave SMs idle (the 300-point y lines of the 800x300
+    // grid: 100 tiles of 19 blocks, 13.3 us against 15.3) run as 8-line tiles too
+    const bool few = m.family == FAM_PIPE && m.lQ && m.P >= 16 && (long long)a.njobs < c->nsm && !mc_ref;
+    if (m.family == FAM_LINE || few) {
+        const int r = launch_lsweep(c, m, d, a, nf, nmembers, cls);
+        if (r != GATT_ERR_STATE) return r;  // GATT_ERR_STATE: more tiles than a launch counts
     }
     if (m.family == FAM_PIPE && m.rpb) {
         int r = launch_psweep(c, m, d, a, nmembers, cls);
@@ -1073,6 +1280,41 @@ struct HostBcOp {
     std::vector<Acc> rd, wr;
 };
 
+typedef std::array<int, 6> BcBox;
+
+bool box_and(const BcBox &a, const BcBox &b, BcBox &out)
+{
+    for (int q = 0; q < 6; q += 2) {
+        out[q] = std::max(a[q], b[q]);
+        out[q + 1] = std::min(a[q + 1], b[q + 1]);
+        if (out[q] > out[q + 1]) return false;
+    }
+    return true;
+}
+
+// The points of b that no box of `cover` holds, as disjoint boxes.
+std::vector<BcBox> box_minus(const BcBox &b, const std::vector<BcBox> &cover)
+{
+    std::vector<BcBox> left{b};
+    for (const BcBox &c : cover) {
+        std::vector<BcBox> next;
+        for (BcBox r : left) {
+            BcBox in;
+            if (!box_and(r, c, in)) { next.push_back(r); continue; }
+            for (int q = 4; q >= 0; q -= 2) {  // the slabs of r outside `in`, z first (long rows)
+                BcBox s = r;
+                if (r[q] < in[q]) { s[q + 1] = in[q] - 1; next.push_back(s); }
+                s = r;
+                if (in[q + 1] < r[q + 1]) { s[q] = in[q + 1] + 1; next.push_back(s); }
+                r[q] = in[q];
+                r[q + 1] = in[q + 1];
+            }
+        }
+        left.swap(next);
+    }
+    return left;
+}
+
 bool bc_overlap(const std::vector<HostBcOp::Acc> &x, const std::vector<HostBcOp::Acc> &y)
 {
     for (const auto &a : x)
@@ -1193,19 +1435,35 @@ int build_bc_program(gatt_ctx *c)
     const int NL = (int)c->coef1.size(), N2 = (int)c->coef2.size();
     const int order[4] = {GATT_VAR_U, GATT_VAR_V, GATT_VAR_W, GATT_VAR_E};
     int box[6], ext[6], rd[6];
-    // Dirichlet (nseq.F90:357-373)
-    for (int v : order) {
+    // Dirichlet (nseq.F90:357-373): within a list later boxes win, so each keeps the points that
+    // no later one covers, and the lists need one level each; the pressure list, which comes
+    // last, is a constant density where E is one
+    std::vector<std::pair<BcBox, double>> fixed[5];
+    for (int v : {GATT_VAR_U, GATT_VAR_V, GATT_VAR_W, GATT_VAR_E, GATT_VAR_R}) {
         const HostBC &h = c->bc[GATT_BC_DIRICHLET][v];
-        for (int i = 0; i < h.n; i++) {
+        std::vector<BcBox> over;
+        for (int i = h.n - 1; i >= 0; i--) {
             row(h, i, box); TRY(check_box(c, box));
-            HostBcOp o = mk(OP_SET, v, box); o.op.val = h.val[i]; both(o, 0, 1u << v);
+            const BcBox bx = {box[0], box[1], box[2], box[3], box[4], box[5]};
+            for (const BcBox &piece : box_minus(bx, over)) fixed[v].push_back({piece, h.val[i]});
+            over.push_back(bx);
         }
     }
-    {
-        const HostBC &h = c->bc[GATT_BC_DIRICHLET][GATT_VAR_R];
-        for (int i = 0; i < h.n; i++) {
-            row(h, i, box); TRY(check_box(c, box));
-            HostBcOp o = mk(OP_DIR_P, GATT_VAR_R, box); o.op.val = h.val[i]; both(o, E, R);
+    for (int v : order)
+        for (const auto &f : fixed[v]) {
+            HostBcOp o = mk(OP_SET, v, f.first.data()); o.op.val = f.second; both(o, 0, 1u << v);
+        }
+    for (const auto &f : fixed[GATT_VAR_R]) {
+        std::vector<BcBox> constant;
+        for (const auto &e : fixed[GATT_VAR_E]) {
+            BcBox in;
+            if (!box_and(f.first, e.first, in)) continue;
+            constant.push_back(in);
+            HostBcOp o = mk(OP_SET, GATT_VAR_R, in.data()); o.op.val = f.second / (c->ph.gamma - 1.0) / e.second;
+            both(o, 0, R);
+        }
+        for (const BcBox &piece : box_minus(f.first, constant)) {
+            HostBcOp o = mk(OP_DIR_P, GATT_VAR_R, piece.data()); o.op.val = f.second; both(o, E, R);
         }
     }
     // P <- its extrapolation along dir at the face of box (P loaded over ext before)
@@ -1369,7 +1627,9 @@ BcProgram bc_program(const gatt_ctx *c, double tfac, int form = 0)
 {
     const gatt_ctx::BcDev &d = c->d_prog[form];
     BcProgram pg;
-    pg.ops = d.ops; pg.lev = d.lev; pg.nops = d.nops; pg.nlev = d.nlev; pg.coef1 = c->d_coef1; pg.coef2 = c->d_coef2; pg.xs = c->d_xs;
+    pg.ops = d.ops; pg.lev = d.lev; pg.nops = d.nops; pg.nlev = d.nlev;
+    pg.n1 = (int)c->coef1.size(); pg.n2 = (int)c->coef2.size();
+    pg.coef1 = c->d_coef1; pg.coef2 = c->d_coef2; pg.xs = c->d_xs;
     pg.gamma = c->ph.gamma; pg.nx = c->nx; pg.ny = c->ny; pg.nz = c->nz;
     pg.sp = c->d_params; pg.tfac = tfac; pg.tfix = 0.0;
     pg.hold = c->d_hold; pg.hstride = c->hold_len; pg.hold_save = 0;
@@ -1386,24 +1646,15 @@ int check_hold(gatt_ctx *c)
     return GATT_OK;
 }
 
-void invalidate_graphs(gatt_ctx *c)
-{
-    if (c->stream && (c->graph[0] || c->graph[1])) cudaStreamSynchronize(c->stream);
-    for (int i = 0; i < 2; i++) {
-        if (c->graph[i]) cudaGraphExecDestroy(c->graph[i]);
-        c->graph[i] = nullptr;
-    }
-}
-
 // Cluster size for a boundary-program kernel: 16 CTAs (non-portable size) when the GPU can
-// schedule such a cluster of 512-thread CTAs, else 8, else 0 (one CTA per member).
+// schedule such a cluster, else 8, else 0 (one CTA per member).
 int bc_cluster_size(const void *k)
 {
     if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
     for (int cs : {16, 8}) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(512);
+        cfg.blockDim = dim3(kBcThreads);
         cfg.dynamicSmemBytes = 48 * 1024;  // the staged ops, at most
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1443,7 +1694,7 @@ int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...),
               Args &&...args)
 {
     const gatt_ctx::BcDev &d = c->d_prog[form];
-    const size_t need = bc_stage_bytes(d.nops, d.nlev), smem = need <= (size_t)kBcStagedBytes ? need : 0;
+    const size_t need = bc_stage_bytes(bc_program(c, 0.0, form)), smem = need <= (size_t)kBcStagedBytes ? need : 0;
     const long long by_work = (d.widest + 2047) / 2048;
     const long long by_sms = std::max(1, c->nsm / std::max(1, nmem));
     int cs = 1;
@@ -1451,7 +1702,7 @@ int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...),
     if (cs >= 2) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(nmem * cs);
-        cfg.blockDim = dim3(512);
+        cfg.blockDim = dim3(kBcThreads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = c->stream;
         cudaLaunchAttribute at[1];
@@ -1463,7 +1714,7 @@ int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...),
         cfg.numAttrs = 1;
         CU(cudaLaunchKernelEx(&cfg, kcluster, std::forward<Args>(args)...));
     } else {
-        kblock<<<nmem, 512, smem, c->stream>>>(std::forward<Args>(args)...);
+        kblock<<<nmem, kBcThreads, smem, c->stream>>>(std::forward<Args>(args)...);
     }
     return GATT_OK;
 }
@@ -2408,7 +2659,7 @@ int vjp(gatt_ctx *c, int nsteps, double t0, double dt, int every, const double *
 // ---------------------------------------------------------------------------
 
 // Candidates for a matrix set: the two register-resident families (16-row blocks) where the
-// line length allows them, and the shared-tile solver at 8, 16, 32 and 64 rows per block.
+// line length allows them, the any-length one, and the shared-tile solver at 8, 16, 32 and 64 rows per block.
 struct TuneCand {
     int family, rpb, P;
 };
@@ -2422,6 +2673,7 @@ std::vector<TuneCand> tune_candidates(const DevDir &m)
     } else if (m.Np > m.N || (m.N % kRPB == 0 && m.N / kRPB > kMaxP && m.family == FAM_PIPE && m.rpb)) {
         out.push_back({FAM_PIPE, kRPB, m.Np / kRPB});  // padded or long lines: the pipelined solver only
     }
+    if (m.lQ) out.push_back({FAM_LINE, 0, choose_blocks(m.N, m.nR, m.Wp)});  // (records of its own)
     for (int rows : {8, 16, 32, 64}) {
         const int P = choose_blocks(m.N, m.nR, m.Wp, rows);
         bool dup = false;
@@ -2457,6 +2709,8 @@ int autotune(gatt_ctx *c, int reps, int *family, int *blocks, double *us)
             if (d >= ndir || !m.set || m.N < 2) continue;
             TuneCand best{m.family, m.rpb, m.P};
             float best_ms = -1.0f;
+            if (!m.lQ && line_fits(d == 0, m.N, m.nR, 8)) rc = upload_line_records(c, m);
+            if (rc != GATT_OK) break;
             for (const TuneCand &t : tune_candidates(m)) {
                 m.family = t.family; m.rpb = t.rpb;
                 rc = upload_records(c, m, t.P, t.rpb ? t.P * t.rpb : m.N);
@@ -2477,8 +2731,8 @@ int autotune(gatt_ctx *c, int reps, int *family, int *blocks, double *us)
             if (rc != GATT_OK) break;
             m.family = best.family; m.rpb = best.rpb;
             rc = upload_records(c, m, best.P, best.rpb ? best.P * best.rpb : m.N);
-            if (family) family[slot] = best.family;
-            if (blocks) blocks[slot] = best.P;
+            if (family) family[slot] = best.family == FAM_LINE ? (int)FAM_REG : best.family;
+            if (blocks) blocks[slot] = best.family == FAM_LINE ? m.lP : best.P;
             if (us) us[slot] = 1e3 * best_ms;
         }
     cudaEventDestroy(e0);
@@ -2600,8 +2854,7 @@ void gatt_destroy(gatt_ctx *c)
     for (int d = 0; d < 3; d++) {
         for (int k = 0; k < kMatKinds; k++) {
             DevDir &m = c->mat[d][k];
-            cudaFree(m.Rm);
-            cudaFree(m.Q);
+            for (void *q : {(void *)m.Rm, (void *)m.Q, (void *)m.lQ}) cudaFree(q);
         }
         cudaFree(c->ltype[d]);
     }
@@ -2652,6 +2905,7 @@ int gatt_set_physics(gatt_ctx *c, double Re, double Ma, double Pr, double gamma,
         if (!std::isfinite(x) || x <= 0) return fail(GATT_ERR_BADARG, "physical parameters must be positive and finite");
     if (gamma <= 1) return fail(GATT_ERR_BADARG, "gamma must exceed 1");
     c->ph.Re = Re; c->ph.Ma = Ma; c->ph.Pr = Pr; c->ph.gamma = gamma; c->ph.T0 = T0;
+    c->bc_dirty = true;  // the program holds densities formed with gamma
     c->phys_set = true;
     invalidate_graphs(c);
     return GATT_OK;
@@ -2726,20 +2980,24 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
         for (uint8_t t : cur)
             if (t >= nTypes) return fail(GATT_ERR_BADARG, "existing block types exceed nTypes");
     }
-    const int Np = padded_rows(c, d, N, nRHS, periodic);
-    const int rpb = choose_rpb(d, N, Np, nRHS, nTypes, (W + 3) / 4 * 4);
+    int Np = padded_rows(c, d, N, nRHS, periodic);
+    int rpb = choose_rpb(d, N, Np, nRHS, nTypes, (W + 3) / 4 * 4);
+    const int want = choose_family();
+    const bool line = (want == FAM_LINE || (want == FAM_PIPE && !rpb)) && line_fits(d == 0, N, nRHS, 8);
+    const int Npipe = rpb ? Np : N;  // a padded length the pipelined solver does not take is not kept
+    if (line) { rpb = 0; Np = N; }  // (its records are its own; the others are the shared-tile solver's)
     const int P = rpb ? Np / rpb : choose_blocks(N, nRHS, (W + 3) / 4 * 4);
     TRY(sync_stream(c));
     DevDir &m = c->mat[d][kind];
-    cudaFree(m.Rm);
-    cudaFree(m.Q);
+    for (void *q : {(void *)m.Rm, (void *)m.Q, (void *)m.lQ}) cudaFree(q);
     m = DevDir();
     m.periodic = periodic; m.nR = nRHS; m.nTypes = nTypes; m.N = N; m.W = W; m.Wp = (W + 3) / 4 * 4;
     m.hA = std::move(hA); m.hB = std::move(hB); m.hC = std::move(hC); m.hD = std::move(hD); m.hR = std::move(hR);
-    m.Np = rpb ? Np : N;  // a padded length the solver does not take is not kept
+    m.Np = Npipe;
     TRY(upload_records(c, m, P, rpb ? Np : N));
+    if (line || (rpb && P >= 16 && line_fits(d == 0, N, nRHS, 8))) TRY(upload_line_records(c, m));
     m.rpb = rpb;
-    m.family = rpb ? choose_family() : FAM_TILE;
+    m.family = line ? FAM_LINE : rpb ? (want == FAM_LINE ? FAM_PIPE : want) : FAM_TILE;
     m.set = true;
     if (nBlocks > 0) {
         if (!c->ltype[d]) CU(cudaMalloc(&c->ltype[d], lt.size()));
