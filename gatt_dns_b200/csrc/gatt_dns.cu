@@ -216,6 +216,7 @@ struct gatt_ctx {
     int time_stepping = 1;  // parameters.F90 timeStepping: 1 RK4, 2 Euler, 3 SSPRK3
     Forcings fc{};          // runForcings (fc.n = 0: none); boxes 0-based
     double *fsum = nullptr, *fpart = nullptr;  // turbulence box sums, per-CTA partials
+    unsigned *fdone = nullptr;  // CTAs that have finished, per member (zero between launches)
     int fblocks = 0;        // CTAs of the sums kernel (fixed: the sums do not depend on timing)
     bool fork_x = true;     // x sweeps beside the y/z sweeps, filter field chains side by side
                             // (GATT_FORK_X=0: everything on one stream)
@@ -1084,10 +1085,7 @@ int forcing_sums(gatt_ctx *c, const StateSet &q, int nmem)
     for (int f = 0; f < c->fc.n; f++) turb |= c->fc.type[f] == FORCE_TURBULENCE;
     if (!turb) return GATT_OK;
     TRY(before_launch(c, PC_OTHER));
-    k_forcing_sums<<<dim3(c->fblocks, nmem), 256, 0, c->stream>>>(q, forcing_args(c), c->fpart);
-    TRY(after_launch(c));
-    TRY(before_launch(c, PC_OTHER));
-    k_forcing_final<<<nmem, 32, 0, c->stream>>>(c->fpart, c->fblocks, c->fsum);
+    k_forcing_sums<<<dim3(c->fblocks, nmem), 256, 0, c->stream>>>(q, forcing_args(c), c->fpart, c->fdone, c->fsum);
     return after_launch(c);
 }
 
@@ -2872,7 +2870,7 @@ void gatt_destroy(gatt_ctx *c)
     for (double *p : bufs) cudaFree(p);
     for (gatt_ctx::BcDev &d : c->d_prog) { cudaFree(d.ops); cudaFree(d.lev); }
     cudaFree(c->acc); cudaFree(c->d_params);
-    cudaFree(c->fsum); cudaFree(c->fpart);
+    cudaFree(c->fsum); cudaFree(c->fpart); cudaFree(c->fdone);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_err) cudaFreeHost(c->h_err);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -3121,6 +3119,8 @@ int gatt_add_forcing(gatt_ctx *c, int type, const int *ind, int npar, const doub
             return fail(GATT_ERR_BADARG, "forcing box outside the grid");
     if (!c->fsum) {
         c->fblocks = 2 * c->nsm;
+        if (!c->fdone) CU(cudaMalloc(&c->fdone, sizeof(unsigned) * (size_t)c->nb));
+        CU(cudaMemsetAsync(c->fdone, 0, sizeof(unsigned) * (size_t)c->nb, c->stream));
         CU(cudaMalloc(&c->fsum, sizeof(double) * (size_t)c->nb * kMaxForcings * 5));
         CU(cudaMalloc(&c->fpart, sizeof(double) * (size_t)c->nb * kMaxForcings * c->fblocks * 5));
     }

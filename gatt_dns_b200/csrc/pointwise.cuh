@@ -108,25 +108,29 @@ struct StateSet {
     long long bstride;
 };
 
-// Box sums of every turbulence forcing: each CTA (blockIdx.x of gridDim.x, member
-// blockIdx.y) sums its grid-stride share of the box points in a fixed order into
-// part[((b * kMaxForcings + f) * gridDim.x + cta) * 5 + q]; k_forcing_final adds the CTAs'
-// partials in CTA order, so the sums do not depend on timing.
-__global__ void __launch_bounds__(256) k_forcing_sums(StateSet q, Forcings fs, double *part)
+// Box sums of every turbulence forcing: each CTA (blockIdx.x of gridDim.x, member blockIdx.y)
+// sums its grid-stride share of the box points in a fixed order into
+// part[((b * kMaxForcings + f) * gridDim.x + cta) * 5 + q]; the member's last CTA to finish adds
+// the partials, lane by lane in CTA order and then over the lanes, so the sums do not depend on
+// timing.  done: one counter per member, zero between launches.
+// Latency-bound (64^3: 10 MB from L2): one launch of 7.5 us; a second launch whose threads added
+// the 296 partials one after the other took 39 us for the pair.
+__global__ void __launch_bounds__(256) k_forcing_sums(StateSet q, Forcings fs, double *part, unsigned *done, double *sums)
 {
-    __shared__ double red[5][256];
-    const int b = blockIdx.y;
+    __shared__ double red[5][8];
+    __shared__ bool last;
+    const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double *U = q.v[0] + b * q.bstride, *V = q.v[1] + b * q.bstride, *W = q.v[2] + b * q.bstride;
     const double *E = q.v[4] + b * q.bstride;
     for (int f = 0; f < fs.n; f++) {
         if (fs.type[f] != FORCE_TURBULENCE) continue;
         const int *bx = fs.box[f];
-        const long long ni = bx[1] - bx[0] + 1, nj = bx[3] - bx[2] + 1, nk = bx[5] - bx[4] + 1;
-        const long long m = ni * nj * nk;
+        const unsigned ni = bx[1] - bx[0] + 1, nj = bx[3] - bx[2] + 1, nk = bx[5] - bx[4] + 1, m = ni * nj * nk;
         double s[5] = {0, 0, 0, 0, 0};
-        for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < m; t += (long long)gridDim.x * blockDim.x) {
-            const long long i = bx[0] + t % ni, j = bx[2] + (t / ni) % nj, kz = bx[4] + t / (ni * nj);
-            const long long p = i + fs.nx * (j + (long long)fs.ny * kz);
+        for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
+            const unsigned jk = t / ni, kz = jk / nj;
+            const long long p = bx[0] + (long long)(t - jk * ni) +
+                                fs.nx * (bx[2] + (long long)(jk - kz * nj) + (long long)fs.ny * (bx[4] + (long long)kz));
             const double u = U[p], v = V[p], w = W[p];
             s[0] += u * u + v * v + w * w;
             s[1] += u;
@@ -134,31 +138,35 @@ __global__ void __launch_bounds__(256) k_forcing_sums(StateSet q, Forcings fs, d
             s[3] += w;
             s[4] += E[p];
         }
-        for (int c = 0; c < 5; c++) red[c][threadIdx.x] = s[c];
-        __syncthreads();
-        for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-            if ((int)threadIdx.x < h)
-                for (int c = 0; c < 5; c++) red[c][threadIdx.x] += red[c][threadIdx.x + h];
-            __syncthreads();
+#pragma unroll
+        for (int c = 0; c < 5; c++) {
+            for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+            if (lane == 0) red[c][warp] = s[c];
         }
-        if (threadIdx.x < 5)
-            part[(((size_t)b * kMaxForcings + f) * gridDim.x + blockIdx.x) * 5 + threadIdx.x] = red[threadIdx.x][0];
+        __syncthreads();
+        if (threadIdx.x < 5) {
+            double v = red[threadIdx.x][0];
+            for (int w = 1; w < 8; w++) v += red[threadIdx.x][w];
+            part[(((size_t)b * kMaxForcings + f) * gridDim.x + blockIdx.x) * 5 + threadIdx.x] = v;
+            __threadfence();
+        }
         __syncthreads();
     }
+    if (threadIdx.x == 0) last = atomicAdd(done + b, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int t = warp; t < kMaxForcings * 5; t += 8) {  // forcing t / 5, quantity t % 5
+        const int f = t / 5, qd = t % 5;
+        if (f >= fs.n || fs.type[f] != FORCE_TURBULENCE) continue;
+        const double *pp = part + ((size_t)b * kMaxForcings + f) * gridDim.x * 5 + qd;
+        double v = 0;
+        for (unsigned c = lane; c < gridDim.x; c += 32) v += __ldcg(pp + (size_t)c * 5);
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) sums[((size_t)b * kMaxForcings + f) * 5 + qd] = v;
+    }
+    if (threadIdx.x == 0) done[b] = 0;
 }
-
-__global__ void k_forcing_final(const double *part, int nblocks, double *sums)
-{
-    // one thread per (member, forcing, quantity): blockIdx.x = member
-    const int t = threadIdx.x;  // f * 5 + q
-    if (t >= kMaxForcings * 5) return;
-    const int f = t / 5, qd = t % 5;
-    const double *pp = part + ((size_t)blockIdx.x * kMaxForcings + f) * nblocks * 5 + qd;
-    double s = 0;
-    for (int c = 0; c < nblocks; c++) s += pp[(size_t)c * 5];
-    sums[((size_t)blockIdx.x * kMaxForcings + f) * 5 + qd] = s;
-}
-
 
 __device__ __forceinline__ double sutherland_mu(const Phys &ph, double E)
 {
