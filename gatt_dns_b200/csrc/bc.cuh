@@ -12,7 +12,8 @@
 // independent whatever their order, and every op finds the values that the reference's order
 // gives it.  The points of a level's ops form one index range spread over all threads; a
 // barrier separates the levels.  One CTA per batch member runs small programs (block barriers),
-// a cluster of up to 16 SMs the larger ones (cluster barriers, release/acquire).
+// a cluster of up to 16 SMs larger ones (cluster barriers, release/acquire); the widest take one
+// launch per level over the whole GPU.
 //
 // What bounds it: the chain of levels, about a microsecond each (a barrier, then dependent
 // loads that miss to L2).  The pressure Neumann items and the corners are therefore one op
@@ -182,26 +183,31 @@ __device__ __forceinline__ void bc_stage(BcProgram &pg, long long *sh)
     pg.coef2 = c2;
 }
 
-// fn(op, r, i, p) for every point of every level, thread tid of nthr: r the point's index in
-// the op's box (x fastest), i its x node, p its element offset; sync() (a barrier over all nthr
-// threads that orders their memory accesses) between levels.  REV: last level first.
+// fn(op, r, i, p) for every point of level lv, thread tid of nthr: r the point's index in the
+// op's box (x fastest), i its x node, p its element offset.  op: the level's first op.
+template <typename Fn>
+__device__ __forceinline__ void bc_level(const BcProgram &pg, const BcOp *op, unsigned total, int tid, int nthr, Fn fn)
+{
+    for (unsigned q = tid; q < total; q += nthr) {
+        while (q >= op->first + op->count) op++;
+        const unsigned r = q - op->first;
+        const unsigned kq = fdiv((int)r, op->fd_nij), rr = r - kq * op->fd_nij.d, jq = fdiv((int)rr, op->fd_ni);
+        const int i = op->box[0] + (int)(rr - jq * op->fd_ni.d);
+        const long long p = (long long)(i - 1) +
+                            (long long)pg.nx * ((op->box[2] - 1 + (int)jq) + (long long)pg.ny * (op->box[4] - 1 + (int)kq));
+        fn(*op, r, i, p);
+    }
+}
+
+// Every level; sync() (a barrier over all nthr threads that orders their memory accesses) between
+// levels.  REV: last level first.
 template <bool REV = false, typename Sync, typename Fn>
 __device__ __forceinline__ void bc_levels(const BcProgram &pg, int tid, int nthr, Sync sync, Fn fn)
 {
     for (int l = 0; l < pg.nlev; l++) {
         if (l) sync();
         const int lv = REV ? pg.nlev - 1 - l : l;
-        const unsigned total = pg.lev[pg.nlev + 1 + lv];
-        const BcOp *op = pg.ops + pg.lev[lv];
-        for (unsigned q = tid; q < total; q += nthr) {
-            while (q >= op->first + op->count) op++;
-            const unsigned r = q - op->first;
-            const unsigned kq = fdiv((int)r, op->fd_nij), rr = r - kq * op->fd_nij.d, jq = fdiv((int)rr, op->fd_ni);
-            const int i = op->box[0] + (int)(rr - jq * op->fd_ni.d);
-            const long long p = (long long)(i - 1) +
-                                (long long)pg.nx * ((op->box[2] - 1 + (int)jq) + (long long)pg.ny * (op->box[4] - 1 + (int)kq));
-            fn(*op, r, i, p);
-        }
+        bc_level(pg, pg.ops + pg.lev[lv], pg.lev[pg.nlev + 1 + lv], tid, nthr, fn);
     }
 }
 
@@ -214,57 +220,83 @@ struct BcFields {
     __device__ __forceinline__ double *operator[](int v) const { return s.v[v] + off; }
 };
 
-// The program on one member: F the five state arrays (U,V,W,R,E), P a scratch field.
+// One point of the program on one member: F the five state arrays (U,V,W,R,E), P a scratch
+// field, tnow the time of the call.
+__device__ __forceinline__ void bc_point(const BcProgram &pg, const BcFields &F, double *P, double *H, double tnow,
+                                         const BcOp &op, unsigned r, int i, long long p)
+{
+    double *Rr = F[3], *Ee = F[4];
+    const double *cf = op.coef ? pg.coef2 : pg.coef1;
+    switch (op.code) {
+    case OP_SET: F[op.var][p] = op.val; break;
+    case OP_DIR_P: Rr[p] = op.val / (pg.gamma - 1.0) / Ee[p]; break;
+    case OP_NEU: F[op.var][p] = bc_extrapolate(F[op.var] + p, op.step[0], op.len, cf); break;
+    case OP_PNEU: Rr[p] = bc_extrapolate_p(Rr + p, Ee + p, op.step[0], op.len, cf) / Ee[p]; break;
+    case OP_CORNER: {
+        if (op.var) {
+            double e = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                if (d < op.aux) e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
+            Ee[p] = e / (double)op.aux;
+        }
+        double v = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            if (d < op.aux) v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
+        Rr[p] = v / Ee[p] / (double)op.aux;
+        break;
+    }
+    case OP_P_LOAD: P[p] = Rr[p] * Ee[p]; break;
+    case OP_P_NEU: P[p] = bc_extrapolate(P + p, op.step[0], op.len, cf); break;
+    case OP_R_FROM_P: Rr[p] = P[p] / Ee[p]; break;
+    case OP_CORNER_E0: Ee[p] = 0.0; break;
+    case OP_P_FROM_E: P[p] = Ee[p]; break;
+    case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; break;
+    case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; break;
+    case OP_R0: Rr[p] = 0.0; break;
+    case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; break;
+    case OP_R_DIV_E: Rr[p] = Rr[p] / Ee[p] / (double)op.aux; break;
+    case OP_LID: F[op.var][p] = bc_lid(pg, op, i); break;
+    case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
+    case OP_HOLD:
+        for (int v = 0; v < op.aux; v++) {
+            double *h = H + op.xoff + (long long)v * op.count + r;
+            if (pg.hold_save) *h = F[bc_hold_field(v)][p];
+            else F[bc_hold_field(v)][p] = *h;
+        }
+        break;
+    default: break;
+    }
+}
+
+// The whole program on one member.
 template <typename Sync>
 __device__ __forceinline__ void bc_run(const BcProgram &pg, const BcFields &F, double *P, double *H, int tid, int nthr,
                                        Sync sync)
 {
-    double *Rr = F[3], *Ee = F[4];
     const double tnow = bc_time(pg);
-    bc_levels(pg, tid, nthr, sync, [&](const BcOp &op, unsigned r, int i, long long p) {
-        const double *cf = op.coef ? pg.coef2 : pg.coef1;
-        switch (op.code) {
-        case OP_SET: F[op.var][p] = op.val; break;
-        case OP_DIR_P: Rr[p] = op.val / (pg.gamma - 1.0) / Ee[p]; break;
-        case OP_NEU: F[op.var][p] = bc_extrapolate(F[op.var] + p, op.step[0], op.len, cf); break;
-        case OP_PNEU: Rr[p] = bc_extrapolate_p(Rr + p, Ee + p, op.step[0], op.len, cf) / Ee[p]; break;
-        case OP_CORNER: {
-            if (op.var) {
-                double e = 0.0;
-#pragma unroll
-                for (int d = 0; d < 3; d++)
-                    if (d < op.aux) e = e + bc_extrapolate(Ee + p, op.step[d], op.len, cf);
-                Ee[p] = e / (double)op.aux;
-            }
-            double v = 0.0;
-#pragma unroll
-            for (int d = 0; d < 3; d++)
-                if (d < op.aux) v = v + bc_extrapolate_p(Rr + p, Ee + p, op.step[d], op.len, cf);
-            Rr[p] = v / Ee[p] / (double)op.aux;
-            break;
-        }
-        case OP_P_LOAD: P[p] = Rr[p] * Ee[p]; break;
-        case OP_P_NEU: P[p] = bc_extrapolate(P + p, op.step[0], op.len, cf); break;
-        case OP_R_FROM_P: Rr[p] = P[p] / Ee[p]; break;
-        case OP_CORNER_E0: Ee[p] = 0.0; break;
-        case OP_P_FROM_E: P[p] = Ee[p]; break;
-        case OP_E_ADD_P: Ee[p] = Ee[p] + P[p]; break;
-        case OP_E_DIV: Ee[p] = Ee[p] / (double)op.aux; break;
-        case OP_R0: Rr[p] = 0.0; break;
-        case OP_R_ADD_P: Rr[p] = Rr[p] + P[p]; break;
-        case OP_R_DIV_E: Rr[p] = Rr[p] / Ee[p] / (double)op.aux; break;
-        case OP_LID: F[op.var][p] = bc_lid(pg, op, i); break;
-        case OP_SINE: F[op.var][p] = bc_sine(F[op.var][p], pg.xs[op.xoff + i - op.box[0]], op.val, tnow); break;
-        case OP_HOLD:
-            for (int v = 0; v < op.aux; v++) {
-                double *h = H + op.xoff + (long long)v * op.count + r;
-                if (pg.hold_save) *h = F[bc_hold_field(v)][p];
-                else F[bc_hold_field(v)][p] = *h;
-            }
-            break;
-        default: break;
-        }
-    });
+    bc_levels(pg, tid, nthr, sync,
+              [&](const BcOp &op, unsigned r, int i, long long p) { bc_point(pg, F, P, H, tnow, op, r, i, p); });
+}
+
+// One level over the whole grid (blockIdx.y: member); dynamic shared memory: the level's ops.
+__global__ void __launch_bounds__(256) k_bc_level(BcProgram pg, const __grid_constant__ StateSet q, double *Pbase,
+                                                  long long pstride, int lv, int op0, int nops, unsigned total)
+{
+    extern __shared__ long long bc_sh[];
+    pdl_launch();
+    const long long *g = reinterpret_cast<const long long *>(pg.ops + op0);
+    for (int i = threadIdx.x; i < nops * (int)(sizeof(BcOp) / sizeof(long long)); i += blockDim.x) bc_sh[i] = g[i];
+    __syncthreads();
+    pdl_wait();
+    const int b = blockIdx.y;
+    const BcFields F(q, b);
+    double *P = Pbase + b * pstride, *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
+    const double tnow = bc_time(pg);
+    bc_level(pg, reinterpret_cast<const BcOp *>(bc_sh), total, blockIdx.x * blockDim.x + threadIdx.x,
+             gridDim.x * blockDim.x,
+             [&](const BcOp &op, unsigned r, int i, long long p) { bc_point(pg, F, P, H, tnow, op, r, i, p); });
 }
 
 // One CTA per batch member (block barriers); dynamic shared memory: the staged program.
@@ -274,7 +306,9 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(BcProgram pg, const __grid_co
     extern __shared__ long long bc_sh[];
     const int b = blockIdx.x;
     const BcFields F(q, b);
-    bc_stage(pg, bc_sh);
+    pdl_launch();
+    bc_stage(pg, bc_sh);  // (the program does not depend on the launch before this one)
+    pdl_wait();
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
     bc_run(pg, F, Pbase + b * pstride, H, threadIdx.x, blockDim.x, [] { __syncthreads(); });
 }
@@ -288,7 +322,9 @@ __global__ void __launch_bounds__(kBcThreads) k_bc_cluster(BcProgram pg, const _
     const int b = blockIdx.x / (int)cl.num_blocks();
     const BcFields F(q, b);
     extern __shared__ long long bc_sh[];
-    bc_stage(pg, bc_sh);
+    pdl_launch();
+    bc_stage(pg, bc_sh);  // (the program does not depend on the launch before this one)
+    pdl_wait();
     double *H = pg.hold ? pg.hold + b * pg.hstride : nullptr;
     bc_run(pg, F, Pbase + b * pstride, H, (int)cl.block_rank() * blockDim.x + threadIdx.x, (int)cl.num_threads(),
            [&] { cl.sync(); });

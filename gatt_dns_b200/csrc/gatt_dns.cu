@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -140,6 +141,7 @@ struct gatt_ctx {
         unsigned *lev = nullptr;
         int nops = 0, nlev = 0;
         long long widest = 0;  // points of the largest level
+        std::vector<unsigned> begin, points;  // the levels' first ops (and nops), their points
     } d_prog[2];
     int nops = 0;
     double *d_coef1 = nullptr, *d_coef2 = nullptr, *d_xs = nullptr;
@@ -186,6 +188,8 @@ struct gatt_ctx {
     bool mean_init = false;                  // SFD mean uploaded or copied from the state
     int cur = 0;
     unsigned long long *acc = nullptr;
+    unsigned long long *mc_acc = nullptr;  // k_maxchange_store: its maxima, zero between launches,
+    unsigned *mc_count = nullptr;          // and its count of finished CTAs, after them
     double *hist = nullptr;
     int hist_cap = 0;
     StepParams *d_params = nullptr;
@@ -196,6 +200,9 @@ struct gatt_ctx {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double *tmp_side = nullptr;  // the side stream's scratch field (the global-memory line solver)
+    cudaStream_t side2 = nullptr;  // 3-D: the z sweep beside the y sweep where they are two launches
+    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;
+    double *tmp_side2 = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     int graph_kernels[2] = {0, 0};
@@ -218,6 +225,7 @@ struct gatt_ctx {
     double *fsum = nullptr, *fpart = nullptr;  // turbulence box sums, per-CTA partials
     unsigned *fdone = nullptr;  // CTAs that have finished, per member (zero between launches)
     int fblocks = 0;        // CTAs of the sums kernel (fixed: the sums do not depend on timing)
+    int chain = 0;          // 1, 2: launches form a chain (launch_chained), 2 after its first
     bool fork_x = true;     // x sweeps beside the y/z sweeps, filter field chains side by side
                             // (GATT_FORK_X=0: everything on one stream)
     bool fz_rev = true;     // last filter direction takes the fields in reverse order (GATT_FZ_REV=0: no)
@@ -284,6 +292,33 @@ int after_launch(gatt_ctx *c)
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(GATT_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     return GATT_OK;
+}
+
+// Launch a kernel; inside a chain (gatt_ctx::chain: every kernel of it calls pdl_wait) its blocks
+// may start while the one before it drains.
+int launch_chained(gatt_ctx *c, int cls, const void *k, dim3 grid, dim3 block, size_t smem, void **args, int cluster = 1)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[2];
+    if (c->chain == 2) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = cluster;
+        at[cfg.numAttrs].val.clusterDim.y = 1;
+        at[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = at;
+    TRY(before_launch(c, cls));
+    CU(cudaLaunchKernelExC(&cfg, k, args));
+    if (c->chain) c->chain = 2;  // the next launch follows a kernel
+    return after_launch(c);
 }
 
 int line_len(const gatt_ctx *c, int d) { return d == 0 ? c->nx : (d == 1 ? c->ny : c->nz); }
@@ -437,6 +472,23 @@ int resident_ctas(const void *k, int threads, size_t smem)
     return n;
 }
 
+// Let a kernel use up to `most` bytes of dynamic shared memory (and, carve, the whole L1 as shared
+// memory): once per device and kernel, when it is first launched -- setting the attributes of
+// every instantiation for each context took half of its creation.
+int allow_smem(const void *k, size_t most, bool carve = false)
+{
+    static std::mutex mu;
+    static std::set<std::pair<int, const void *>> seen;
+    int dev = 0;
+    CU(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    if (seen.count({dev, k})) return GATT_OK;
+    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    if (carve) CU(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    seen.insert({dev, k});
+    return GATT_OK;
+}
+
 // Line-solve family for new matrices: GATT_SWEEP = tile | reg | line | pipe (default pipe).
 int choose_family()
 {
@@ -512,45 +564,6 @@ int choose_blocks(int N, int nR, int Wp, int rows = 0)
     while (P * 2 <= kMaxP && N / (P * 2) >= rows && N / (P * 2) >= nR + 1) P *= 2;
     while (P > 1 && sweep_smem(N, P, nR, Wp, false) > kMaxSmem) P /= 2;
     return P;
-}
-
-// Allow every line-solve instantiation the full shared-memory budget once per context,
-// outside any stream capture.
-int set_sweep_attributes()
-{
-    for (int big = 0; big < 2; big++)
-        for (int xd = 0; xd < 2; xd++)
-            for (int per = 0; per < 2; per++)
-                for (int nR = 2; nR <= kMaxNR; nR++) {
-                    void *k = sweep_kernel(xd != 0, per != 0, nR, big != 0);
-                    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-                }
-    for (int xd = 0; xd < 2; xd++)
-        for (int per = 0; per < 2; per++)
-            for (int nR = 2; nR <= kMaxNRreg; nR++)
-                for (int wide = 0; wide < 2; wide++) {
-                    void *k = reg_kernel(true, xd != 0, per != 0, nR, wide != 0);
-                    if (!k) continue;
-                    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-                    CU(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-                }
-    for (int xd = 0; xd < 2; xd++)  // the uniform-band instantiations
-        for (int nR = 2; nR <= kMaxNRreg; nR++) {
-            void *k = xd ? pick_ub_kernel<true>(nR) : pick_ub_kernel<false>(nR);
-            if (!k) continue;
-            CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-            CU(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        }
-    for (int xd = 0; xd < 2; xd++)
-        for (int per = 0; per < 2; per++)
-            for (int LL : {4, 8, 16, 32})
-                for (int nR = 2; nR <= kMaxNRreg; nR++) {
-                    void *k = xd ? line_kernel_x(per != 0, nR, LL) : line_kernel_yz(per != 0, nR, LL);
-                    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-                }
-    CU(cudaFuncSetAttribute((const void *)k_assemble3d_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)pw_smem_bytes(kPwStages)));
-    return GATT_OK;
 }
 
 void invalidate_graphs(gatt_ctx *c)
@@ -716,6 +729,7 @@ int launch_psweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nmember
     }
     const bool cmp = ub && xd && c->x_compact;  // the compact shared-memory layout
     if (!k) return GATT_ERR_STATE;
+    TRY(allow_smem(k, kMaxSmem, true));
     // ring depth: the deepest ring that keeps the most CTAs resident (one stage suffices
     // when a tile's solve outlasts the next tile's copy)
     int nst = 0, per_sm = 0;
@@ -843,6 +857,7 @@ LinePlan line_plan_for(const gatt_ctx *c, const DevDir &m, int d, int nf, int nm
     pl.LL = LL;
     pl.jobs = line_tiles(c, d, LL) * nf * nmem;
     pl.kernel = xd ? line_kernel_x(m.periodic != 0, m.nR, LL) : line_kernel_yz(m.periodic != 0, m.nR, LL);
+    if (allow_smem(pl.kernel, kMaxSmem) != GATT_OK) return best;
     const int warps = (m.lP * LL + 31) / 32;
     const bool S = m.nspecial > 0 && (size_t)m.nspecial * line_band_doubles(m.Wp) * sizeof(double) <= kLineBandBytes;
     for (int v = S ? 0 : 2; v < 4; v++) {
@@ -862,36 +877,36 @@ LinePlan line_plan_for(const gatt_ctx *c, const DevDir &m, int d, int nf, int nm
     return best;
 }
 
-// Tile width.  Wide tiles read the records at one address a warp instead of 32/LL, narrow ones
-// make more and smaller CTAs: 32 lines where they fill the SMs (y lines of the 90x75x54 box: 15.4
-// us against 18.5 with 16 and 20.8 with 8), fewer for launches that would leave SMs idle, and 8
-// for lines of 20 blocks and more, whose wide CTAs hold an SM alone (400-point x lines of the
-// plate boundary layer: 118 us against 137 with 16).  4 where 8-line tiles just miss one round
-// (800-point x lines, 152 tiles on 148 SMs: 21.7 us against 28.9).
-LinePlan line_plan(const gatt_ctx *c, const DevDir &m, int d, int nf, int nmem)
+// Tile width, from the grid alone: it enters the order in which a line's blocks are joined, and a
+// batch member's arithmetic must be that of the member alone.  Counted for the fields of a first
+// derivative sweep of one member.  Wide tiles read the records at one address a warp instead of
+// 32/LL, narrow ones make more and smaller CTAs: 32 lines where they fill the SMs (y lines of the
+// 90x75x54 box: 15.4 us against 18.5 with 16 and 20.8 with 8), fewer for launches that would
+// leave SMs idle, and 8 for lines of 20 blocks and more, whose wide CTAs hold an SM alone
+// (400-point x lines of the plate boundary layer: 118 us against 137 with 16).  4 where 8-line
+// tiles just miss one round (800-point x lines, 152 tiles on 148 SMs: 21.7 us against 28.9).
+int line_lanes(const gatt_ctx *c, const DevDir &m, int d)
 {
     const char *e = getenv("GATT_LINES");  // 4, 8, 16 or 32 lines a tile, where they fit
     if (e) {
-        const LinePlan pl = line_plan_for(c, m, d, nf, nmem, atoi(e) == 4 || atoi(e) == 16 || atoi(e) == 32 ? atoi(e) : 8);
-        if (pl.LL) return pl;
+        const int LL = atoi(e) == 4 || atoi(e) == 16 || atoi(e) == 32 ? atoi(e) : 8;
+        if (line_fits(d == 0, m.N, m.nR, LL)) return LL;
     }
+    const int nf = c->is3d ? 5 : 4;
     if (m.lP < 20)
-        for (int LL : {32, 16}) {
-            const LinePlan pl = line_plan_for(c, m, d, nf, nmem, LL);
-            if (pl.LL && pl.jobs >= c->nsm) return pl;
-        }
-    const LinePlan pl = line_plan_for(c, m, d, nf, nmem, 8), half = line_plan_for(c, m, d, nf, nmem, 4);
+        for (int LL : {32, 16})
+            if (line_fits(d == 0, m.N, m.nR, LL) && line_tiles(c, d, LL) * nf >= c->nsm) return LL;
+    const LinePlan pl = line_plan_for(c, m, d, nf, 1, 8), half = line_plan_for(c, m, d, nf, 1, 4);
     const long long at_once = (long long)pl.per_sm * c->nsm;
     if (half.LL && (!pl.LL || (pl.jobs > at_once && pl.jobs < 2 * at_once && half.jobs <= (long long)half.per_sm * c->nsm)))
-        return half;
-    return pl;
+        return 4;
+    return 8;
 }
 
-int launch_lsweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nf, int nmem, int cls)
+// Direction d's part of a k_lsweep / k_lsweep_xy launch.
+LineArgs line_args(const gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, const LinePlan &pl, int nf)
 {
-    const LinePlan pl = line_plan(c, m, d, nf, nmem);
-    if (!pl.LL || pl.jobs > INT_MAX / 2) return GATT_ERR_STATE;
-    a.P = m.lP;
+    a.N = m.N; a.Nreal = m.N; a.P = m.lP;
     a.nst = pl.nst;
     a.tiles_per_row = (c->nx + pl.LL - 1) / pl.LL;
     a.fd_tpr = make_fastdiv(a.tiles_per_row);
@@ -904,11 +919,18 @@ int launch_lsweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nf, int
     la.stageS = pl.stageS;
     memcpy(la.band, m.lband, sizeof(la.band));
     la.fd_ntiles = make_fastdiv(a.ntiles); la.fd_nf = make_fastdiv(nf);
+    return la;
+}
+
+int launch_lsweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nf, int nmem, int cls)
+{
+    const LinePlan pl = line_plan_for(c, m, d, nf, nmem, line_lanes(c, m, d));
+    if (!pl.LL || pl.jobs > INT_MAX / 2) return GATT_ERR_STATE;
+    SweepArgs x = a;
+    const LineArgs la = line_args(c, m, d, x, pl, nf);
     const int grid = (int)std::min<long long>(pl.jobs, (long long)pl.per_sm * c->nsm);
-    void *args[] = {&a, &la};
-    TRY(before_launch(c, cls));
-    CU(cudaLaunchKernel(pl.kernel, dim3(grid), dim3((m.lP * pl.LL + 31) / 32 * 32), args, pl.smem, c->stream));
-    return after_launch(c);
+    void *args[] = {&x, (void *)&la};
+    return launch_chained(c, cls, pl.kernel, dim3(grid), dim3((m.lP * pl.LL + 31) / 32 * 32), pl.smem, args);
 }
 
 // Run one compact solve (direction d, coefficient kind) over nf fields.
@@ -947,8 +969,9 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
     }
     // lines of many blocks whose 32-line tiles leave SMs idle (the 300-point y lines of the 800x300
     // grid: 100 tiles of 19 blocks, 13.3 us against 15.3) run as 8-line tiles too
-    const bool few = m.family == FAM_PIPE && m.lQ && m.P >= 16 && (long long)a.njobs < c->nsm && !mc_ref;
-    if (m.family == FAM_LINE || few) {
+    // (decided by the grid alone, as line_lanes; a chain takes no other solver)
+    const bool few = m.family == FAM_PIPE && m.lQ && m.P >= 16 && (long long)a.ntiles * (c->is3d ? 5 : 4) < c->nsm;
+    if (m.family == FAM_LINE || (few && !mc_ref) || (c->chain && m.lQ)) {
         const int r = launch_lsweep(c, m, d, a, nf, nmembers, cls);
         if (r != GATT_ERR_STATE) return r;  // GATT_ERR_STATE: more tiles than a launch counts
     }
@@ -968,6 +991,7 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
                          : a.tiles_per_row * (d == 1 ? c->nz : c->ny),
                   nf, nmembers);
         void *args[] = {&a};
+        if (smem > 48 * 1024) TRY(allow_smem(k, kMaxSmem));
         TRY(before_launch(c, cls));
         CU(cudaLaunchKernel(k, grid, dim3(32 * m.P), args, smem, c->stream));
         return after_launch(c);
@@ -1035,8 +1059,95 @@ int sweep_yz(gatt_ctx *c, const double *in, long long in_bs, const int *sy, cons
         const int r = launch_psweep(c, my, 1, a, nmembers, cls_yz, &mz);
         if (r != GATT_ERR_STATE) return r;  // GATT_ERR_STATE: layout refused, two launches
     }
+    // two launches: the z sweep beside the y sweep on a third stream
+    const bool fork = c->fork_x && !c->profiling && c->side2;
+    if (fork) {
+        CU(cudaEventRecord(c->ev_fork2, c->stream));
+        CU(cudaStreamWaitEvent(c->side2, c->ev_fork2, 0));
+        std::swap(c->stream, c->side2);
+        std::swap(c->tmp, c->tmp_side2);
+    }
+    int r = sweep(c, 2, 0, in, in_bs, sz, out, out_bs, oz, nf, nmembers, 0, nullptr, cls_z);
+    if (fork) {
+        std::swap(c->stream, c->side2);
+        std::swap(c->tmp, c->tmp_side2);
+        if (r == GATT_OK) CU(cudaEventRecord(c->ev_join2, c->side2));
+    }
+    TRY(r);
     TRY(sweep(c, 1, 0, in, in_bs, sy, out, out_bs, oy, nf, nmembers, 0, nullptr, cls_y));
-    return sweep(c, 2, 0, in, in_bs, sz, out, out_bs, oz, nf, nmembers, 0, nullptr, cls_z);
+    if (fork) CU(cudaStreamWaitEvent(c->stream, c->ev_join2, 0));
+    return GATT_OK;
+}
+
+// The x and y sweeps of a 2-D stage in one launch: input slots sx / sy, output slots ox / oy.
+struct XyPlan {
+    LinePlan x, y;
+    void *kernel = nullptr;
+    int threads = 0, per_sm = 0;
+    size_t smem = 0;
+};
+
+XyPlan xy_plan(const gatt_ctx *c, int nf, int nmem)
+{
+    const DevDir &mx = c->mat[0][0], &my = c->mat[1][0];
+    XyPlan p;
+    p.x = line_plan_for(c, mx, 0, nf, nmem, 8);
+    p.y = line_plan_for(c, my, 1, nf, nmem, 8);
+    if (!p.x.LL || !p.y.LL) return p;
+    void *k = line_kernel_xy(mx.periodic != 0, my.periodic != 0, mx.nR);
+    if (!k || allow_smem(k, kMaxSmem) != GATT_OK) return p;
+    p.threads = (std::max(mx.lP, my.lP) * 8 + 31) / 32 * 32;
+    p.smem = std::max(p.x.smem, p.y.smem);
+    p.per_sm = resident_ctas(k, p.threads, p.smem);
+    if (p.per_sm > 0) p.kernel = k;
+    return p;
+}
+
+// Whether the context's 2-D steps take that launch (and the whole step the chained form):
+// decided by the grid alone, as a batch member's arithmetic must be that of the member alone.
+// Both directions' tiles of one member fit in one round, and neither direction leaves more than
+// a third of the CTA idle (the 800x300 grid: 13 warps of x beside 5 of y would).  On the 128^2
+// cavity a stage is so five launches in a row instead of seven on two streams.
+bool chained_2d(const gatt_ctx *c)
+{
+    const DevDir &mx = c->mat[0][0], &my = c->mat[1][0];
+    if (c->is3d || !mx.lQ || !my.lQ || mx.nR != my.nR) return false;
+    for (int d = 0; d < 2; d++)
+        if (c->filt[d] && !c->mat[d][1].lQ) return false;
+    if (3 * mx.lP < 2 * my.lP || 3 * my.lP < 2 * mx.lP) return false;
+    const XyPlan p = xy_plan(c, 4, 1);
+    return p.kernel && p.x.jobs + p.y.jobs <= (long long)p.per_sm * c->nsm;
+}
+
+int sweep_xy(gatt_ctx *c, const double *in, long long in_bs, const int *sx, const int *sy, double *out, long long out_bs,
+             const int *ox, const int *oy, int nf, int nmem, int cls)
+{
+    const XyPlan p = xy_plan(c, nf, nmem);
+    if (!p.kernel || p.x.jobs + p.y.jobs > INT_MAX / 2) return fail(GATT_ERR_STATE, "x and y sweeps do not fit one launch");
+    SweepArgs a[2];
+    LineArgs la[2];
+    for (int d = 0; d < 2; d++) {
+        SweepArgs &q = a[d];
+        memset(&q, 0, sizeof(q));
+        q.in = in; q.out = out; q.in_bstride = in_bs; q.out_bstride = out_bs; q.npts = c->npts;
+        for (int f = 0; f < nf; f++) { q.in_slot[f] = d ? sy[f] : sx[f]; q.out_slot[f] = d ? oy[f] : ox[f]; }
+        q.nx = c->nx; q.ny = c->ny; q.nz = c->nz;
+        q.nlines = nlines(c, d);
+        q.es = c->nx;
+        q.os = c->npts;
+        q.ltype = c->ltype[d]; q.ntypes = c->mat[d][0].nTypes;
+        q.epi = EPI_STORE; q.dir = d; q.nf = nf;
+        la[d] = line_args(c, c->mat[d][0], d, q, d ? p.y : p.x, nf);
+    }
+    // each direction its share of the resident CTAs
+    const long long all = p.x.jobs + p.y.jobs, room = (long long)p.per_sm * c->nsm;
+    int gx = (int)p.x.jobs, gy = (int)p.y.jobs;
+    if (all > room) {
+        gx = (int)std::max(1LL, room * p.x.jobs / all);
+        gy = (int)std::max(1LL, std::min(p.y.jobs, room - gx));
+    }
+    void *args[] = {&a[0], &la[0], &a[1], &la[1], &gx};
+    return launch_chained(c, cls, p.kernel, dim3(gx + gy), dim3(p.threads), p.smem, args);
 }
 
 // ---------------------------------------------------------------------------
@@ -1076,6 +1187,8 @@ Forcings forcing_args(const gatt_ctx *c)
     f.sums = c->fsum;
     f.nx = c->nx;
     f.ny = c->ny;
+    f.fd_nx = make_fastdiv(c->nx);
+    f.fd_ny = make_fastdiv(c->ny);
     return f;
 }
 
@@ -1121,6 +1234,7 @@ int launch_assemble3d_pipe(gatt_ctx *c, const StateSet &q, const StateSet &q0, c
     if (a.use_q0 && !pw_map(c, &maps.m[PW_Q0], q0b, 5, q0.bstride, nmem)) return GATT_ERR_STATE;
     if (a.use_delta && !pw_map(c, &maps.m[PW_DL], dlb, 5, delta.bstride, nmem)) return GATT_ERR_STATE;
     const size_t smem = pw_smem_bytes(a.nst);
+    TRY(allow_smem((const void *)k_assemble3d_pipe, smem));
     const int per_sm = resident_ctas((const void *)k_assemble3d_pipe, 2 * kPwC, smem);
     if (per_sm < 1) return GATT_ERR_STATE;
     const long long grid = std::min<long long>(a.njobs, (long long)per_sm * c->nsm);
@@ -1179,6 +1293,25 @@ int join_side(gatt_ctx *c)
     return GATT_OK;
 }
 
+int launch_visc2d(gatt_ctx *c, StateSet q, double *d1, double *tq, int nmem)
+{
+    FieldSet f1 = fset(c, d1, D2_N), ft = fset(c, tq, T2_N);
+    long long n = c->npts;
+    void *args[] = {&c->ph, &q, &f1, &ft, &n};
+    return launch_chained(c, PC_VISC, (const void *)k_visc2d, dim3(grid_for(c, n), nmem), dim3(kBlock), 0, args);
+}
+
+int launch_assemble2d(gatt_ctx *c, StateSet q, StateSet q0, StateSet out, int mode, int nmem, double *d1, double *tq,
+                      double *d2, double *delta)
+{
+    FieldSet fd = fset(c, delta, 5), f1 = fset(c, d1, D2_N), ft = fset(c, tq, T2_N), f2 = fset(c, d2, S2_N);
+    Forcings fs = forcing_args(c);
+    long long n = c->npts;
+    const StepParams *sp = c->d_params;
+    void *args[] = {&c->ph, &q, &q0, &out, &fd, &f1, &ft, &f2, &n, &mode, &sp, &fs};
+    return launch_chained(c, PC_ASSEMBLE, (const void *)k_assemble2d, dim3(grid_for(c, n), nmem), dim3(kBlock), 0, args);
+}
+
 // nseq2d/nseq3d on stage input q, fused with the RK4 update into out (mode).
 int rhs_stage(gatt_ctx *c, const StateSet &q, const StateSet &q0, const StateSet &out, int mode, int nmem,
               double *d1, double *tq, double *d2, double *delta, bool assemble = true)
@@ -1220,22 +1353,23 @@ int rhs_stage(gatt_ctx *c, const StateSet &q, const StateSet &q0, const StateSet
     const int fin[4] = {0, 1, 3, 4};
     const int ox[4] = {D2_UX, D2_VX, D2_RX, D2_EX};
     const int oy[4] = {D2_UY, D2_VY, D2_RY, D2_EY};
+    const int ix[3] = {T2_XY, T2_XX, T2_QX}, sx[3] = {S2_TXYX, S2_TXXX, S2_HTX};
+    const int iy[3] = {T2_XY, T2_YY, T2_QY}, sy[3] = {S2_TXYY, S2_TYYY, S2_HTY};
+    if (c->chain) {
+        // both directions in one launch
+        TRY(sweep_xy(c, qin, qbs, fin, fin, d1, bd1, ox, oy, 4, nmem, PC_D1X));
+        TRY(launch_visc2d(c, q, d1, tq, nmem));
+        TRY(sweep_xy(c, tq, btq, ix, iy, d2, bd2, sx, sy, 3, nmem, PC_D2X));
+        return launch_assemble2d(c, q, q0, out, mode, nmem, d1, tq, d2, delta);
+    }
     TRY(beside(c, [&] { return sweep(c, 0, 0, qin, qbs, fin, d1, bd1, ox, 4, nmem, 0, nullptr, PC_D1X); }));
     TRY(sweep(c, 1, 0, qin, qbs, fin, d1, bd1, oy, 4, nmem, 0, nullptr, PC_D1Y));
     TRY(join_side(c));
-    TRY(before_launch(c, PC_VISC));
-    k_visc2d<<<dim3(grid_for(c, n), nmem), kBlock, 0, c->stream>>>(c->ph, q, fset(c, d1, D2_N), fset(c, tq, T2_N), n);
-    TRY(after_launch(c));
-    const int ix[3] = {T2_XY, T2_XX, T2_QX}, sx[3] = {S2_TXYX, S2_TXXX, S2_HTX};
-    const int iy[3] = {T2_XY, T2_YY, T2_QY}, sy[3] = {S2_TXYY, S2_TYYY, S2_HTY};
+    TRY(launch_visc2d(c, q, d1, tq, nmem));
     TRY(beside(c, [&] { return sweep(c, 0, 0, tq, btq, ix, d2, bd2, sx, 3, nmem, 0, nullptr, PC_D2X); }));
     TRY(sweep(c, 1, 0, tq, btq, iy, d2, bd2, sy, 3, nmem, 0, nullptr, PC_D2Y));
     TRY(join_side(c));
-    TRY(before_launch(c, PC_ASSEMBLE));
-    k_assemble2d<<<dim3(grid_for(c, n), nmem), kBlock, 0, c->stream>>>(
-        c->ph, q, q0, out, fset(c, delta, 5), fset(c, d1, D2_N), fset(c, tq, T2_N), fset(c, d2, S2_N), n, mode, sp,
-        forcing_args(c));
-    return after_launch(c);
+    return launch_assemble2d(c, q, q0, out, mode, nmem, d1, tq, d2, delta);
 }
 
 // ---------------------------------------------------------------------------
@@ -1369,9 +1503,11 @@ int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict
     cudaFree(d.lev); d.lev = nullptr;
     d.nops = (int)out.size();
     d.nlev = (int)begin.size();
+    begin.push_back((unsigned)out.size());
+    d.begin = begin;
+    d.points = points;
     if (out.empty()) return GATT_OK;
     std::vector<unsigned> lev(begin);
-    lev.push_back((unsigned)out.size());
     lev.insert(lev.end(), points.begin(), points.end());
     lev.push_back(0);  // whole 8-byte words
     CU(cudaMalloc(&d.ops, out.size() * sizeof(BcOp)));
@@ -1687,9 +1823,9 @@ int choose_bc_cluster(gatt_ctx *c)
 // that keeps the clusters of all members within the SMs and gives every CTA about 2048 points of
 // the largest level (smaller programs gain nothing from more CTAs and pay a dearer barrier per
 // level); with cs < 2 the one-CTA form.
-template <typename... KArgs, typename... Args>
+template <typename... KArgs>
 int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...), int cs_max, int nmem, int form,
-              Args &&...args)
+              std::decay_t<KArgs>... args)
 {
     const gatt_ctx::BcDev &d = c->d_prog[form];
     const size_t need = bc_stage_bytes(bc_program(c, 0.0, form)), smem = need <= (size_t)kBcStagedBytes ? need : 0;
@@ -1697,25 +1833,16 @@ int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...),
     const long long by_sms = std::max(1, c->nsm / std::max(1, nmem));
     int cs = 1;
     while (cs * 2 <= cs_max && cs * 2 <= by_work && cs * 2 <= by_sms) cs *= 2;
-    if (cs >= 2) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(nmem * cs);
-        cfg.blockDim = dim3(kBcThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = c->stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cs;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        CU(cudaLaunchKernelEx(&cfg, kcluster, std::forward<Args>(args)...));
-    } else {
-        kblock<<<nmem, kBcThreads, smem, c->stream>>>(std::forward<Args>(args)...);
-    }
-    return GATT_OK;
+    void *argp[] = {(void *)&args...};
+    return launch_chained(c, PC_BC, cs >= 2 ? (const void *)kcluster : (const void *)kblock, dim3(nmem * cs),
+                          dim3(kBcThreads), smem, argp, cs);
 }
+
+// Levels of a program up to which each is a launch of its own over the whole GPU, chained: a
+// cluster's 16 SMs took 56 us an application on the 400x150x64 plate (five levels, the widest
+// 176 000 points) against 12, and even the two small levels of the 128^2 cavity 6 us in one
+// launch against 2 and 2.
+constexpr int kBcLaunches = 16;
 
 // applyBoundCond at time t + tfac dt of the step (timeIntegration.F90 passes t + dt/2 or
 // t + dt by stage); fixed: at time tfix, keeping the holdInlet values on a first call
@@ -1730,9 +1857,29 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
     } else if (c->hold_len > 0 && !c->hold_saved) {
         return fail(GATT_ERR_STATE, "holdInlet: call gatt_apply_bc on the initial state before stepping");
     }
-    TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc, k_bc_cluster, c->bc_cluster, nmem, 0, pg, q, c->P, (long long)c->npts));
-    return after_launch(c);
+    const gatt_ctx::BcDev &d = c->d_prog[0];
+    if (c->bc_cluster && d.nlev <= kBcLaunches) {
+        // one launch per level, chained
+        const int chain = c->chain;
+        int rc = GATT_OK;
+        for (int l = 0; l < d.nlev && rc == GATT_OK; l++) {
+            if (l) c->chain = 2;
+            int op0 = (int)d.begin[l], nops = (int)(d.begin[l + 1] - d.begin[l]);
+            unsigned total = d.points[l];
+            long long stride = c->npts;
+            StateSet qs = q;
+            const size_t smem = (size_t)nops * sizeof(BcOp);
+            if (smem > 48 * 1024) rc = smem <= kMaxSmem ? allow_smem((const void *)k_bc_level, kMaxSmem)
+                                                        : fail(GATT_ERR_BADARG, "too many boundary items in one level");
+            if (rc != GATT_OK) break;
+            void *args[] = {&pg, &qs, &c->P, &stride, &l, &op0, &nops, &total};
+            const unsigned blocks = std::min((total + 255) / 256, (unsigned)c->nsm * 8);
+            rc = launch_chained(c, PC_BC, (const void *)k_bc_level, dim3(blocks, nmem), dim3(256), smem, args);
+        }
+        c->chain = chain ? 2 : 0;
+        return rc;
+    }
+    return launch_bc(c, k_bc, k_bc_cluster, c->bc_cluster, nmem, 0, pg, q, c->P, (long long)c->npts);
 }
 
 // applyFilters2D/3D in place on set q (derivs.F90:303-552)
@@ -1763,7 +1910,7 @@ int filter_set(gatt_ctx *c, const StateSet &q, int nmem, double blend, const dou
         }
         return GATT_OK;
     };
-    if (!c->fork_x || c->profiling || !c->side) return chain(fl, rl, nf);
+    if (!c->fork_x || c->profiling || !c->side || c->chain) return chain(fl, rl, nf);
     // the fields' filters are independent -- U, V (and W) on the context's stream, R, E beside
     // them on the side stream, so that each direction's last partial wave overlaps the other
     // chain's launches
@@ -1799,6 +1946,19 @@ int check_ready(const gatt_ctx *c, bool need_filter)
     return GATT_OK;
 }
 
+// The integrator's stages (main.F90:304-352 by timeStepping): assembly mode, and the fraction of
+// dt at which its boundary conditions are taken.
+struct Stage {
+    int mode;
+    double tfac;
+};
+std::vector<Stage> stages_of(const gatt_ctx *c)
+{
+    if (c->time_stepping == 2) return {{RK_EULER, c->is3d ? 0.0 : 1.0}};  // EULER_3D passes t, EULER_2D t + dt
+    if (c->time_stepping == 3) return {{SSP_STAGE1, 1.0}, {SSP_STAGE2, 0.5}, {SSP_STAGE3, 1.0}};
+    return {{RK_STAGE1, 0.5}, {RK_STAGE2, 0.5}, {RK_STAGE3, 1.0}, {RK_STAGE4, 1.0}};
+}
+
 // The whole of main.F90:255-420 for all members, enqueued on the stream.
 int step_body(gatt_ctx *c)
 {
@@ -1806,22 +1966,20 @@ int step_body(gatt_ctx *c)
     StateSet qst = qs;  // stage BC set: in 2-D RK4_2D hands the caller's W to applyBoundCond
     if (!c->is3d) qst.v[2] = q0.v[2];
     const int nm = c->nb;
-    CU(cudaMemsetAsync(c->acc, 0, sizeof(unsigned long long) * 5 * nm, c->stream));
-    // the time integrator (main.F90:304-352 by timeStepping): every stage forms the RHS of its
-    // input, updates the stage state and applies the boundary conditions
-    if (c->time_stepping == 2) {  // EULER_2D/3D (timeIntegration.F90:158-223, 500-567)
-        TRY(rhs_stage(c, q0, q0, qs, RK_EULER, nm, c->d1, c->tq, c->d2, c->delta));
-        TRY(apply_bc(c, qst, nm, c->is3d ? 0.0 : 1.0));  // EULER_3D passes t, EULER_2D t + dt
-    } else if (c->time_stepping == 3) {  // SSPRK3_2D/3D (timeIntegration.F90:225-336, 569-680)
-        for (int s = 0; s < 3; s++) {
-            TRY(rhs_stage(c, s == 0 ? q0 : qs, q0, qs, SSP_STAGE1 + s, nm, c->d1, c->tq, c->d2, c->delta));
-            TRY(apply_bc(c, qst, nm, s == 1 ? 0.5 : 1.0));
-        }
-    } else {  // RK4_2D/3D (timeIntegration.F90:8-156, 338-498)
-        for (int s = 1; s <= 4; s++) {
-            TRY(rhs_stage(c, s == 1 ? q0 : qs, q0, qs, s, nm, c->d1, c->tq, c->d2, c->delta));
-            TRY(apply_bc(c, qst, nm, s <= 2 ? 0.5 : 1.0));
-        }
+    // small 2-D grids: one chain of launches on one stream
+    struct Chain {
+        gatt_ctx *c;
+        Chain(gatt_ctx *cc, bool on) : c(cc) { c->chain = on; }
+        ~Chain() { c->chain = 0; }
+    } chain(c, chained_2d(c));
+    if (!c->chain) CU(cudaMemsetAsync(c->acc, 0, sizeof(unsigned long long) * 5 * nm, c->stream));
+    // every stage forms the RHS of its input, updates the stage state and applies the boundary
+    // conditions (timeIntegration.F90)
+    bool first = true;
+    for (const Stage &s : stages_of(c)) {
+        TRY(rhs_stage(c, first ? q0 : qs, q0, qs, s.mode, nm, c->d1, c->tq, c->d2, c->delta));
+        TRY(apply_bc(c, qst, nm, s.tfac));
+        first = false;
     }
     // nothing after the filter (no SFD, no boundary program): its last sweep can take the
     // max-change (main.F90:413-418) in its epilogue; the state sets must be equally spaced
@@ -1831,12 +1989,19 @@ int step_body(gatt_ctx *c)
     else TRY(filter_set(c, qs, nm, 0.0, nullptr, mc_in_filter ? &q0 : nullptr));
     const bool mc_done = mc_in_filter && c->mc_done;
     if (c->sfd_type > 0) {
-        TRY(before_launch(c, PC_SFD));
-        k_sfd<<<dim3(grid_for(c, c->npts), nm), kBlock, 0, c->stream>>>(qs, fset(c, c->mean, 5), c->chi, c->sfd_delta,
-                                                                          c->is3d ? 5 : 4, c->npts, c->d_params);
-        TRY(after_launch(c));
+        StateSet q = qs;
+        FieldSet mean = fset(c, c->mean, 5);
+        int nvar = c->is3d ? 5 : 4;
+        void *args[] = {&q, &mean, &c->chi, &c->sfd_delta, &nvar, &c->npts, &c->d_params};
+        TRY(launch_chained(c, PC_SFD, (const void *)k_sfd, dim3(grid_for(c, c->npts), nm), dim3(kBlock), 0, args));
     }
     TRY(apply_bc(c, qs, nm, 1.0));  // main.F90:405, at t + dt
+    if (c->chain) {
+        StateSet x = qs, y = q0;
+        void *args[] = {&x, &y, &c->mc_acc, &c->mc_count, &c->hist, &c->npts, &c->d_params};
+        return launch_chained(c, PC_MAXCHANGE, (const void *)k_maxchange_store, dim3(grid_for(c, c->npts), nm), dim3(kBlock),
+                              0, args);
+    }
     if (!mc_done) {
         TRY(before_launch(c, PC_MAXCHANGE));
         k_maxchange<<<dim3(grid_for(c, c->npts), nm), kBlock, 0, c->stream>>>(qs, q0, c->acc, c->npts);
@@ -2254,10 +2419,8 @@ int diff_alloc(gatt_ctx *c, bool adjoint)
 int bc_tl(gatt_ctx *c, const StateSet &x, const StateSet &y, double tfac)
 {
     if (c->nops == 0) return GATT_OK;
-    TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc_tl, k_bc_tl_cluster, c->bc_cluster_tl, c->nb, 0, bc_program(c, tfac), x, c->P, y, c->t_P,
-                  (long long)c->npts));
-    return after_launch(c);
+    return launch_bc(c, k_bc_tl, k_bc_tl_cluster, c->bc_cluster_tl, c->nb, 0, bc_program(c, tfac), x, c->P, y, c->t_P,
+                  (long long)c->npts);
 }
 
 // boundary program on base x at time t + tfac dt, recording tape number `which` (0..4)
@@ -2265,10 +2428,8 @@ int bc_rec(gatt_ctx *c, const StateSet &x, int which, double tfac)
 {
     if (c->nops == 0) return GATT_OK;
     const long long ts = std::max(1LL, c->tape_len);
-    TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc_rec, k_bc_rec_cluster, c->bc_cluster_rec, c->nb, 1, bc_program(c, tfac, 1), x, c->P,
-                  (long long)c->npts, c->a_tape + which * ts * c->nb, ts));
-    return after_launch(c);
+    return launch_bc(c, k_bc_rec, k_bc_rec_cluster, c->bc_cluster_rec, c->nb, 1, bc_program(c, tfac, 1), x, c->P,
+                  (long long)c->npts, c->a_tape + which * ts * c->nb, ts);
 }
 
 // transposed boundary program on lambda, from tape `which`
@@ -2277,10 +2438,8 @@ int bc_adj(gatt_ctx *c, const StateSet &lam, int which)
     if (c->nops == 0) return GATT_OK;
     const long long ts = std::max(1LL, c->tape_len);
     CU(cudaMemsetAsync(c->a_lP, 0, sizeof(double) * (size_t)c->npts * c->nb, c->stream));
-    TRY(before_launch(c, PC_BC));
-    TRY(launch_bc(c, k_bc_adj, k_bc_adj_cluster, c->bc_cluster_adj, c->nb, 1, bc_program(c, 1.0, 1), lam, c->a_lP,
-                  (long long)c->npts, (const double *)(c->a_tape + which * ts * c->nb), ts));
-    return after_launch(c);
+    return launch_bc(c, k_bc_adj, k_bc_adj_cluster, c->bc_cluster_adj, c->nb, 1, bc_program(c, 1.0, 1), lam, c->a_lP,
+                  (long long)c->npts, (const double *)(c->a_tape + which * ts * c->nb), ts);
 }
 
 int set_params(gatt_ctx *c, int slot, double t, double dt)
@@ -2811,9 +2970,15 @@ int gatt_create(gatt_ctx **out, int nx, int ny, int nz, int nbatch)
         if (es == cudaSuccess) es = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
         if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
         if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
+        if (c->is3d) {
+            if (es == cudaSuccess) es = cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking);
+            if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_fork2, cudaEventDisableTiming);
+            if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming);
+        }
         if (es != cudaSuccess && rc == GATT_OK) rc = fail(GATT_ERR_CUDA, cudaGetErrorString(es));
     }
     if (rc == GATT_OK) {
+        if (c->is3d) chk(alloc_fields(c, &c->tmp_side2, 1, 1));
         chk(alloc_fields(c, &c->qA, 5, nbatch));
         chk(alloc_fields(c, &c->qB, 5, nbatch));
         chk(alloc_fields(c, &c->delta, 5, nbatch));
@@ -2826,13 +2991,16 @@ int gatt_create(gatt_ctx **out, int nx, int ny, int nz, int nbatch)
     }
     if (rc == GATT_OK) {
         cudaError_t ea = cudaMalloc(&c->acc, sizeof(unsigned long long) * 5 * nbatch);
+        if (ea == cudaSuccess) ea = cudaMalloc(&c->mc_acc, sizeof(unsigned long long) * (5 * (size_t)nbatch + 1));
+        if (ea == cudaSuccess)
+            ea = cudaMemsetAsync(c->mc_acc, 0, sizeof(unsigned long long) * (5 * (size_t)nbatch + 1), c->stream);
+        if (ea == cudaSuccess) c->mc_count = reinterpret_cast<unsigned *>(c->mc_acc + 5 * (size_t)nbatch);
         if (ea == cudaSuccess) ea = cudaMalloc(&c->d_params, sizeof(StepParams));
         if (ea == cudaSuccess) ea = cudaMemsetAsync(c->d_params, 0, sizeof(StepParams), c->stream);
         if (ea == cudaSuccess) ea = cudaHostAlloc(&c->h_err, sizeof(int), cudaHostAllocMapped);
         if (ea == cudaSuccess) { *c->h_err = 0; ea = cudaHostGetDevicePointer(&c->d_err, c->h_err, 0); }
         if (ea != cudaSuccess) rc = fail(GATT_ERR_NOMEM, cudaGetErrorString(ea));
     }
-    if (rc == GATT_OK) chk(set_sweep_attributes());
     if (rc == GATT_OK) chk(choose_bc_cluster(c));
     if (rc == GATT_OK) chk(ensure_hist(c, 64));
     if (rc == GATT_OK) {
@@ -2856,7 +3024,7 @@ void gatt_destroy(gatt_ctx *c)
         }
         cudaFree(c->ltype[d]);
     }
-    double *bufs[] = {c->qA, c->qB, c->delta, c->mean, c->d1, c->tq, c->d2, c->P, c->tmp, c->tmp_side, c->tin, c->tout, c->chi, c->hist,
+    double *bufs[] = {c->qA, c->qB, c->delta, c->mean, c->d1, c->tq, c->d2, c->P, c->tmp, c->tmp_side, c->tmp_side2, c->tin, c->tout, c->chi, c->hist,
                       c->d_coef1, c->d_coef2, c->d_xs, c->d_hold, c->arn_zeta, c->arn_B, c->arn_base, c->arn_um,
                       c->arn_part, c->arn_h};
     cudaFree(c->arn_region);
@@ -2869,12 +3037,15 @@ void gatt_destroy(gatt_ctx *c)
     for (double *p : dbufs) cudaFree(p);
     for (double *p : bufs) cudaFree(p);
     for (gatt_ctx::BcDev &d : c->d_prog) { cudaFree(d.ops); cudaFree(d.lev); }
-    cudaFree(c->acc); cudaFree(c->d_params);
+    cudaFree(c->acc); cudaFree(c->mc_acc); cudaFree(c->d_params);
     cudaFree(c->fsum); cudaFree(c->fpart); cudaFree(c->fdone);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_err) cudaFreeHost(c->h_err);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     if (c->side) cudaStreamDestroy(c->side);
+    if (c->side2) cudaStreamDestroy(c->side2);
+    if (c->ev_fork2) cudaEventDestroy(c->ev_fork2);
+    if (c->ev_join2) cudaEventDestroy(c->ev_join2);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     delete c;
@@ -2993,7 +3164,8 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     m.hA = std::move(hA); m.hB = std::move(hB); m.hC = std::move(hC); m.hD = std::move(hD); m.hR = std::move(hR);
     m.Np = Npipe;
     TRY(upload_records(c, m, P, rpb ? Np : N));
-    if (line || (rpb && P >= 16 && line_fits(d == 0, N, nRHS, 8))) TRY(upload_line_records(c, m));
+    // (2-D: also for the chained step's sweeps)
+    if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_fits(d == 0, N, nRHS, 8))) TRY(upload_line_records(c, m));
     m.rpb = rpb;
     m.family = line ? FAM_LINE : rpb ? (want == FAM_LINE ? FAM_PIPE : want) : FAM_TILE;
     m.set = true;

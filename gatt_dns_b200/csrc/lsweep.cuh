@@ -84,17 +84,20 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src)
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// a.Nreal: rows of a line, a.P: blocks, a.nst: stages (1 or 2), a.tiles_per_row: y/z tiles of LL
-// points per row of x, a.njobs: tiles x fields x members.
+// One direction's tiles job0, job0 + jstep, ...  a.Nreal: rows of a line, a.P: blocks, a.nst:
+// stages (1 or 2), a.tiles_per_row: y/z tiles of LL points per row of x, a.njobs: tiles x fields
+// x members.  The CTA's first ceil(P LL / 32) warps run it, the others leave.
 template <bool XD, bool PER, int NR, int LL>
-__global__ void __launch_bounds__(line_max_threads(NR))
-    k_lsweep(const __grid_constant__ SweepArgs a, const __grid_constant__ LineArgs c)
+__device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, int job0, int jstep)
 {
     constexpr int H = NR - 1, W = 2 * NR - 1, WP = (W + 3) / 4 * 4, M = kLineRows, Q6 = kLineQ;
     constexpr int BB = 32 / LL;         // row blocks in a warp
     constexpr int YP = LL <= 8 ? LL : 0;  // pads per 16 rows of a y/z tile
     extern __shared__ __align__(16) double lsm[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (a.P * LL + 31) >> 5;
+    const int T = nw * 32;
+    if (warp >= nw) return;
+    auto sync = [&] { asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory"); };
     const int l = lane & (LL - 1), sub = lane / LL;
     const int p = warp * BB + sub, sp = p * M;
     const int N = a.Nreal, P = a.P;
@@ -104,11 +107,11 @@ __global__ void __launch_bounds__(line_max_threads(NR))
     // coefficients: one type's records and (where they fit) the band rows
     double *sx = lsm + a.nst * tsize, *sc = sx + 5 * nw * LL;
     auto stage_type = [&](int t0) {
-        for (int i = threadIdx.x; i < td; i += blockDim.x) cp_async8(sc + i, c.Q + t0 * td + i);
+        for (int i = threadIdx.x; i < td; i += T) cp_async8(sc + i, c.Q + t0 * td + i);
     };
     const double *S = c.S;
     if (c.stageS) {
-        for (int i = threadIdx.x; i < c.nspecial * bd; i += blockDim.x) cp_async8(sc + td + i, c.S + i);
+        for (int i = threadIdx.x; i < c.nspecial * bd; i += T) cp_async8(sc + td + i, c.S + i);
         S = sc + td;
     }
     double *xs = sx + l;
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(line_max_threads(NR))
                 for (int r = lane; r < N; r += 32, src += 32, d += 34) cp_async8(d, src);
             }
         } else {
-            const int i = threadIdx.x % LL, r0 = threadIdx.x / LL, dr = blockDim.x / LL;
+            const int i = threadIdx.x % LL, r0 = threadIdx.x / LL, dr = T / LL;
             if (i < q.nl) {
                 const double *src = in + i + (long long)r0 * a.es;
 #pragma unroll 4
@@ -155,26 +158,25 @@ __global__ void __launch_bounds__(line_max_threads(NR))
         }
     };
     const bool blend_on = a.epi == EPI_BLEND;
-    const double blend = blend_on ? sweep_blend(a) : 0.0;
     const int pc = min(p, P - 1);  // threads past the last block hold zero rows
     const bool two = a.nst == 2;
     int stage = 0;
     int t;
     // type of this thread's line, taken a tile ahead (its load is not waited for in the solve)
     auto type_of = [&](const Tile &q) { return a.ntypes > 1 && l < q.nl ? (int)a.ltype[q.L0 + l] : 0; };
-    {
-        const Tile first = tile_of(blockIdx.x);
-        issue(first, lsm);
-        t = type_of(first);
-    }
+    t = type_of(tile_of(job0));
     int staged = __shfl_sync(0xffffffffu, t, 0);  // lane 0 holds the first line
     stage_type(staged);
     int sb = c.blk[t * P + pc];
-    for (int job = blockIdx.x; job < a.njobs; job += gridDim.x) {
+    // the coefficients do not depend on the launch before this one, the lines do
+    pdl_wait();
+    issue(tile_of(job0), lsm);
+    const double blend = blend_on ? sweep_blend(a) : 0.0;
+    for (int job = job0; job < a.njobs; job += jstep) {
     double *tl = lsm + stage * tsize;
     cp_async_wait_all();
-    __syncthreads();  // the tile has landed, and the other stage's results have left
-    const int ahead = job + gridDim.x;
+    sync();  // the tile has landed, and the other stage's results have left
+    const int ahead = job + jstep;
     int tnext = 0;
     if (ahead < a.njobs) {
         const Tile next = tile_of(ahead);
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(line_max_threads(NR))
 #pragma unroll
         for (int o = 16; o >= LL; o >>= 1) dot = dot + __shfl_xor_sync(0xffffffffu, dot, o);
         if (sub == 0) xs[warp * LL] = dot;
-        __syncthreads();
+        sync();
         x1 = xs[0];
         for (int k = 1; k < nw; k++) x1 = x1 + xs[k * LL];
         cc = *reinterpret_cast<const double2 *>(Qt + td - 2);
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(line_max_threads(NR))
             xs[(nw + warp) * LL] = e + pe * yl;
             xs[(2 * nw + warp) * LL] = pe * pl;
         }
-        __syncthreads();
+        sync();
         double Yw = 0.0;
         for (int k = 0; k < warp; k++) Yw = xs[(nw + k) * LL] + xs[(2 * nw + k) * LL] * Yw;
         Y = yl + pl * Yw;
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(line_max_threads(NR))
             xs[(3 * nw + warp) * LL] = e + re * xl;
             xs[(4 * nw + warp) * LL] = re * pl;
         }
-        __syncthreads();
+        sync();
         double Xw = 0.0;
         for (int k = nw - 1; k > warp; k--) Xw = xs[(3 * nw + k) * LL] + xs[(4 * nw + k) * LL] * Xw;
         X = xl + pl * Xw;
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(line_max_threads(NR))
         }
     }
     if (XD) {
-        __syncthreads();
+        sync();
         for (int n = warp; n < cur.nl; n += nw) {
             double *dst = out + (long long)n * N + lane;
             const double *src = tl + n * pitch + lane + (lane >> 4);
@@ -379,14 +381,14 @@ __global__ void __launch_bounds__(line_max_threads(NR))
     if (ahead < a.njobs) {
         if (two) stage ^= 1;
         else {
-            __syncthreads();  // the stage has been read
+            sync();  // the stage has been read
             issue(tile_of(ahead), lsm);
         }
         t = tnext;
         sb = c.blk[t * P + pc];
         const int t0 = __shfl_sync(0xffffffffu, t, 0);
         if (t0 != staged) {  // the same decision in every warp
-            __syncthreads();
+            sync();
             stage_type(t0);
             staged = t0;
         }
@@ -394,10 +396,36 @@ __global__ void __launch_bounds__(line_max_threads(NR))
     }
 }
 
+// One direction.
+template <bool XD, bool PER, int NR, int LL>
+__global__ void __launch_bounds__(line_max_threads(NR))
+    k_lsweep(const __grid_constant__ SweepArgs a, const __grid_constant__ LineArgs c)
+{
+    pdl_launch();
+    line_run<XD, PER, NR, LL>(a, c, blockIdx.x, gridDim.x);
+}
+
+// The x sweep (the first nx CTAs) and the y sweep of a 2-D stage in one launch, 8-line tiles.
+// Each is a fraction of a round on a small grid: one launch after another took 4.5 us each and
+// two streams a fork and a join.  (Forming the stresses while the second sweeps load them, which
+// would save a launch more, took 22 us a sweep against 11 and 2 for the stress kernel: each
+// thread forms sixteen of them, a division and a square root apiece, before its solve.)
+template <bool PERX, bool PERY, int NR>
+__global__ void __launch_bounds__(line_max_threads(NR))
+    k_lsweep_xy(const __grid_constant__ SweepArgs ax, const __grid_constant__ LineArgs cx,
+                const __grid_constant__ SweepArgs ay, const __grid_constant__ LineArgs cy, int nx)
+{
+    pdl_launch();
+    if ((int)blockIdx.x < nx) line_run<true, PERX, NR, 8>(ax, cx, blockIdx.x, nx);
+    else line_run<false, PERY, NR, 8>(ay, cy, blockIdx.x - nx, gridDim.x - nx);
+}
+
 // The instantiation for a direction, kind of line, band and lines per tile (4, 8, 16 or 32); null for
 // bands outside 2..7.  Defined in lsweep_x.cu and lsweep_yz.cu.
 void *line_kernel_x(bool per, int nR, int LL);
 void *line_kernel_yz(bool per, int nR, int LL);
+// k_lsweep_xy (lsweep_xy.cu)
+void *line_kernel_xy(bool perx, bool pery, int nR);
 
 template <bool XD, bool PER, int LL>
 void *pick_line_kernel(int nR)

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sweep.cuh"
+
 namespace gatt {
 
 // slot numbering of the per-member scratch sets
@@ -57,15 +59,15 @@ struct Forcings {
     double N[kMaxForcings];   // points of each box
     const double *sums;       // [member][kMaxForcings][5]: ET, U, V, W, E sums (turbulence)
     int nx, ny;
+    FastDiv fd_nx, fd_ny;     // dividers by the two
 };
 
 // k[] in U, V, W, R, E order; mom / en: apply the momentum (U, V, W) / energy rows only.
 __device__ __forceinline__ void apply_forcings(const Forcings &fs, int b, long long p, double u, double v,
                                                double w, double r, double e, double k[5], bool mom, bool en)
 {
-    const int i = (int)(p % fs.nx);
-    const long long jk = p / fs.nx;
-    const int j = (int)(jk % fs.ny), kz = (int)(jk / fs.ny);
+    // (a grid holds at most 2^31 points)
+    const int jk = fdiv((int)p, fs.fd_nx), i = (int)p - jk * fs.nx, kz = fdiv(jk, fs.fd_ny), j = jk - kz * fs.ny;
     for (int f = 0; f < fs.n; f++) {
         const int *bx = fs.box[f];
         if (i < bx[0] || i > bx[1] || j < bx[2] || j > bx[3] || kz < bx[4] || kz > bx[5]) continue;
@@ -256,6 +258,8 @@ __global__ void __launch_bounds__(256) k_visc3d_v2(Phys ph, StateSet q, FieldSet
 __global__ void k_visc2d(Phys ph, StateSet q, FieldSet d1, FieldSet tq, long long n)
 {
     const int b = blockIdx.y;
+    pdl_launch();
+    pdl_wait();
     const double *E = q.v[4] + b * q.bstride;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const double mu = sutherland_mu(ph, E[p]);
@@ -378,6 +382,8 @@ __global__ void k_assemble2d(Phys ph, StateSet q, StateSet q0, StateSet out, Fie
                              const StepParams *sp, Forcings fs)
 {
     const int b = blockIdx.y;
+    pdl_launch();
+    pdl_wait();
     const double dt = sp ? sp->dt : 0.0;
     const double g = ph.gamma;
     const double *U = q.v[0] + b * q.bstride, *V = q.v[1] + b * q.bstride;
@@ -420,6 +426,8 @@ __global__ void k_sfd(StateSet q, FieldSet mean, const double *chi, double delta
                       long long n, const StepParams *sp)
 {
     const int b = blockIdx.y;
+    pdl_launch();
+    pdl_wait();
     const double dt = sp->dt;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const double x = chi[p];
@@ -436,7 +444,7 @@ __global__ void k_sfd(StateSet q, FieldSet mean, const double *chi, double delta
 
 // max|a - b| per variable, accumulated with an unsigned 64-bit max on the IEEE bits of
 // the (non-negative) differences; a NaN (positive payload) wins over every number.
-__global__ void k_maxchange(StateSet a, StateSet bset, unsigned long long *acc, long long n)
+__device__ __forceinline__ void maxchange_block(const StateSet &a, const StateSet &bset, unsigned long long *acc, long long n)
 {
     const int b = blockIdx.y;
     __shared__ unsigned long long red[5][32];
@@ -472,6 +480,31 @@ __global__ void k_maxchange(StateSet a, StateSet bset, unsigned long long *acc, 
             if (lane == 0) atomicMax(acc + b * 5 + f, v);
         }
     }
+}
+
+__global__ void k_maxchange(StateSet a, StateSet bset, unsigned long long *acc, long long n)
+{
+    maxchange_block(a, bset, acc, n);
+}
+
+// The same with the step's row of the history written by the last CTA (done: CTAs that have
+// finished), which leaves acc and done zero for the next launch.
+__global__ void __launch_bounds__(256) k_maxchange_store(StateSet a, StateSet bset, unsigned long long *acc, unsigned *done,
+                                                         double *hist, long long n, const StepParams *sp)
+{
+    pdl_launch();
+    pdl_wait();
+    maxchange_block(a, bset, acc, n);
+    __shared__ bool last;
+    if (threadIdx.x < 32) __threadfence();  // the warp that added this CTA's maxima
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (!last) return;
+    const int nvals = 5 * gridDim.y;
+    for (int i = threadIdx.x; i < nvals; i += blockDim.x)
+        hist[sp->slot * nvals + i] = __longlong_as_double((long long)atomicExch(acc + i, 0ull));
+    if (threadIdx.x == 0) *done = 0;
 }
 
 // Max-change over independent (a, b) pointer sets: set s, variable v compares

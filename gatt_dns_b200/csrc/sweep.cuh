@@ -60,6 +60,11 @@ __device__ __forceinline__ int fdiv(int n, const FastDiv &f)
     return (int)((t + (uint32_t)n) >> f.l);
 }
 
+// Programmatic dependent launch: a kernel's blocks may start while the kernel before it in the
+// stream drains, and wait here before they touch anything it writes (no-ops otherwise).
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Per-row coefficient record, in the kernel's uniform row semantics:
 //   forward  y(r) = (rhs(r) - fA(r) y(r-1)) * fB(r)
 //   backward x(r) = y(r) - bC(r) x(r+1)
