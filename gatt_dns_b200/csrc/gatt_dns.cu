@@ -173,7 +173,11 @@ struct gatt_ctx {
     double *t_delta = nullptr, *t_d1 = nullptr, *t_tq = nullptr, *t_d2 = nullptr;  // tangent RK increment, 15, 9, 12
     double *a_lam = nullptr, *a_acc = nullptr, *a_arg = nullptr, *a_prev = nullptr, *a_g = nullptr;
     double *a_lq = nullptr, *a_ld1 = nullptr, *a_ltau = nullptr, *a_lvt = nullptr;  // 5, 15, 9, 4
-    double *a_s1 = nullptr, *a_s2 = nullptr, *a_scr = nullptr;                       // 15, 12, 5
+    double *a_s1 = nullptr, *a_s2 = nullptr, *a_scr[3] = {};                         // 15, 12, 5 each
+    // first derivatives and second sweeps of the stage states 1..3 of the adjoint's recomputed step
+    // (stage 0's stay in d1 / d2); null where there is no room: recomputed
+    double *a_sd1[3] = {}, *a_sd2[3] = {};
+    bool a_sd_full = false;
     double *a_ckpt = nullptr, *a_seg = nullptr;
     int a_nckpt = 0, a_nseg = 0;
     bool a_ckpt_sfd = false, a_seg_sfd = false;  // checkpoint / segment slots hold a mean too
@@ -925,7 +929,7 @@ LineArgs line_args(const gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, cons
 int launch_lsweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nf, int nmem, int cls)
 {
     const LinePlan pl = line_plan_for(c, m, d, nf, nmem, line_lanes(c, m, d));
-    if (!pl.LL || pl.jobs > INT_MAX / 2) return GATT_ERR_STATE;
+    if (!pl.LL || pl.jobs > INT_MAX / 2) return fail(GATT_ERR_STATE, "no launch plan for this line sweep");
     SweepArgs x = a;
     const LineArgs la = line_args(c, m, d, x, pl, nf);
     const int grid = (int)std::min<long long>(pl.jobs, (long long)pl.per_sm * c->nsm);
@@ -973,7 +977,7 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
     const bool few = m.family == FAM_PIPE && m.lQ && m.P >= 16 && (long long)a.ntiles * (c->is3d ? 5 : 4) < c->nsm;
     if (m.family == FAM_LINE || (few && !mc_ref) || (c->chain && m.lQ)) {
         const int r = launch_lsweep(c, m, d, a, nf, nmembers, cls);
-        if (r != GATT_ERR_STATE) return r;  // GATT_ERR_STATE: more tiles than a launch counts
+        if (r != GATT_ERR_STATE || m.family == FAM_LINE) return r;  // GATT_ERR_STATE: no plan for this launch
     }
     if (m.family == FAM_PIPE && m.rpb) {
         int r = launch_psweep(c, m, d, a, nmembers, cls);
@@ -1310,6 +1314,32 @@ int launch_assemble2d(gatt_ctx *c, StateSet q, StateSet q0, StateSet out, int mo
     const StepParams *sp = c->d_params;
     void *args[] = {&c->ph, &q, &q0, &out, &fd, &f1, &ft, &f2, &n, &mode, &sp, &fs};
     return launch_chained(c, PC_ASSEMBLE, (const void *)k_assemble2d, dim3(grid_for(c, n), nmem), dim3(kBlock), 0, args);
+}
+
+// launch(d) for every direction, the x direction's launches on the side stream and (3-D) the z
+// direction's on a third one beside the y direction's.
+template <typename F>
+int each_direction(gatt_ctx *c, F &&launch)
+{
+    const bool fork = c->fork_x && !c->profiling && c->side && (!c->is3d || c->side2);
+    if (!fork) {
+        for (int d = 0; d < (c->is3d ? 3 : 2); d++) TRY(launch(d));
+        return GATT_OK;
+    }
+    TRY(beside(c, [&] { return launch(0); }));
+    if (c->is3d) {
+        CU(cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
+        std::swap(c->stream, c->side2);
+        std::swap(c->tmp, c->tmp_side2);
+        const int r = launch(2);
+        std::swap(c->stream, c->side2);
+        std::swap(c->tmp, c->tmp_side2);
+        TRY(r);
+        CU(cudaEventRecord(c->ev_join2, c->side2));
+    }
+    TRY(launch(1));
+    if (c->is3d) CU(cudaStreamWaitEvent(c->stream, c->ev_join2, 0));
+    return join_side(c);
 }
 
 // nseq2d/nseq3d on stage input q, fused with the RK4 update into out (mode).
@@ -2390,7 +2420,7 @@ int diff_alloc(gatt_ctx *c, bool adjoint)
         if (diff_sfd(c)) TRY(alloc_zeroed(c, &c->dym, 5));
         return GATT_OK;
     }
-    double **five[] = {&c->a_lam, &c->a_acc, &c->a_arg, &c->a_prev, &c->a_g, &c->a_lq, &c->a_scr};
+    double **five[] = {&c->a_lam, &c->a_acc, &c->a_arg, &c->a_prev, &c->a_g, &c->a_lq, &c->a_scr[0], &c->a_scr[1], &c->a_scr[2]};
     for (double **p : five) TRY(alloc_zeroed(c, p, 5));
     TRY(alloc_zeroed(c, &c->a_ld1, D3_N));
     TRY(alloc_zeroed(c, &c->a_ltau, T3_N));
@@ -2402,6 +2432,25 @@ int diff_alloc(gatt_ctx *c, bool adjoint)
     if (diff_sfd(c)) {
         TRY(alloc_zeroed(c, &c->a_lm, 5));
         TRY(alloc_zeroed(c, &c->a_mscr, 5));
+    }
+    // the stage derivatives of a recomputed step, if there is room (81 fields a member); without them
+    // the reverse sweep forms three of the four again
+    if (!c->a_sd1[0] && !c->a_sd_full) {
+        int rc = GATT_OK;
+        for (int s = 0; s < 3 && rc == GATT_OK; s++) {
+            rc = alloc_zeroed(c, &c->a_sd1[s], D3_N);
+            if (rc == GATT_OK) rc = alloc_zeroed(c, &c->a_sd2[s], S3_N);
+        }
+        if (rc == GATT_ERR_NOMEM) {
+            cudaGetLastError();
+            for (int s = 0; s < 3; s++) {
+                cudaFree(c->a_sd1[s]); c->a_sd1[s] = nullptr;
+                cudaFree(c->a_sd2[s]); c->a_sd2[s] = nullptr;
+            }
+            c->a_sd_full = true;
+        } else if (rc != GATT_OK) {
+            return rc;
+        }
     }
     // five boundary-program tapes per step (after each stage and after the filter / SFD)
     const long long need = 5 * std::max(1LL, c->tape_len) * c->nb;
@@ -2458,28 +2507,30 @@ double *diff_d2(gatt_ctx *c) { return c->is3d ? c->d2 : c->g_d2; }
 // 3-D data flow without the z direction (x and y sweeps into the 3-D slots, the z slots stay
 // zero), so the stage matches nseq2d + RK4_2D to rounding and leaves the base data in the
 // 3-D layouts.
-int rhs_stage_d(gatt_ctx *c, const StateSet &q, const StateSet &q0, const StateSet &out, int mode,
+int rhs_stage_d(gatt_ctx *c, const StateSet &q, const StateSet &q0, const StateSet &out, int mode, double *d1, double *d2,
                 bool assemble = true)
 {
     const int nm = c->nb;
-    if (c->is3d) return rhs_stage(c, q, q0, out, mode, nm, c->d1, c->tq, c->d2, c->delta, assemble);
+    if (c->is3d) return rhs_stage(c, q, q0, out, mode, nm, d1, c->tq, d2, c->delta, assemble);
     const long long n = c->npts;
     const long long bd1 = D3_N * n, btq = T3_N * n, bd2 = S3_N * n;
     const int fin[5] = {0, 1, 2, 3, 4};
     const int ox[5] = {D3_UX, D3_VX, D3_WX, D3_RX, D3_EX};
     const int oy[5] = {D3_UY, D3_VY, D3_WY, D3_RY, D3_EY};
-    TRY(sweep(c, 0, 0, q.v[0], q.bstride, fin, c->g_d1, bd1, ox, 5, nm, 0, nullptr, PC_D1X));
-    TRY(sweep(c, 1, 0, q.v[0], q.bstride, fin, c->g_d1, bd1, oy, 5, nm, 0, nullptr, PC_D1Y));
+    TRY(each_direction(c, [&](int d) {
+        return sweep(c, d, 0, q.v[0], q.bstride, fin, d1, bd1, d ? oy : ox, 5, nm, 0, nullptr, PC_D1X + d);
+    }));
     TRY(before_launch(c, PC_VISC));
-    k_visc3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(c->ph, q, fset(c, c->g_d1, D3_N),
+    k_visc3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(c->ph, q, fset(c, d1, D3_N),
                                                                 fset(c, c->g_tq, T3_N), n);
     TRY(after_launch(c));
     const int ix[4] = {T3_XX, T3_XY, T3_XZ, T3_QX}, sx[4] = {S3_TXXX, S3_TXYX, S3_TXZX, S3_HTX};
     const int iy[4] = {T3_XY, T3_YY, T3_YZ, T3_QY}, sy[4] = {S3_TXYY, S3_TYYY, S3_TYZY, S3_HTY};
-    TRY(sweep(c, 0, 0, c->g_tq, btq, ix, c->g_d2, bd2, sx, 4, nm, 0, nullptr, PC_D2X));
-    TRY(sweep(c, 1, 0, c->g_tq, btq, iy, c->g_d2, bd2, sy, 4, nm, 0, nullptr, PC_D2Y));
+    TRY(each_direction(c, [&](int d) {
+        return sweep(c, d, 0, c->g_tq, btq, d ? iy : ix, d2, bd2, d ? sy : sx, 4, nm, 0, nullptr, PC_D2X + d);
+    }));
     if (!assemble) return GATT_OK;
-    return assemble3d(c, q, q0, out, mode, nm, c->g_d1, c->g_d2, c->delta);
+    return assemble3d(c, q, q0, out, mode, nm, d1, d2, c->delta);
 }
 
 // Tangent of one RK stage (mode 1..4, or RK_STORE_RHS for the bare RHS): the base stage
@@ -2489,16 +2540,17 @@ int tl_stage(gatt_ctx *c, const StateSet &xin, const StateSet &x0, const StateSe
 {
     const int nm = c->nb;
     const long long n = c->npts;
-    TRY(rhs_stage_d(c, xin, x0, xout, mode));
     double *d1 = diff_d1(c), *d2 = diff_d2(c);
+    TRY(rhs_stage_d(c, xin, x0, xout, mode, d1, d2));
     const long long bd1 = D3_N * n, btq = T3_N * n, bd2 = S3_N * n;
     const int fin[5] = {0, 1, 2, 3, 4};
     const int ox[5] = {D3_UX, D3_VX, D3_WX, D3_RX, D3_EX};
     const int oy[5] = {D3_UY, D3_VY, D3_WY, D3_RY, D3_EY};
     const int oz[5] = {D3_UZ, D3_VZ, D3_WZ, D3_RZ, D3_EZ};
-    TRY(sweep(c, 0, 0, yin.v[0], yin.bstride, fin, c->t_d1, bd1, ox, 5, nm, 0, nullptr, PC_D1X));
-    TRY(sweep(c, 1, 0, yin.v[0], yin.bstride, fin, c->t_d1, bd1, oy, 5, nm, 0, nullptr, PC_D1Y));
-    if (c->is3d) TRY(sweep(c, 2, 0, yin.v[0], yin.bstride, fin, c->t_d1, bd1, oz, 5, nm, 0, nullptr, PC_D1Z));
+    const int *const o1[3] = {ox, oy, oz};
+    TRY(each_direction(c, [&](int d) {
+        return sweep(c, d, 0, yin.v[0], yin.bstride, fin, c->t_d1, bd1, o1[d], 5, nm, 0, nullptr, PC_D1X + d);
+    }));
     TRY(before_launch(c, PC_VISC));
     k_tl_tau3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(c->ph, xin, fset(c, d1, D3_N), yin,
                                                                   fset(c, c->t_d1, D3_N), fset(c, c->t_tq, T3_N), n);
@@ -2506,9 +2558,10 @@ int tl_stage(gatt_ctx *c, const StateSet &xin, const StateSet &x0, const StateSe
     const int ix[4] = {T3_XX, T3_XY, T3_XZ, T3_QX}, sx[4] = {S3_TXXX, S3_TXYX, S3_TXZX, S3_HTX};
     const int iy[4] = {T3_XY, T3_YY, T3_YZ, T3_QY}, sy[4] = {S3_TXYY, S3_TYYY, S3_TYZY, S3_HTY};
     const int iz[4] = {T3_XZ, T3_YZ, T3_ZZ, T3_QZ}, sz[4] = {S3_TXZZ, S3_TYZZ, S3_TZZZ, S3_HTZ};
-    TRY(sweep(c, 0, 0, c->t_tq, btq, ix, c->t_d2, bd2, sx, 4, nm, 0, nullptr, PC_D2X));
-    TRY(sweep(c, 1, 0, c->t_tq, btq, iy, c->t_d2, bd2, sy, 4, nm, 0, nullptr, PC_D2Y));
-    if (c->is3d) TRY(sweep(c, 2, 0, c->t_tq, btq, iz, c->t_d2, bd2, sz, 4, nm, 0, nullptr, PC_D2Z));
+    const int *const i2[3] = {ix, iy, iz}, *const o2[3] = {sx, sy, sz};
+    TRY(each_direction(c, [&](int d) {
+        return sweep(c, d, 0, c->t_tq, btq, i2[d], c->t_d2, bd2, o2[d], 4, nm, 0, nullptr, PC_D2X + d);
+    }));
     TRY(before_launch(c, PC_ASSEMBLE));
     k_tl_assemble3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(
         c->ph, xin, fset(c, d1, D3_N), fset(c, d2, S3_N), yin, fset(c, c->t_d1, D3_N), fset(c, c->t_d2, S3_N), y0,
@@ -2561,18 +2614,17 @@ int sweep_T(gatt_ctx *c, int d, int k0, const double *in, long long in_bs, const
 {
     int sl[16];
     for (int f = 0; f < nf; f++) sl[f] = f;
-    TRY(sweep(c, d, k0, in, in_bs, in_slots, c->a_scr, 5 * c->npts, sl, nf, c->nb, 0.0, nullptr, PC_OTHER));
-    return sweep(c, d, k0 + 1, c->a_scr, 5 * c->npts, sl, out, out_bs, out_slots, nf, c->nb, 0.0, nullptr, PC_OTHER);
+    // (a scratch set per direction: the directions' sweeps run side by side)
+    TRY(sweep(c, d, k0, in, in_bs, in_slots, c->a_scr[d], 5 * c->npts, sl, nf, c->nb, 0.0, nullptr, PC_OTHER));
+    return sweep(c, d, k0 + 1, c->a_scr[d], 5 * c->npts, sl, out, out_bs, out_slots, nf, c->nb, 0.0, nullptr, PC_OTHER);
 }
 
-// G = F'(q)^T a (the adjoint of the RHS at state q)
-int adj_rhs(gatt_ctx *c, const StateSet &q, const StateSet &a, const StateSet &G)
+// G = F'(q)^T a (the adjoint of the RHS at state q, whose first derivatives and second sweeps are
+// d1 and d2).  2-D: no z direction, its slots of a_s1 / a_s2 stay zero.
+int adj_rhs(gatt_ctx *c, const StateSet &q, const StateSet &a, const StateSet &G, double *d1, double *d2)
 {
     const int nm = c->nb;
     const long long n = c->npts;
-    const int ndir = c->is3d ? 3 : 2;  // 2-D: no z direction, its slots of a_s1 / a_s2 stay zero
-    TRY(rhs_stage_d(c, q, q, q, RK_STORE_RHS, false));
-    double *d1 = diff_d1(c), *d2 = diff_d2(c);
     TRY(before_launch(c, PC_OTHER));
     k_adj_asm3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(
         c->ph, q, fset(c, d1, D3_N), fset(c, d2, S3_N), a, fset(c, c->a_lq, 5), fset(c, c->a_ld1, D3_N),
@@ -2580,21 +2632,21 @@ int adj_rhs(gatt_ctx *c, const StateSet &q, const StateSet &a, const StateSet &G
     TRY(after_launch(c));
     // transposed second sweeps: (vtx, vty, vtz, ht) -> stress / heat-flux contributions
     const int v4[4] = {0, 1, 2, 3};
-    for (int d = 0; d < ndir; d++) {
+    TRY(each_direction(c, [&](int d) {
         const int o4[4] = {4 * d, 4 * d + 1, 4 * d + 2, 4 * d + 3};
-        TRY(sweep_T(c, d, 2, c->a_lvt, 4 * n, v4, c->a_s2, 12 * n, o4, 4));
-    }
+        return sweep_T(c, d, 2, c->a_lvt, 4 * n, v4, c->a_s2, 12 * n, o4, 4);
+    }));
     TRY(before_launch(c, PC_OTHER));
     k_adj_tau3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(c->ph, q, fset(c, d1, D3_N),
                                                                    fset(c, c->a_ltau, T3_N), fset(c, c->a_s2, 12),
                                                                    fset(c, c->a_ld1, D3_N), fset(c, c->a_lq, 5), n);
     TRY(after_launch(c));
     // transposed first sweeps: gradient lambdas -> state lambdas
-    for (int d = 0; d < ndir; d++) {
+    TRY(each_direction(c, [&](int d) {
         const int i5[5] = {D3_UX + d, D3_VX + d, D3_WX + d, D3_RX + d, D3_EX + d};
         const int o5[5] = {5 * d, 5 * d + 1, 5 * d + 2, 5 * d + 3, 5 * d + 4};
-        TRY(sweep_T(c, d, 2, c->a_ld1, (long long)D3_N * n, i5, c->a_s1, 15 * n, o5, 5));
-    }
+        return sweep_T(c, d, 2, c->a_ld1, (long long)D3_N * n, i5, c->a_s1, 15 * n, o5, 5);
+    }));
     TRY(before_launch(c, PC_OTHER));
     k_adj_q3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(fset(c, c->a_lq, 5), fset(c, c->a_s1, 15), G, n);
     return after_launch(c);
@@ -2618,8 +2670,14 @@ int adj_step(gatt_ctx *c, double dt)
                            set5(c, c->dx[4])};
     // recompute the stage states q1..q4 (after their boundary conditions) and the end state,
     // recording the boundary program's tapes: 0..3 after the stages, 4 after filter and SFD
+    double *d1[4], *d2[4];  // the derivatives of q_0 .. q_3, which the reverse sweep reads again
+    const bool keep = c->a_sd1[0] != nullptr;
+    for (int s = 0; s < 4; s++) {
+        d1[s] = s && keep ? c->a_sd1[s - 1] : diff_d1(c);
+        d2[s] = s && keep ? c->a_sd2[s - 1] : diff_d2(c);
+    }
     for (int s = 1; s <= 4; s++) {
-        TRY(rhs_stage_d(c, X[s - 1], X[0], X[s], s));
+        TRY(rhs_stage_d(c, X[s - 1], X[0], X[s], s, d1[s - 1], d2[s - 1]));
         TRY(bc_rec(c, X[s], s - 1, s <= 2 ? 0.5 : 1.0));
     }
     if (c->nops > 0) {
@@ -2663,7 +2721,8 @@ int adj_step(gatt_ctx *c, double dt)
     for (int i = 0; i < 4; i++) {
         const int s = 3 - i;  // stage state q_s feeds k_{s+1}
         TRY(axpby5(c, c->a_arg, c->a_lam, i ? c->a_prev : nullptr, wl[i], wp[i]));
-        TRY(adj_rhs(c, X[s], A, G));
+        if (!keep && s < 3) TRY(rhs_stage_d(c, X[s], X[s], X[s], RK_STORE_RHS, d1[s], d2[s], false));
+        TRY(adj_rhs(c, X[s], A, G, d1[s], d2[s]));
         if (s > 0) TRY(bc_adj(c, G, s - 1));  // q_s came out of the boundary conditions of stage s
         TRY(axpby5(c, c->a_acc, c->a_acc, c->a_g, 1.0, 1.0));
         if (s > 0) TRY(copy_set5(c, c->a_prev, c->a_g));
@@ -2722,7 +2781,9 @@ int rhs_vjp(gatt_ctx *c, const double *q, const double *a, double *lam)
     TRY(diff_alloc(c, true));
     TRY(upload5(c, c->dx[0], q));
     TRY(upload5(c, c->a_arg, a));
-    TRY(adj_rhs(c, set5(c, c->dx[0]), set5(c, c->a_arg), set5(c, c->a_g)));
+    const StateSet X0 = set5(c, c->dx[0]);
+    TRY(rhs_stage_d(c, X0, X0, X0, RK_STORE_RHS, diff_d1(c), diff_d2(c), false));
+    TRY(adj_rhs(c, X0, set5(c, c->a_arg), set5(c, c->a_g), diff_d1(c), diff_d2(c)));
     TRY(zero_w(c, c->a_g));
     return download5(c, lam, c->a_g);
 }
@@ -2735,11 +2796,11 @@ int jvp(gatt_ctx *c, int nsteps, double t0, double dt, const double *dq0, double
     TRY(state_to_set(c, state_set(c, 0), c->dx[0], true));
     if (diff_sfd(c)) TRY(copy_set5(c, c->dxm, c->mean));
     TRY(upload_vec(c, c->dy[0], c->dym, dq0));
+    TRY(ensure_hist(c, nsteps));  // a parameter slot per step: no wait in between
     double t = t0;
     for (int s = 0; s < nsteps; s++) {
-        TRY(set_params(c, 0, t, dt));
+        TRY(set_params(c, s, t, dt));
         TRY(tl_step(c));
-        TRY(sync_stream(c));  // the parameter slot is reused
         t = t + dt;
     }
     TRY(state_to_set(c, state_set(c, 0), c->dx[0], false));
@@ -2783,6 +2844,7 @@ int vjp(gatt_ctx *c, int nsteps, double t0, double dt, int every, const double *
         TRY(state_to_set(c, state_set(c, 0), const_cast<double *>(src), false));
         return sfd ? copy_set5(c, c->mean, src + s5) : GATT_OK;
     };
+    TRY(ensure_hist(c, seg));
     // forward: checkpoints at steps 0, every, 2*every, ...; slot nck keeps the final state
     for (int k = 0; k < nck; k++) {
         TRY(save(c->a_ckpt + st * k));
@@ -2801,10 +2863,10 @@ int vjp(gatt_ctx *c, int nsteps, double t0, double dt, int every, const double *
         for (int i = len - 1; i >= 0; i--) {
             TRY(copy_set5(c, c->dx[0], c->a_seg + st * i));
             if (sfd) TRY(copy_set5(c, c->dxm, c->a_seg + st * i + s5));
-            TRY(set_params(c, 0, t0 + (double)(k * every + i) * dt, dt));
+            TRY(set_params(c, i, t0 + (double)(k * every + i) * dt, dt));
             TRY(adj_step(c, dt));
-            TRY(sync_stream(c));
         }
+        TRY(sync_stream(c));  // the forward steps of the next segment use the parameter slots
     }
     TRY(restore(c->a_ckpt + st * nck));
     return download_vec(c, lam0, c->a_lam, c->a_lm);
@@ -3031,7 +3093,8 @@ void gatt_destroy(gatt_ctx *c)
     for (double *p : c->dx) cudaFree(p);
     for (double *p : c->dy) cudaFree(p);
     double *dbufs[] = {c->t_delta, c->t_d1, c->t_tq, c->t_d2, c->a_lam, c->a_acc, c->a_arg, c->a_prev, c->a_g,
-                       c->a_lq, c->a_ld1, c->a_ltau, c->a_lvt, c->a_s1, c->a_s2, c->a_scr, c->a_ckpt, c->a_seg,
+                       c->a_lq, c->a_ld1, c->a_ltau, c->a_lvt, c->a_s1, c->a_s2, c->a_scr[0], c->a_scr[1], c->a_scr[2], c->a_sd1[0], c->a_sd1[1], c->a_sd1[2],
+                       c->a_sd2[0], c->a_sd2[1], c->a_sd2[2], c->a_ckpt, c->a_seg,
                        c->t_P, c->a_lP, c->a_tape, c->a_tmp, c->g_d1, c->g_tq, c->g_d2, c->dxm, c->dym,
                        c->a_lm, c->a_mscr};
     for (double *p : dbufs) cudaFree(p);
@@ -3152,7 +3215,8 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     int Np = padded_rows(c, d, N, nRHS, periodic);
     int rpb = choose_rpb(d, N, Np, nRHS, nTypes, (W + 3) / 4 * 4);
     const int want = choose_family();
-    const bool line = (want == FAM_LINE || (want == FAM_PIPE && !rpb)) && line_fits(d == 0, N, nRHS, 8);
+    const bool line = (want == FAM_LINE || (want == FAM_PIPE && !rpb)) && line_fits(d == 0, N, nRHS, 8) &&
+                      line_tiles(c, d, 4) * 16 * c->nb <= INT_MAX / 2;
     const int Npipe = rpb ? Np : N;  // a padded length the pipelined solver does not take is not kept
     if (line) { rpb = 0; Np = N; }  // (its records are its own; the others are the shared-tile solver's)
     const int P = rpb ? Np / rpb : choose_blocks(N, nRHS, (W + 3) / 4 * 4);
@@ -3163,7 +3227,9 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     m.periodic = periodic; m.nR = nRHS; m.nTypes = nTypes; m.N = N; m.W = W; m.Wp = (W + 3) / 4 * 4;
     m.hA = std::move(hA); m.hB = std::move(hB); m.hC = std::move(hC); m.hD = std::move(hD); m.hR = std::move(hR);
     m.Np = Npipe;
-    TRY(upload_records(c, m, P, rpb ? Np : N));
+    m.P = P; m.rows = N;
+    if (!line) TRY(upload_records(c, m, P, rpb ? Np : N));
+    else TRY(sync_stream(c));
     // (2-D: also for the chained step's sweeps)
     if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_fits(d == 0, N, nRHS, 8))) TRY(upload_line_records(c, m));
     m.rpb = rpb;

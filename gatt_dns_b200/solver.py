@@ -49,6 +49,7 @@ class GattDNS:
     def __init__(self, case: Case, nbatch: int = 1, stream=None):
         self.lib = _lib.load()
         self.case = case
+        self._vec = None  # the packed input of the last jvp / vjp
         self.nbatch = nbatch
         h = ctypes.c_void_p()
         _lib.check(self.lib.gatt_create(ctypes.byref(h), case.nx, case.ny, case.nz, nbatch), "gatt_create")
@@ -253,6 +254,14 @@ class GattDNS:
             flows = [flows]
         return np.concatenate([_f64(f[k]).ravel(order="F") for f in flows for k in ("U", "V", "W", "R", "E")])
 
+    def _joined(self, parts):
+        """The 1-D parts one after the other, in a buffer that the context's owner keeps (its pages
+        are touched once, not on every call); valid until the next call."""
+        n = sum(p.size for p in parts)
+        if self._vec is None or self._vec.size != n:
+            self._vec = np.empty(n)
+        return np.concatenate(parts, out=self._vec)
+
     def _unpack(self, vec):
         s = (self.case.nx, self.case.ny, self.case.nz)
         n = self.case.nx * self.case.ny * self.case.nz
@@ -281,12 +290,12 @@ class GattDNS:
     _MEAN_KEYS = ("mU", "mV", "mW", "mR", "mE")
 
     def _pack_vec(self, flows):
-        if not self.case.sfd_type:
-            return self._pack(flows)
         if isinstance(flows, dict):
             flows = [flows]
+        if not self.case.sfd_type:
+            return self._joined([_f64(f[k]).ravel(order="F") for f in flows for k in ("U", "V", "W", "R", "E")])
         z = np.zeros(self.case.npts)
-        return np.concatenate([_f64(f[k]).ravel(order="F") if k in f else z
+        return self._joined([_f64(f[k]).ravel(order="F") if k in f else z
                                for f in flows for k in ("U", "V", "W", "R", "E") + self._MEAN_KEYS])
 
     def _unpack_vec(self, vec):
@@ -303,14 +312,14 @@ class GattDNS:
         """Tangent over nsteps steps from the current state (which advances, as run()); with
         SFD the vectors carry the mean's tangent under the keys mU ... mE."""
         dv = self._pack_vec(dq0)
-        out = np.zeros_like(dv)
+        out = np.empty_like(dv)
         _lib.check(self.lib.gatt_jvp(self.h, nsteps, t0, dt, _dp(dv), _dp(out)), "gatt_jvp")
         return self._unpack_vec(out)
 
     def vjp(self, lamN, nsteps, t0, dt, checkpoint_every=20):
         """Adjoint over nsteps steps from the current state, checkpointed (mean keys as jvp)."""
         lv = self._pack_vec(lamN)
-        out = np.zeros_like(lv)
+        out = np.empty_like(lv)
         _lib.check(self.lib.gatt_vjp(self.h, nsteps, t0, dt, checkpoint_every, _dp(lv), _dp(out)), "gatt_vjp")
         return self._unpack_vec(out)
 
