@@ -884,11 +884,11 @@ LinePlan line_plan_for(const gatt_ctx *c, const DevDir &m, int d, int nf, int nm
 // Tile width, from the grid alone: it enters the order in which a line's blocks are joined, and a
 // batch member's arithmetic must be that of the member alone.  Counted for the fields of a first
 // derivative sweep of one member.  Wide tiles read the records at one address a warp instead of
-// 32/LL, narrow ones make more and smaller CTAs: 32 lines where they fill the SMs (y lines of the
-// 90x75x54 box: 15.4 us against 18.5 with 16 and 20.8 with 8), fewer for launches that would
-// leave SMs idle, and 8 for lines of 20 blocks and more, whose wide CTAs hold an SM alone
-// (400-point x lines of the plate boundary layer: 118 us against 137 with 16).  4 where 8-line
-// tiles just miss one round (800-point x lines, 152 tiles on 148 SMs: 21.7 us against 28.9).
+// 32/LL, narrow ones make more and smaller CTAs: 32 lines where they fill the SMs
+// (y lines of the 90x75x54 box: 15.4 us against 18.5 with 16 and 20.8 with 8), fewer for launches
+// that would leave SMs idle, and 8 for lines of 20 blocks and more, whose wide CTAs hold an SM
+// alone (400-point x lines of the plate boundary layer: 118 us against 137 with 16).  4 where
+// 8-line tiles just miss one round (800-point x lines, 152 tiles on 148 SMs: 21.7 us against 28.9).
 int line_lanes(const gatt_ctx *c, const DevDir &m, int d)
 {
     const char *e = getenv("GATT_LINES");  // 4, 8, 16 or 32 lines a tile, where they fit
@@ -973,7 +973,8 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
     }
     // lines of many blocks whose 32-line tiles leave SMs idle (the 300-point y lines of the 800x300
     // grid: 100 tiles of 19 blocks, 13.3 us against 15.3) run as 8-line tiles too
-    // (decided by the grid alone, as line_lanes; a chain takes no other solver)
+    // (decided by the grid alone: a batch member's arithmetic is that of the member alone; a chain
+    // takes no other solver)
     const bool few = m.family == FAM_PIPE && m.lQ && m.P >= 16 && (long long)a.ntiles * (c->is3d ? 5 : 4) < c->nsm;
     if (m.family == FAM_LINE || (few && !mc_ref) || (c->chain && m.lQ)) {
         const int r = launch_lsweep(c, m, d, a, nf, nmembers, cls);
@@ -1091,16 +1092,16 @@ struct XyPlan {
     size_t smem = 0;
 };
 
-XyPlan xy_plan(const gatt_ctx *c, int nf, int nmem)
+XyPlan xy_plan(const gatt_ctx *c, int nf, int nmem, int LL)
 {
     const DevDir &mx = c->mat[0][0], &my = c->mat[1][0];
     XyPlan p;
-    p.x = line_plan_for(c, mx, 0, nf, nmem, 8);
-    p.y = line_plan_for(c, my, 1, nf, nmem, 8);
+    p.x = line_plan_for(c, mx, 0, nf, nmem, LL);
+    p.y = line_plan_for(c, my, 1, nf, nmem, LL);
     if (!p.x.LL || !p.y.LL) return p;
-    void *k = line_kernel_xy(mx.periodic != 0, my.periodic != 0, mx.nR);
+    void *k = line_kernel_xy(mx.periodic != 0, my.periodic != 0, mx.nR, LL);
     if (!k || allow_smem(k, kMaxSmem) != GATT_OK) return p;
-    p.threads = (std::max(mx.lP, my.lP) * 8 + 31) / 32 * 32;
+    p.threads = (std::max(mx.lP, my.lP) * LL + 31) / 32 * 32;
     p.smem = std::max(p.x.smem, p.y.smem);
     p.per_sm = resident_ctas(k, p.threads, p.smem);
     if (p.per_sm > 0) p.kernel = k;
@@ -1119,14 +1120,16 @@ bool chained_2d(const gatt_ctx *c)
     for (int d = 0; d < 2; d++)
         if (c->filt[d] && !c->mat[d][1].lQ) return false;
     if (3 * mx.lP < 2 * my.lP || 3 * my.lP < 2 * mx.lP) return false;
-    const XyPlan p = xy_plan(c, 4, 1);
+    const XyPlan p = xy_plan(c, 4, 1, 8);
     return p.kernel && p.x.jobs + p.y.jobs <= (long long)p.per_sm * c->nsm;
 }
 
 int sweep_xy(gatt_ctx *c, const double *in, long long in_bs, const int *sx, const int *sy, double *out, long long out_bs,
              const int *ox, const int *oy, int nf, int nmem, int cls)
 {
-    const XyPlan p = xy_plan(c, nf, nmem);
+    // 8-line tiles for a member or two, 32-line ones for batches that fill the SMs with those
+    XyPlan p = xy_plan(c, nf, nmem, 32);
+    if (!p.kernel || p.x.jobs + p.y.jobs < c->nsm) p = xy_plan(c, nf, nmem, 8);
     if (!p.kernel || p.x.jobs + p.y.jobs > INT_MAX / 2) return fail(GATT_ERR_STATE, "x and y sweeps do not fit one launch");
     SweepArgs a[2];
     LineArgs la[2];

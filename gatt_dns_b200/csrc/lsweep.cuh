@@ -6,8 +6,10 @@
 // Same recurrences and block recombination as rsweep.cuh.  A thread keeps 16 rows of one line in
 // registers (plus NR-1 halo rows either side).  A warp holds LL lines times 32/LL row blocks, a
 // tile the ceil(N/16) blocks of LL lines; rows past the line's end are identity rows (host
-// records).  The blocks are joined in two steps: inside a warp by shuffles, across warps through
-// shared memory, one value and one propagator per warp and line.
+// records).  Narrow tiles (a warp holds four blocks or more) join the blocks in two steps, four to
+// a group by shuffles inside the warp and then group to group through shared memory; wide ones
+// block to block through shared memory, or (GROUPS) in the narrow ones' order, so that the x+y
+// sweep of a batch can take wide tiles and keep the bits of a member alone.
 //
 // Persistent CTAs walk the tiles.  A tile is staged in shared memory by 8-byte asynchronous
 // copies, which need no alignment beyond the element's and so take every grid: x lines
@@ -34,6 +36,9 @@ constexpr int kLineQ = 6;      // doubles of a compact row record: (fA, fB), (bC
 
 // Threads a CTA may have: bands of 6 and 7 take up to 128 registers a thread, the others 80.
 __host__ __device__ constexpr int line_max_threads(int nR) { return nR >= 6 ? 512 : 768; }
+// Launch bound of an instantiation: tiles narrower than 32 lines get 96 registers (their CTAs are
+// small; at 80 the solve spills).
+__host__ __device__ constexpr int line_bound(int nR, int LL) { return nR >= 6 ? 512 : LL == 32 ? 768 : 640; }
 
 // Pitch of an x line in shared memory (doubles).
 __host__ __device__ __forceinline__ int line_pitch(int N, int LL)
@@ -57,6 +62,9 @@ __host__ __device__ __forceinline__ int line_type_doubles(int P) { return P * (k
 // Doubles of one block of non-uniform band rows.
 __host__ __device__ __forceinline__ int line_band_doubles(int Wp) { return kLineRows * Wp + 2; }
 
+// Values of a line in an exchange region: its groups of four blocks (narrow tiles) or its blocks.
+__host__ __device__ __forceinline__ int line_slots(int P, int LL) { return LL <= 8 ? (P + 3) / 4 : P; }
+
 // Coefficients of a k_lsweep launch (SweepArgs holds the rest).
 struct LineArgs {
     const double *Q;   // [type][line_type_doubles]
@@ -71,8 +79,7 @@ struct LineArgs {
 __host__ __device__ __forceinline__ size_t line_smem_bytes(bool xd, int N, int P, int LL, int nst, int nspecial,
                                                            int Wp, bool stageS)
 {
-    const size_t nw = ((size_t)P * LL + 31) / 32;
-    size_t n = (size_t)nst * line_tile_doubles(xd, N, LL) + 5 * nw * LL + line_type_doubles(P);
+    size_t n = (size_t)nst * line_tile_doubles(xd, N, LL) + 5 * (size_t)line_slots(P, LL) * LL + line_type_doubles(P);
     if (stageS) n += (size_t)nspecial * line_band_doubles(Wp);
     return n * sizeof(double);
 }
@@ -87,7 +94,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // One direction's tiles job0, job0 + jstep, ...  a.Nreal: rows of a line, a.P: blocks, a.nst:
 // stages (1 or 2), a.tiles_per_row: y/z tiles of LL points per row of x, a.njobs: tiles x fields
 // x members.  The CTA's first ceil(P LL / 32) warps run it, the others leave.
-template <bool XD, bool PER, int NR, int LL>
+template <bool XD, bool PER, int NR, int LL, bool GROUPS>
 __device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, int job0, int jstep)
 {
     constexpr int H = NR - 1, W = 2 * NR - 1, WP = (W + 3) / 4 * 4, M = kLineRows, Q6 = kLineQ;
@@ -101,11 +108,14 @@ __device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, 
     const int l = lane & (LL - 1), sub = lane / LL;
     const int p = warp * BB + sub, sp = p * M;
     const int N = a.Nreal, P = a.P;
+    constexpr bool narrow = LL <= 8;     // a warp holds whole groups of four blocks
+    const int NS = line_slots(P, LL), sg = sub & 3, gi = narrow ? warp * (BB / 4) + (sub >> 2) : p >> 2;
+    const int ng = (P + 3) / 4;
     const int pitch = XD ? line_pitch(N, LL) : 0, tsize = line_tile_doubles(XD, N, LL);
     const int td = line_type_doubles(P), bd = line_band_doubles(WP);
 
     // coefficients: one type's records and (where they fit) the band rows
-    double *sx = lsm + a.nst * tsize, *sc = sx + 5 * nw * LL;
+    double *sx = lsm + a.nst * tsize, *sc = sx + 5 * NS * LL;
     auto stage_type = [&](int t0) {
         for (int i = threadIdx.x; i < td; i += T) cp_async8(sc + i, c.Q + t0 * td + i);
     };
@@ -266,12 +276,29 @@ __device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, 
 #pragma unroll
         for (int j = 0; j < M; j++) dot = j == 0 ? w[0] * Qr[4] : dot + w[j] * Qr[j * Q6 + 4];
         if (p >= P) dot = 0.0;
+        // a group's sum is (d0 + d2) + (d1 + d3)
+        if constexpr (narrow) {
+            dot = dot + __shfl_xor_sync(0xffffffffu, dot, 2 * LL);
+            dot = dot + __shfl_xor_sync(0xffffffffu, dot, LL);
+            if (sg == 0 && gi < ng) xs[gi * LL] = dot;
+            sync();
+            x1 = xs[0];
+            for (int k = 1; k < ng; k++) x1 = x1 + xs[k * LL];
+        } else {
+            if (p < P) xs[p * LL] = dot;
+            sync();
+            if constexpr (!GROUPS) {
+                x1 = xs[0];
+                for (int k = 1; k < P; k++) x1 = x1 + xs[k * LL];
+            }
+            for (int k = 0; GROUPS && k < ng; k++) {
+                double d[4];
 #pragma unroll
-        for (int o = 16; o >= LL; o >>= 1) dot = dot + __shfl_xor_sync(0xffffffffu, dot, o);
-        if (sub == 0) xs[warp * LL] = dot;
-        sync();
-        x1 = xs[0];
-        for (int k = 1; k < nw; k++) x1 = x1 + xs[k * LL];
+                for (int q = 0; q < 4; q++) d[q] = 4 * k + q < P ? xs[(4 * k + q) * LL] : 0.0;
+                const double g = (d[0] + d[2]) + (d[1] + d[3]);
+                x1 = k ? x1 + g : g;
+            }
+        }
         cc = *reinterpret_cast<const double2 *>(Qt + td - 2);
         jl = N - 1 - sp;  // the line's last row in this block, if it is here
     }
@@ -293,19 +320,44 @@ __device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, 
     double Y = 0.0;
     {
         const double e = yprev, pe = Qr[(M - 1) * Q6 + 3];
-        double yl = 0.0, pl = 1.0;
+        double yl = 0.0, pl = 1.0, Yw = 0.0;
+        double *const se = xs + NS * LL, *const sp_ = xs + 2 * NS * LL;
+        if constexpr (narrow) {
 #pragma unroll
-        for (int s = 1; s < BB; s++) {
-            const double ue = __shfl_up_sync(0xffffffffu, e + pe * yl, LL), up = __shfl_up_sync(0xffffffffu, pe * pl, LL);
-            if (sub == s) { yl = ue; pl = up; }
+            for (int s = 1; s < 4; s++) {
+                const double ue = __shfl_up_sync(0xffffffffu, e + pe * yl, LL), up = __shfl_up_sync(0xffffffffu, pe * pl, LL);
+                if (sg == s) { yl = ue; pl = up; }
+            }
+            if (sg == 3 && gi < ng) {
+                se[gi * LL] = e + pe * yl;
+                sp_[gi * LL] = pe * pl;
+            }
+            sync();
+            for (int k = 0; k < gi; k++) Yw = se[k * LL] + sp_[k * LL] * Yw;
+        } else {
+            if (p < P) {
+                se[p * LL] = e;
+                sp_[p * LL] = pe;
+            }
+            sync();
+            if constexpr (!GROUPS)
+                for (int k = 0; k < p; k++) Yw = se[k * LL] + sp_[k * LL] * Yw;
+            for (int k = 0; GROUPS && k < gi; k++) {
+                double ge = 0.0, gp = 1.0;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const double ek = se[(4 * k + q) * LL], pk = sp_[(4 * k + q) * LL];
+                    ge = ek + pk * ge;
+                    gp = pk * gp;
+                }
+                Yw = ge + gp * Yw;
+            }
+            for (int k = 4 * gi; GROUPS && k < p; k++) {
+                const double ek = se[k * LL], pk = sp_[k * LL];
+                yl = ek + pk * yl;
+                pl = pk * pl;
+            }
         }
-        if (sub == BB - 1) {
-            xs[(nw + warp) * LL] = e + pe * yl;
-            xs[(2 * nw + warp) * LL] = pe * pl;
-        }
-        sync();
-        double Yw = 0.0;
-        for (int k = 0; k < warp; k++) Yw = xs[(nw + k) * LL] + xs[(2 * nw + k) * LL] * Yw;
         Y = yl + pl * Yw;
     }
     double xprev = 0.0;
@@ -321,19 +373,45 @@ __device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, 
     double X = 0.0;
     {
         const double e = p < P ? xprev : 0.0, re = Qr[5];
-        double xl = 0.0, pl = 1.0;
+        double xl = 0.0, pl = 1.0, Xw = 0.0;
+        double *const se = xs + 3 * NS * LL, *const sr = xs + 4 * NS * LL;
+        if constexpr (narrow) {
 #pragma unroll
-        for (int s = BB - 2; s >= 0; s--) {
-            const double ue = __shfl_down_sync(0xffffffffu, e + re * xl, LL), up = __shfl_down_sync(0xffffffffu, re * pl, LL);
-            if (sub == s) { xl = ue; pl = up; }
+            for (int s = 2; s >= 0; s--) {
+                const double ue = __shfl_down_sync(0xffffffffu, e + re * xl, LL), up = __shfl_down_sync(0xffffffffu, re * pl, LL);
+                if (sg == s) { xl = ue; pl = up; }
+            }
+            if (sg == 0 && gi < ng) {
+                se[gi * LL] = e + re * xl;
+                sr[gi * LL] = re * pl;
+            }
+            sync();
+            for (int k = ng - 1; k > gi; k--) Xw = se[k * LL] + sr[k * LL] * Xw;
+        } else {
+            if (p < P) {
+                se[p * LL] = e;
+                sr[p * LL] = re;
+            }
+            sync();
+            if constexpr (!GROUPS)
+                for (int k = P - 1; k > p; k--) Xw = se[k * LL] + sr[k * LL] * Xw;
+            for (int k = ng - 1; GROUPS && k > gi; k--) {
+                double ge = 0.0, gp = 1.0;
+#pragma unroll
+                for (int q = 3; q >= 0; q--) {
+                    if (4 * k + q >= P) continue;
+                    const double ek = se[(4 * k + q) * LL], rk = sr[(4 * k + q) * LL];
+                    ge = ek + rk * ge;
+                    gp = rk * gp;
+                }
+                Xw = ge + gp * Xw;
+            }
+            for (int k = min(4 * gi + 3, P - 1); GROUPS && k > p; k--) {
+                const double ek = se[k * LL], rk = sr[k * LL];
+                xl = ek + rk * xl;
+                pl = rk * pl;
+            }
         }
-        if (sub == 0) {
-            xs[(3 * nw + warp) * LL] = e + re * xl;
-            xs[(4 * nw + warp) * LL] = re * pl;
-        }
-        sync();
-        double Xw = 0.0;
-        for (int k = nw - 1; k > warp; k--) Xw = xs[(3 * nw + k) * LL] + xs[(4 * nw + k) * LL] * Xw;
         X = xl + pl * Xw;
     }
 #pragma unroll
@@ -398,34 +476,34 @@ __device__ __forceinline__ void line_run(const SweepArgs &a, const LineArgs &c, 
 
 // One direction.
 template <bool XD, bool PER, int NR, int LL>
-__global__ void __launch_bounds__(line_max_threads(NR))
+__global__ void __launch_bounds__(line_bound(NR, LL))
     k_lsweep(const __grid_constant__ SweepArgs a, const __grid_constant__ LineArgs c)
 {
     pdl_launch();
-    line_run<XD, PER, NR, LL>(a, c, blockIdx.x, gridDim.x);
+    line_run<XD, PER, NR, LL, false>(a, c, blockIdx.x, gridDim.x);
 }
 
-// The x sweep (the first nx CTAs) and the y sweep of a 2-D stage in one launch, 8-line tiles.
+// The x sweep (the first nx CTAs) and the y sweep of a 2-D stage in one launch, LL-line tiles.
 // Each is a fraction of a round on a small grid: one launch after another took 4.5 us each and
 // two streams a fork and a join.  (Forming the stresses while the second sweeps load them, which
 // would save a launch more, took 22 us a sweep against 11 and 2 for the stress kernel: each
 // thread forms sixteen of them, a division and a square root apiece, before its solve.)
-template <bool PERX, bool PERY, int NR>
-__global__ void __launch_bounds__(line_max_threads(NR))
+template <bool PERX, bool PERY, int NR, int LL>
+__global__ void __launch_bounds__(line_bound(NR, LL))
     k_lsweep_xy(const __grid_constant__ SweepArgs ax, const __grid_constant__ LineArgs cx,
                 const __grid_constant__ SweepArgs ay, const __grid_constant__ LineArgs cy, int nx)
 {
     pdl_launch();
-    if ((int)blockIdx.x < nx) line_run<true, PERX, NR, 8>(ax, cx, blockIdx.x, nx);
-    else line_run<false, PERY, NR, 8>(ay, cy, blockIdx.x - nx, gridDim.x - nx);
+    if ((int)blockIdx.x < nx) line_run<true, PERX, NR, LL, true>(ax, cx, blockIdx.x, nx);
+    else line_run<false, PERY, NR, LL, true>(ay, cy, blockIdx.x - nx, gridDim.x - nx);
 }
 
 // The instantiation for a direction, kind of line, band and lines per tile (4, 8, 16 or 32); null for
 // bands outside 2..7.  Defined in lsweep_x.cu and lsweep_yz.cu.
 void *line_kernel_x(bool per, int nR, int LL);
 void *line_kernel_yz(bool per, int nR, int LL);
-// k_lsweep_xy (lsweep_xy.cu)
-void *line_kernel_xy(bool perx, bool pery, int nR);
+// k_lsweep_xy, tiles of 8 or 32 lines (lsweep_xy.cu)
+void *line_kernel_xy(bool perx, bool pery, int nR, int LL);
 
 template <bool XD, bool PER, int LL>
 void *pick_line_kernel(int nR)

@@ -603,8 +603,11 @@ __global__ void __launch_bounds__(WIDE ? 32 * kMaxPx : ((NR == 6 && !XD) ? 32 * 
         const double *stg = psm + s * stage_d;
         const bool late = !mbar_wait(bar0 + 8 * s, par);
 
-        // window rows from the stage
+        // window rows from the stage; the halo rows are the neighbouring blocks' (N is a whole
+        // number of blocks), the other end's for cyclic lines, zero outside the others
         double w[NW];
+        const int hlo = p > 0 ? p - 1 : P - 1, hhi = p < P - 1 ? p + 1 : 0;
+        const bool lo = PER || p > 0, hi = PER || p < P - 1;
         // x: row r of this lane's line sits in chunk r/16, line row `lane`, 16-byte unit
         // (r%16)/2 XOR (lane%8); y/z: row r at [r][lane]
         auto xoff = [&](int r) {
@@ -623,13 +626,19 @@ __global__ void __launch_bounds__(WIDE ? 32 * kMaxPx : ((NR == 6 && !XD) ? 32 * 
             }
 #pragma unroll
             for (int kk = 0; kk < H; kk++) {
-                w[kk] = halo_row<PER>(sp - H + kk, N, lds);
-                w[H + RPB + kk] = halo_row<PER>(sp + RPB + kk, N, lds);
+                w[kk] = lo ? stg[(hlo * kLanes + lane) * RPB + ((((RPB - H + kk) >> 1) ^ (lane & 7)) << 1) + ((RPB - H + kk) & 1)] : 0.0;
+                w[H + RPB + kk] = hi ? stg[(hhi * kLanes + lane) * RPB + (((kk >> 1) ^ (lane & 7)) << 1) + (kk & 1)] : 0.0;
             }
         } else {
+            const double *own = stg + sp * kLanes + lane, *before = stg + (hlo * RPB + RPB - H) * kLanes + lane,
+                         *after = stg + hhi * RPB * kLanes + lane;
 #pragma unroll
-            for (int kk = 0; kk < NW; kk++)
-                w[kk] = (kk >= H && kk < H + RPB) ? lds(sp - H + kk) : halo_row<PER>(sp - H + kk, N, lds);
+            for (int kk = 0; kk < RPB; kk++) w[H + kk] = own[kk * kLanes];
+#pragma unroll
+            for (int kk = 0; kk < H; kk++) {
+                w[kk] = lo ? before[kk * kLanes] : 0.0;
+                w[H + RPB + kk] = hi ? after[kk * kLanes] : 0.0;
+            }
         }
         if (wstore && lane == 0) bulk_wait_read0();  // this warp's last store has read its stage
         if (__syncthreads_or(late)) {
