@@ -205,7 +205,8 @@ struct gatt_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double *tmp_side = nullptr;  // the side stream's scratch field (the global-memory line solver)
     cudaStream_t side2 = nullptr;  // 3-D: the z sweep beside the y sweep where they are two launches
-    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;
+    cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr, ev_sums = nullptr;
+    bool sums_ahead = false;       // this stage's forcing sums are under way on it (ev_sums)
     double *tmp_side2 = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -1199,11 +1200,16 @@ Forcings forcing_args(const gatt_ctx *c)
     return f;
 }
 
-int forcing_sums(gatt_ctx *c, const StateSet &q, int nmem)
+bool has_turbulence(const gatt_ctx *c)
 {
     bool turb = false;
     for (int f = 0; f < c->fc.n; f++) turb |= c->fc.type[f] == FORCE_TURBULENCE;
-    if (!turb) return GATT_OK;
+    return turb;
+}
+
+int forcing_sums(gatt_ctx *c, const StateSet &q, int nmem)
+{
+    if (!has_turbulence(c)) return GATT_OK;
     TRY(before_launch(c, PC_OTHER));
     k_forcing_sums<<<dim3(c->fblocks, nmem), 256, 0, c->stream>>>(q, forcing_args(c), c->fpart, c->fdone, c->fsum);
     return after_launch(c);
@@ -1257,7 +1263,9 @@ int assemble3d(gatt_ctx *c, const StateSet &q, const StateSet &q0, const StateSe
 {
     const long long n = c->npts;
     const FieldSet fd = fset(c, delta, 5), f1 = fset(c, d1, D3_N), f2 = fset(c, d2, S3_N);
-    TRY(forcing_sums(c, q, nmem));
+    if (!c->sums_ahead) TRY(forcing_sums(c, q, nmem));
+    else CU(cudaStreamWaitEvent(c->stream, c->ev_sums, 0));
+    c->sums_ahead = false;
     const int pr = launch_assemble3d_pipe(c, q, q0, out, fd, f1, f2, mode, nmem);
     if (pr != GATT_ERR_STATE) return pr;
     TRY(before_launch(c, PC_ASSEMBLE));
@@ -1360,6 +1368,18 @@ int rhs_stage(gatt_ctx *c, const StateSet &q, const StateSet &q0, const StateSet
         const int ox[5] = {D3_UX, D3_VX, D3_WX, D3_RX, D3_EX};
         const int oy[5] = {D3_UY, D3_VY, D3_WY, D3_RY, D3_EY};
         const int oz[5] = {D3_UZ, D3_VZ, D3_WZ, D3_RZ, D3_EZ};
+        // the forcings' box sums of the stage input run beside the sweeps (64^3: 8 us a stage)
+        c->sums_ahead = false;
+        if (assemble && has_turbulence(c) && c->fork_x && !c->profiling && c->side2) {
+            CU(cudaEventRecord(c->ev_fork2, c->stream));
+            CU(cudaStreamWaitEvent(c->side2, c->ev_fork2, 0));
+            std::swap(c->stream, c->side2);
+            const int r = forcing_sums(c, q, nmem);
+            std::swap(c->stream, c->side2);
+            TRY(r);
+            CU(cudaEventRecord(c->ev_sums, c->side2));
+            c->sums_ahead = true;
+        }
         TRY(beside(c, [&] { return sweep(c, 0, 0, qin, qbs, fin, d1, bd1, ox, 5, nmem, 0, nullptr, PC_D1X); }));
         TRY(sweep_yz(c, qin, qbs, fin, fin, d1, bd1, oy, oz, 5, nmem, PC_D1Y, PC_D1Z, PC_D1YZ));
         TRY(join_side(c));
@@ -3039,6 +3059,7 @@ int gatt_create(gatt_ctx **out, int nx, int ny, int nz, int nbatch)
             if (es == cudaSuccess) es = cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking);
             if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_fork2, cudaEventDisableTiming);
             if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming);
+            if (es == cudaSuccess) es = cudaEventCreateWithFlags(&c->ev_sums, cudaEventDisableTiming);
         }
         if (es != cudaSuccess && rc == GATT_OK) rc = fail(GATT_ERR_CUDA, cudaGetErrorString(es));
     }
@@ -3112,6 +3133,7 @@ void gatt_destroy(gatt_ctx *c)
     if (c->side2) cudaStreamDestroy(c->side2);
     if (c->ev_fork2) cudaEventDestroy(c->ev_fork2);
     if (c->ev_join2) cudaEventDestroy(c->ev_join2);
+    if (c->ev_sums) cudaEventDestroy(c->ev_sums);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     delete c;
