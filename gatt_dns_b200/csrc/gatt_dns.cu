@@ -134,15 +134,19 @@ struct gatt_ctx {
     std::vector<double> coef1, coef2;
     std::vector<Dist> dists;
     std::vector<double> distx;
-    // two forms of it (bc.cuh): d_prog[0] for steps and the tangent, d_prog[1] (the scratch-field
-    // ops) for the recorded program and its adjoint
+    // forms of it (bc.cuh): d_prog[0] whole, d_prog[1] of scratch-field ops for the recorded program
+    // and its adjoint, d_prog[2] without the Dirichlet values, for stages whose assembly sets them
     struct BcDev {
         BcOp *ops = nullptr;
         unsigned *lev = nullptr;
         int nops = 0, nlev = 0;
         long long widest = 0;  // points of the largest level
         std::vector<unsigned> begin, points;  // the levels' first ops (and nops), their points
-    } d_prog[2];
+    } d_prog[3];
+    uint8_t *d_cls = nullptr;        // the Dirichlet values by point (FixedPoints), null: not held so
+    FixedClass *d_clstab = nullptr;
+    bool fix_in_stage = false;       // the assembly being launched sets them
+    double *wset = nullptr;          // (2-D: and W's there)
     int nops = 0;
     double *d_coef1 = nullptr, *d_coef2 = nullptr, *d_xs = nullptr;
     // holdInlet: the values the first gatt_apply_bc kept, hold_len per member, laid out as the
@@ -1323,7 +1327,11 @@ int launch_assemble2d(gatt_ctx *c, StateSet q, StateSet q0, StateSet out, int mo
     Forcings fs = forcing_args(c);
     long long n = c->npts;
     const StepParams *sp = c->d_params;
-    void *args[] = {&c->ph, &q, &q0, &out, &fd, &f1, &ft, &f2, &n, &mode, &sp, &fs};
+    FixedPoints fixed;
+    fixed.cls = c->fix_in_stage ? c->d_cls : nullptr;
+    fixed.tab = c->d_clstab;
+    double *wset = c->wset;
+    void *args[] = {&c->ph, &q, &q0, &out, &fd, &f1, &ft, &f2, &n, &mode, &sp, &fs, &fixed, &wset};
     return launch_chained(c, PC_ASSEMBLE, (const void *)k_assemble2d, dim3(grid_for(c, n), nmem), dim3(kBlock), 0, args);
 }
 
@@ -1570,10 +1578,54 @@ int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict
     return GATT_OK;
 }
 
+// The Dirichlet values as a class per point (FixedPoints); more than 255 classes: not held so.
+struct FixedBox {
+    BcBox box;
+    int var;
+    double val;
+};
+int upload_fixed_points(gatt_ctx *c, const std::vector<FixedBox> &boxes)
+{
+    cudaFree(c->d_cls); c->d_cls = nullptr;
+    cudaFree(c->d_clstab); c->d_clstab = nullptr;
+    if (boxes.empty() || c->is3d) return GATT_OK;  // (2-D stages: see FixedPoints)
+    std::vector<uint8_t> cls((size_t)c->npts, 0);
+    std::vector<FixedClass> tab(1, FixedClass{});
+    for (const FixedBox &f : boxes) {
+        int to[256];  // class a point of this box moves to, by its class before
+        std::fill(to, to + 256, -1);
+        for (int k = f.box[4] - 1; k < f.box[5]; k++)
+            for (int j = f.box[2] - 1; j < f.box[3]; j++) {
+                uint8_t *row = &cls[(size_t)c->nx * (j + (size_t)c->ny * k)];
+                for (int i = f.box[0] - 1; i < f.box[1]; i++) {
+                    int &t = to[row[i]];
+                    if (t < 0) {
+                        FixedClass n = tab[row[i]];
+                        n.mask |= 1u << f.var;
+                        n.val[f.var] = f.val;
+                        for (size_t q = 1; q < tab.size() && t < 0; q++)
+                            if (tab[q].mask == n.mask && !memcmp(tab[q].val, n.val, sizeof(n.val))) t = (int)q;
+                        if (t < 0) {
+                            if (tab.size() > 255) return GATT_OK;
+                            t = (int)tab.size();
+                            tab.push_back(n);
+                        }
+                    }
+                    row[i] = (uint8_t)t;
+                }
+            }
+    }
+    CU(cudaMalloc(&c->d_cls, cls.size()));
+    CU(cudaMemcpy(c->d_cls, cls.data(), cls.size(), cudaMemcpyHostToDevice));
+    CU(cudaMalloc(&c->d_clstab, tab.size() * sizeof(FixedClass)));
+    CU(cudaMemcpy(c->d_clstab, tab.data(), tab.size() * sizeof(FixedClass), cudaMemcpyHostToDevice));
+    return GATT_OK;
+}
+
 int build_bc_program(gatt_ctx *c)
 {
     constexpr unsigned R = 1u << 3, E = 1u << 4, P = 1u << 5;
-    std::vector<HostBcOp> ops[2];  // with fused pressure items and corners, and in scratch form
+    std::vector<HostBcOp> ops[3];  // with fused pressure items and corners, in scratch form, and d_prog[2]'s
     auto mk = [&](int code, int var, const int *box) {
         HostBcOp o;
         memset(&o.op, 0, sizeof(o.op));
@@ -1636,9 +1688,11 @@ int build_bc_program(gatt_ctx *c)
             over.push_back(bx);
         }
     }
+    std::vector<FixedBox> fixed_points;
     for (int v : order)
         for (const auto &f : fixed[v]) {
             HostBcOp o = mk(OP_SET, v, f.first.data()); o.op.val = f.second; both(o, 0, 1u << v);
+            fixed_points.push_back({f.first, v, f.second});
         }
     for (const auto &f : fixed[GATT_VAR_R]) {
         std::vector<BcBox> constant;
@@ -1648,11 +1702,13 @@ int build_bc_program(gatt_ctx *c)
             constant.push_back(in);
             HostBcOp o = mk(OP_SET, GATT_VAR_R, in.data()); o.op.val = f.second / (c->ph.gamma - 1.0) / e.second;
             both(o, 0, R);
+            fixed_points.push_back({in, (int)GATT_VAR_R, o.op.val});
         }
         for (const BcBox &piece : box_minus(f.first, constant)) {
             HostBcOp o = mk(OP_DIR_P, GATT_VAR_R, piece.data()); o.op.val = f.second; both(o, E, R);
         }
     }
+    const size_t nfixed = ops[0].size();
     // P <- its extrapolation along dir at the face of box (P loaded over ext before)
     auto p_neumann = [&](int var, const int *bx, int dir, int len, int coef) {
         HostBcOp o = extrapolate(OP_P_NEU, var, bx, dir, len, coef);
@@ -1779,6 +1835,11 @@ int build_bc_program(gatt_ctx *c)
                 (o.box[5] - o.box[4] + 1);
     }
     c->tape_len = tape;
+    TRY(upload_fixed_points(c, fixed_points));
+    // (pressure Dirichlet values where E is not constant stay ops)
+    for (size_t i = 0; i < ops[0].size(); i++)
+        if (i >= nfixed || ops[0][i].op.code != OP_SET) ops[2].push_back(ops[0][i]);
+    TRY(upload_bc_levels(c->d_prog[2], ops[2], false));
     TRY(upload_bc_levels(c->d_prog[0], ops[0], false));
     TRY(upload_bc_levels(c->d_prog[1], ops[1], true));
     c->nops = c->d_prog[0].nops;
@@ -1894,23 +1955,23 @@ int launch_bc(gatt_ctx *c, void (*kblock)(KArgs...), void (*kcluster)(KArgs...),
 // Levels of a program up to which each is a launch of its own over the whole GPU, chained: a
 // cluster's 16 SMs took 56 us an application on the 400x150x64 plate (five levels, the widest
 // 176 000 points) against 12, and even the two small levels of the 128^2 cavity 6 us in one
-// launch against 2 and 2.
+// launch against 2.4 in two.
 constexpr int kBcLaunches = 16;
 
 // applyBoundCond at time t + tfac dt of the step (timeIntegration.F90 passes t + dt/2 or
 // t + dt by stage); fixed: at time tfix, keeping the holdInlet values on a first call
-int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed = false, double tfix = 0.0)
+int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed = false, double tfix = 0.0, int form = 0)
 {
     if (c->bc_dirty) TRY(build_bc_program(c));
-    if (c->nops == 0) return GATT_OK;
-    BcProgram pg = bc_program(c, tfac);
+    const gatt_ctx::BcDev &d = c->d_prog[form];
+    if (d.nops == 0) return GATT_OK;
+    BcProgram pg = bc_program(c, tfac, form);
     if (fixed) {
         pg.sp = nullptr; pg.tfix = tfix;
         pg.hold_save = c->hold_saved ? 0 : 1;
     } else if (c->hold_len > 0 && !c->hold_saved) {
         return fail(GATT_ERR_STATE, "holdInlet: call gatt_apply_bc on the initial state before stepping");
     }
-    const gatt_ctx::BcDev &d = c->d_prog[0];
     if (c->bc_cluster && d.nlev <= kBcLaunches) {
         // one launch per level, chained
         const int chain = c->chain;
@@ -1932,7 +1993,7 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
         c->chain = chain ? 2 : 0;
         return rc;
     }
-    return launch_bc(c, k_bc, k_bc_cluster, c->bc_cluster, nmem, 0, pg, q, c->P, (long long)c->npts);
+    return launch_bc(c, k_bc, k_bc_cluster, c->bc_cluster, nmem, form, pg, q, c->P, (long long)c->npts);
 }
 
 // applyFilters2D/3D in place on set q (derivs.F90:303-552)
@@ -2030,8 +2091,14 @@ int step_body(gatt_ctx *c)
     // conditions (timeIntegration.F90)
     bool first = true;
     for (const Stage &s : stages_of(c)) {
-        TRY(rhs_stage(c, first ? q0 : qs, q0, qs, s.mode, nm, c->d1, c->tq, c->d2, c->delta));
-        TRY(apply_bc(c, qst, nm, s.tfac));
+        // (2-D) the assembly sets the Dirichlet values, the program that follows the rest
+        c->fix_in_stage = c->d_cls != nullptr;
+        c->wset = qst.v[2];
+        const int r = rhs_stage(c, first ? q0 : qs, q0, qs, s.mode, nm, c->d1, c->tq, c->d2, c->delta);
+        const int form = c->fix_in_stage ? 2 : 0;
+        c->fix_in_stage = false;
+        TRY(r);
+        TRY(apply_bc(c, qst, nm, s.tfac, false, 0.0, form));
         first = false;
     }
     // nothing after the filter (no SFD, no boundary program): its last sweep can take the
@@ -3124,7 +3191,7 @@ void gatt_destroy(gatt_ctx *c)
     for (double *p : dbufs) cudaFree(p);
     for (double *p : bufs) cudaFree(p);
     for (gatt_ctx::BcDev &d : c->d_prog) { cudaFree(d.ops); cudaFree(d.lev); }
-    cudaFree(c->acc); cudaFree(c->mc_acc); cudaFree(c->d_params);
+    cudaFree(c->acc); cudaFree(c->mc_acc); cudaFree(c->d_cls); cudaFree(c->d_clstab); cudaFree(c->d_params);
     cudaFree(c->fsum); cudaFree(c->fpart); cudaFree(c->fdone);
     if (c->h_params) cudaFreeHost(c->h_params);
     if (c->h_err) cudaFreeHost(c->h_err);

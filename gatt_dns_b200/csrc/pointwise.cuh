@@ -115,8 +115,8 @@ struct StateSet {
 // part[((b * kMaxForcings + f) * gridDim.x + cta) * 5 + q]; the member's last CTA to finish adds
 // the partials, lane by lane in CTA order and then over the lanes, so the sums do not depend on
 // timing.  done: one counter per member, zero between launches.
-// Latency-bound (64^3: 10 MB from L2): one launch of 7.5 us; a second launch whose threads added
-// the 296 partials one after the other took 39 us for the pair.
+// Latency-bound (64^3: 10 MB from L2): one launch of 8 us; with a second launch whose threads added
+// the 296 partials one after the other the pair took 39 us.
 __global__ void __launch_bounds__(256) k_forcing_sums(StateSet q, Forcings fs, double *part, unsigned *done, double *sums)
 {
     __shared__ double red[5][8];
@@ -274,6 +274,26 @@ __global__ void k_visc2d(Phys ph, StateSet q, FieldSet d1, FieldSet tq, long lon
     }
 }
 
+// Dirichlet values of the boundary program, applied where a 2-D stage state is written: a class per
+// point (0: none) and per class the variables it fixes (bits U, V, W, R, E) and their values.  The
+// Dirichlet items come first in applyBoundCond, so the rest of the program runs after them as it
+// would have; a stage's program so has one level less (128^2 cavity 129 -> 125 us a step, 800x300
+// 361 -> 354).  Not in 3-D: there the class is one more load on each chunk's critical path (plate
+// 400x150x64 3.47 -> 3.72 ms).
+struct FixedClass {
+    unsigned mask;
+    double val[5];
+};
+struct FixedPoints {
+    const uint8_t *cls;  // [points], or null
+    const FixedClass *tab;
+    __device__ __forceinline__ const FixedClass *at(long long p) const
+    {
+        const int c = cls ? cls[p] : 0;
+        return c ? tab + c : nullptr;
+    }
+};
+
 // RK4 update of one variable at one point (timeIntegration.F90:393-487)
 __device__ __forceinline__ void rk_update(int mode, double dt, double k, double q0, double *delta, double *qn)
 {
@@ -376,10 +396,11 @@ __global__ void __launch_bounds__(256, 3) k_assemble3d(Phys ph, StateSet q, Stat
     }
 }
 
-// 2-D assembly (nseq.F90:126-132) fused with the RK4 stage update.  W is left alone.
+// 2-D assembly (nseq.F90:126-132) fused with the RK4 stage update.  W is left alone but for its
+// Dirichlet values (wset: the W that the stage's boundary conditions act on).
 __global__ void k_assemble2d(Phys ph, StateSet q, StateSet q0, StateSet out, FieldSet delta,
                              FieldSet d1, FieldSet tq, FieldSet d2, long long n, int mode,
-                             const StepParams *sp, Forcings fs)
+                             const StepParams *sp, Forcings fs, FixedPoints fixed, double *wset)
 {
     const int b = blockIdx.y;
     pdl_launch();
@@ -389,6 +410,8 @@ __global__ void k_assemble2d(Phys ph, StateSet q, StateSet q0, StateSet out, Fie
     const double *U = q.v[0] + b * q.bstride, *V = q.v[1] + b * q.bstride;
     const double *R = q.v[3] + b * q.bstride, *E = q.v[4] + b * q.bstride;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
+        const FixedClass *fc = fixed.at(p);
+        if (fc && (fc->mask & 4)) wset[b * out.bstride + p] = fc->val[2];
         const double u = U[p], v = V[p], r = R[p], e = E[p];
         const double dux = d1.f(b, D2_UX)[p], duy = d1.f(b, D2_UY)[p];
         const double dvx = d1.f(b, D2_VX)[p], dvy = d1.f(b, D2_VY)[p];
@@ -416,6 +439,7 @@ __global__ void k_assemble2d(Phys ph, StateSet q, StateSet q0, StateSet out, Fie
             double dtmp = (dl && mode_reads_delta(mode)) ? *dl : 0.0;  // stage 1 overwrites delta
             rk_update(mode, dt, k[f], q0v, &dtmp, &res);
             if (dl && mode_writes_delta(mode)) *dl = dtmp;
+            if (fc && (fc->mask >> f & 1)) res = fc->val[f];
             out.v[f][b * out.bstride + p] = res;
         }
     }
