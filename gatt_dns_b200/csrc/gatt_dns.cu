@@ -1001,7 +1001,9 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
                          : a.tiles_per_row * (d == 1 ? c->nz : c->ny),
                   nf, nmembers);
         void *args[] = {&a};
-        if (smem > 48 * 1024) TRY(allow_smem(k, kMaxSmem));
+        // for every size: the tile of 128 rows in 4 blocks is 48 KB to the byte, past the default
+        // limit with the kernel's static variable
+        TRY(allow_smem(k, kMaxSmem));
         TRY(before_launch(c, cls));
         CU(cudaLaunchKernel(k, grid, dim3(32 * m.P), args, smem, c->stream));
         return after_launch(c);
