@@ -140,6 +140,7 @@ struct gatt_ctx {
         BcOp *ops = nullptr;
         unsigned *lev = nullptr;
         int nops = 0, nlev = 0;
+        int most = 0;          // ops of the level that has most
         long long widest = 0;  // points of the largest level
         std::vector<unsigned> begin, points;  // the levels' first ops (and nops), their points
     } d_prog[3];
@@ -1567,6 +1568,8 @@ int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict
     d.nops = (int)out.size();
     d.nlev = (int)begin.size();
     begin.push_back((unsigned)out.size());
+    d.most = 0;
+    for (int l = 0; l < d.nlev; l++) d.most = std::max(d.most, (int)(begin[l + 1] - begin[l]));
     d.begin = begin;
     d.points = points;
     if (out.empty()) return GATT_OK;
@@ -1974,8 +1977,9 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
     } else if (c->hold_len > 0 && !c->hold_saved) {
         return fail(GATT_ERR_STATE, "holdInlet: call gatt_apply_bc on the initial state before stepping");
     }
-    if (c->bc_cluster && d.nlev <= kBcLaunches) {
-        // one launch per level, chained
+    if (c->bc_cluster && d.nlev <= kBcLaunches && d.most * sizeof(BcOp) <= kMaxSmem) {
+        // one launch per level, chained; its ops in shared memory (longer levels: launch_bc, whose
+        // kernels read from global memory what does not fit)
         const int chain = c->chain;
         int rc = GATT_OK;
         for (int l = 0; l < d.nlev && rc == GATT_OK; l++) {
@@ -1985,8 +1989,7 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
             long long stride = c->npts;
             StateSet qs = q;
             const size_t smem = (size_t)nops * sizeof(BcOp);
-            if (smem > 48 * 1024) rc = smem <= kMaxSmem ? allow_smem((const void *)k_bc_level, kMaxSmem)
-                                                        : fail(GATT_ERR_BADARG, "too many boundary items in one level");
+            if (smem > 48 * 1024) rc = allow_smem((const void *)k_bc_level, kMaxSmem);
             if (rc != GATT_OK) break;
             void *args[] = {&pg, &qs, &c->P, &stride, &l, &op0, &nops, &total};
             const unsigned blocks = std::min((total + 255) / 256, (unsigned)c->nsm * 8);
