@@ -140,7 +140,7 @@ struct gatt_ctx {
         BcOp *ops = nullptr;
         unsigned *lev = nullptr;
         int nops = 0, nlev = 0;
-        int most = 0;          // ops of the level that has most
+        int depth = 0;         // levels before long ones were cut
         long long widest = 0;  // points of the largest level
         std::vector<unsigned> begin, points;  // the levels' first ops (and nops), their points
     } d_prog[3];
@@ -1488,14 +1488,17 @@ bool box_and(const BcBox &a, const BcBox &b, BcBox &out)
     return true;
 }
 
-// The points of b that no box of `cover` holds, as disjoint boxes.
-std::vector<BcBox> box_minus(const BcBox &b, const std::vector<BcBox> &cover)
+// The points of b that no box of `cover` holds, as disjoint boxes; some more than `most` boxes, and
+// not those, where it takes more.
+std::vector<BcBox> box_minus(const BcBox &b, const std::vector<BcBox> &cover, size_t most)
 {
     std::vector<BcBox> left{b};
     for (const BcBox &c : cover) {
+        BcBox in;
+        if (left.size() > most) break;
+        if (!box_and(b, c, in)) continue;
         std::vector<BcBox> next;
         for (BcBox r : left) {
-            BcBox in;
             if (!box_and(r, c, in)) { next.push_back(r); continue; }
             for (int q = 4; q >= 0; q -= 2) {  // the slabs of r outside `in`, z first (long rows)
                 BcBox s = r;
@@ -1523,16 +1526,45 @@ bool bc_overlap(const std::vector<HostBcOp::Acc> &x, const std::vector<HostBcOp:
     return false;
 }
 
+// Ops of a level at most: what a launch stages in shared memory without an opt-in.  Longer levels are
+// cut into several: every thread looks for its points' ops in order, from shared memory (6000 ops in
+// 15 launches 0.20 ms, as one level read from global memory 1.0 and more).
+constexpr size_t kBcLevelOps = 48 * 1024 / sizeof(BcOp);
+
 // Sort the ops into levels (bc.cuh) and upload them: an op's level is one more than the highest
 // level of the earlier ops it conflicts with.  strict: ops that read the same point conflict too
-// (their adjoints add to it).
-int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict)
+// (their adjoints add to it).  The first nfree ops are known to be independent.
+int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict, size_t nfree)
 {
+    // an op's fields and the box around its points: most pairs differ in these
+    struct Around {
+        unsigned rd, wr;
+        int box[6];
+    };
+    std::vector<Around> at(ops.size());
+    for (size_t j = 0; j < ops.size(); j++) {
+        Around &a = at[j];
+        a = {0, 0, {INT_MAX, 0, INT_MAX, 0, INT_MAX, 0}};
+        auto add = [&](const HostBcOp::Acc &x, unsigned &fields) {
+            fields |= x.fields;
+            for (int q = 0; q < 6; q += 2) {
+                a.box[q] = std::min(a.box[q], x.box[q]);
+                a.box[q + 1] = std::max(a.box[q + 1], x.box[q + 1]);
+            }
+        };
+        for (const auto &x : ops[j].rd) add(x, a.rd);
+        for (const auto &x : ops[j].wr) add(x, a.wr);
+    }
+    auto apart = [&](const Around &a, const Around &b) {
+        return !((a.wr & (b.rd | b.wr)) | (a.rd & b.wr) | (strict ? a.rd & b.rd : 0)) || a.box[1] < b.box[0] ||
+               b.box[1] < a.box[0] || a.box[3] < b.box[2] || b.box[3] < a.box[2] || a.box[5] < b.box[4] ||
+               b.box[5] < a.box[4];
+    };
     std::vector<int> level(ops.size(), 0);
     int top = 0;
-    for (size_t j = 0; j < ops.size(); j++) {
+    for (size_t j = nfree; j < ops.size(); j++) {
         for (size_t i = 0; i < j; i++) {
-            if (level[i] < level[j]) continue;
+            if (level[i] < level[j] || apart(at[i], at[j])) continue;
             const HostBcOp &a = ops[i], &b = ops[j];
             if (bc_overlap(a.wr, b.rd) || bc_overlap(a.wr, b.wr) || bc_overlap(a.rd, b.wr) ||
                 (strict && bc_overlap(a.rd, b.rd)))
@@ -1550,7 +1582,8 @@ int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict
             if (level[j] != l) continue;
             BcOp o = ops[j].op;
             const long long ni = o.box[1] - o.box[0] + 1, nj = o.box[3] - o.box[2] + 1, nk = o.box[5] - o.box[4] + 1;
-            if (points.back() && (long long)points.back() + ni * nj * nk > INT_MAX) {  // its index range ends here
+            // its index range or its share of shared memory ends here: a level more
+            if (points.back() && ((long long)points.back() + ni * nj * nk > INT_MAX || out.size() - begin.back() == kBcLevelOps)) {
                 begin.push_back((unsigned)out.size());
                 points.push_back(0);
             }
@@ -1568,8 +1601,7 @@ int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict
     d.nops = (int)out.size();
     d.nlev = (int)begin.size();
     begin.push_back((unsigned)out.size());
-    d.most = 0;
-    for (int l = 0; l < d.nlev; l++) d.most = std::max(d.most, (int)(begin[l + 1] - begin[l]));
+    d.depth = ops.empty() ? 0 : top + 1;
     d.begin = begin;
     d.points = points;
     if (out.empty()) return GATT_OK;
@@ -1681,39 +1713,66 @@ int build_bc_program(gatt_ctx *c)
     int box[6], ext[6], rd[6];
     // Dirichlet (nseq.F90:357-373): within a list later boxes win, so each keeps the points that
     // no later one covers, and the lists need one level each; the pressure list, which comes
-    // last, is a constant density where E is one
+    // last, is a constant density where E is one.  Lists whose boxes come apart into many pieces
+    // (a large box under hundreds of small ones: ten and more each) stay as they are, in order.
     std::vector<std::pair<BcBox, double>> fixed[5];
+    bool split[5];
     for (int v : {GATT_VAR_U, GATT_VAR_V, GATT_VAR_W, GATT_VAR_E, GATT_VAR_R}) {
         const HostBC &h = c->bc[GATT_BC_DIRICHLET][v];
-        std::vector<BcBox> over;
-        for (int i = h.n - 1; i >= 0; i--) {
+        std::vector<BcBox> boxes;
+        for (int i = 0; i < h.n; i++) {
             row(h, i, box); TRY(check_box(c, box));
-            const BcBox bx = {box[0], box[1], box[2], box[3], box[4], box[5]};
-            for (const BcBox &piece : box_minus(bx, over)) fixed[v].push_back({piece, h.val[i]});
-            over.push_back(bx);
+            boxes.push_back({box[0], box[1], box[2], box[3], box[4], box[5]});
         }
+        std::vector<BcBox> over;
+        const size_t most = 2 * (size_t)h.n + 64;
+        split[v] = true;
+        for (int i = h.n - 1; i >= 0 && split[v]; i--) {
+            for (const BcBox &piece : box_minus(boxes[i], over, most)) fixed[v].push_back({piece, h.val[i]});
+            over.push_back(boxes[i]);
+            split[v] = fixed[v].size() <= most;
+        }
+        if (split[v]) continue;
+        fixed[v].clear();
+        for (int i = 0; i < h.n; i++) fixed[v].push_back({boxes[i], h.val[i]});
     }
     std::vector<FixedBox> fixed_points;
-    for (int v : order)
+    size_t nfree = 0;  // ops before the first list that may overlap
+    bool disjoint = true;
+    for (int v : order) {
         for (const auto &f : fixed[v]) {
             HostBcOp o = mk(OP_SET, v, f.first.data()); o.op.val = f.second; both(o, 0, 1u << v);
             fixed_points.push_back({f.first, v, f.second});
         }
+        disjoint = disjoint && split[v];
+        if (disjoint) nfree = ops[0].size();
+    }
+    std::vector<FixedBox> dens;   // constant densities (var R), and pressures to divide by E (var -1)
+    bool fold = split[GATT_VAR_E] && split[GATT_VAR_R];
+    const size_t most = 2 * (size_t)(c->bc[GATT_BC_DIRICHLET][GATT_VAR_R].n + c->bc[GATT_BC_DIRICHLET][GATT_VAR_E].n) + 64;
     for (const auto &f : fixed[GATT_VAR_R]) {
+        if (!fold) break;
         std::vector<BcBox> constant;
         for (const auto &e : fixed[GATT_VAR_E]) {
             BcBox in;
             if (!box_and(f.first, e.first, in)) continue;
             constant.push_back(in);
-            HostBcOp o = mk(OP_SET, GATT_VAR_R, in.data()); o.op.val = f.second / (c->ph.gamma - 1.0) / e.second;
-            both(o, 0, R);
-            fixed_points.push_back({in, (int)GATT_VAR_R, o.op.val});
+            dens.push_back({in, (int)GATT_VAR_R, f.second / (c->ph.gamma - 1.0) / e.second});
         }
-        for (const BcBox &piece : box_minus(f.first, constant)) {
-            HostBcOp o = mk(OP_DIR_P, GATT_VAR_R, piece.data()); o.op.val = f.second; both(o, E, R);
-        }
+        for (const BcBox &piece : box_minus(f.first, constant, most)) dens.push_back({piece, -1, f.second});
+        fold = dens.size() <= most;
+    }
+    if (!fold) {
+        dens.clear();
+        for (const auto &f : fixed[GATT_VAR_R]) dens.push_back({f.first, -1, f.second});
+    }
+    for (const FixedBox &f : dens) {
+        HostBcOp o = mk(f.var < 0 ? OP_DIR_P : OP_SET, GATT_VAR_R, f.box.data()); o.op.val = f.val;
+        both(o, f.var < 0 ? E : 0, R);
+        if (f.var >= 0) fixed_points.push_back(f);
     }
     const size_t nfixed = ops[0].size();
+    if (disjoint && fold) nfree = nfixed;
     // P <- its extrapolation along dir at the face of box (P loaded over ext before)
     auto p_neumann = [&](int var, const int *bx, int dir, int len, int coef) {
         HostBcOp o = extrapolate(OP_P_NEU, var, bx, dir, len, coef);
@@ -1842,11 +1901,15 @@ int build_bc_program(gatt_ctx *c)
     c->tape_len = tape;
     TRY(upload_fixed_points(c, fixed_points));
     // (pressure Dirichlet values where E is not constant stay ops)
-    for (size_t i = 0; i < ops[0].size(); i++)
-        if (i >= nfixed || ops[0][i].op.code != OP_SET) ops[2].push_back(ops[0][i]);
-    TRY(upload_bc_levels(c->d_prog[2], ops[2], false));
-    TRY(upload_bc_levels(c->d_prog[0], ops[0], false));
-    TRY(upload_bc_levels(c->d_prog[1], ops[1], true));
+    size_t nkept = 0;
+    for (size_t i = 0; c->d_cls && i < ops[0].size(); i++)
+        if (i >= nfixed || ops[0][i].op.code != OP_SET) {
+            ops[2].push_back(ops[0][i]);
+            nkept += i < nfixed;
+        }
+    TRY(upload_bc_levels(c->d_prog[2], ops[2], false, split[GATT_VAR_R] ? nkept : 0));
+    TRY(upload_bc_levels(c->d_prog[0], ops[0], false, nfree));
+    TRY(upload_bc_levels(c->d_prog[1], ops[1], true, nfree));
     c->nops = c->d_prog[0].nops;
     cudaFree(c->d_coef1); c->d_coef1 = nullptr;
     cudaFree(c->d_coef2); c->d_coef2 = nullptr;
@@ -1977,9 +2040,8 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
     } else if (c->hold_len > 0 && !c->hold_saved) {
         return fail(GATT_ERR_STATE, "holdInlet: call gatt_apply_bc on the initial state before stepping");
     }
-    if (c->bc_cluster && d.nlev <= kBcLaunches && d.most * sizeof(BcOp) <= kMaxSmem) {
-        // one launch per level, chained; its ops in shared memory (longer levels: launch_bc, whose
-        // kernels read from global memory what does not fit)
+    if (c->bc_cluster && d.depth <= kBcLaunches) {
+        // one launch per level, chained
         const int chain = c->chain;
         int rc = GATT_OK;
         for (int l = 0; l < d.nlev && rc == GATT_OK; l++) {
@@ -1989,8 +2051,6 @@ int apply_bc(gatt_ctx *c, const StateSet &q, int nmem, double tfac, bool fixed =
             long long stride = c->npts;
             StateSet qs = q;
             const size_t smem = (size_t)nops * sizeof(BcOp);
-            if (smem > 48 * 1024) rc = allow_smem((const void *)k_bc_level, kMaxSmem);
-            if (rc != GATT_OK) break;
             void *args[] = {&pg, &qs, &c->P, &stride, &l, &op0, &nops, &total};
             const unsigned blocks = std::min((total + 255) / 256, (unsigned)c->nsm * 8);
             rc = launch_chained(c, PC_BC, (const void *)k_bc_level, dim3(blocks, nmem), dim3(256), smem, args);
