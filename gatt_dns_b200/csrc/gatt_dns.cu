@@ -180,9 +180,10 @@ struct gatt_ctx {
     double *a_lq = nullptr, *a_ld1 = nullptr, *a_ltau = nullptr, *a_lvt = nullptr;  // 5, 15, 9, 4
     double *a_s1 = nullptr, *a_s2 = nullptr, *a_scr[3] = {};                         // 15, 12, 5 each
     // first derivatives and second sweeps of the stage states 1..3 of the adjoint's recomputed step
-    // (stage 0's stay in d1 / d2); null where there is no room: recomputed
+    // (stage 0's stay in d1 / d2); null where there is no room: recomputed.  a_scr[1], a_scr[2] are
+    // null there too: the directions' transposed sweeps then take turns with a_scr[0].
     double *a_sd1[3] = {}, *a_sd2[3] = {};
-    bool a_sd_full = false;
+    bool adj_keep = true;   // (GATT_ADJ_KEEP=0: always null)
     double *a_ckpt = nullptr, *a_seg = nullptr;
     int a_nckpt = 0, a_nseg = 0;
     bool a_ckpt_sfd = false, a_seg_sfd = false;  // checkpoint / segment slots hold a mean too
@@ -212,7 +213,8 @@ struct gatt_ctx {
     cudaStream_t side2 = nullptr;  // 3-D: the z sweep beside the y sweep where they are two launches
     cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr, ev_sums = nullptr;
     bool sums_ahead = false;       // this stage's forcing sums are under way on it (ev_sums)
-    double *tmp_side2 = nullptr;
+    double *tmp_side2 = nullptr;   // its scratch field: there for z lines that need one (long_z)
+    bool long_z = false;
     bool own_stream = false;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     int graph_kernels[2] = {0, 0};
@@ -264,6 +266,33 @@ int sync_stream(gatt_ctx *c)
         return fail(GATT_ERR_TIMEOUT, "a copy pipeline gave up (tile wait timed out or misaligned ring)");
     }
     return GATT_OK;
+}
+
+// Free what the adjoint only keeps to be faster (adjoint_room); whether there was any.
+bool give_room(gatt_ctx *c)
+{
+    bool any = false;
+    for (double **p : {&c->a_scr[1], &c->a_scr[2], &c->a_sd1[0], &c->a_sd1[1], &c->a_sd1[2], &c->a_sd2[0], &c->a_sd2[1], &c->a_sd2[2]}) {
+        any = any || *p;
+        cudaFree(*p);
+        *p = nullptr;
+    }
+    return any;
+}
+
+// Device memory that the context needs: before it fails, the optional sets give way.
+template <typename T>
+int dev_alloc(gatt_ctx *c, T **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // (the next launch check would read it)
+    if (e == cudaErrorMemoryAllocation && give_room(c)) {
+        e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    if (e == cudaSuccess) return GATT_OK;
+    *p = nullptr;
+    return fail(e == cudaErrorMemoryAllocation ? GATT_ERR_NOMEM : GATT_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
 }
 
 int grid_for(const gatt_ctx *c, long long n)
@@ -560,6 +589,9 @@ size_t sweep_smem(int N, int P, int nR, int Wp, bool stage = true)
 // 227 KB per block, less a margin for the kernel's few static shared variables
 constexpr int kMaxNR = 11;  // widest band the shared-tile solver is instantiated for
 
+// Whether z sweeps can run on the third stream.
+bool z_beside(const gatt_ctx *c) { return c->side2 && (!c->long_z || c->tmp_side2); }
+
 // Row blocks per line: about 32 rows per block (shorter dependency chains, more warps per
 // tile), a power of two up to kMaxP, every block at least nR+1 rows long, and few enough
 // that the shared tile fits (long lines: fewer blocks, halo and exchange rows).
@@ -671,7 +703,7 @@ int upload_line_records(gatt_ctx *c, DevDir &m)
     hQ.insert(hQ.end(), hS.begin(), hS.end());
     hQ.resize(nQ + nS + (hB.size() + 1) / 2, 0.0);
     memcpy(&hQ[nQ + nS], hB.data(), hB.size() * sizeof(int));
-    CU(cudaMalloc(&m.lQ, hQ.size() * sizeof(double)));
+    TRY(dev_alloc(c, &m.lQ, hQ.size() * sizeof(double)));
     CU(cudaMemcpy(m.lQ, hQ.data(), hQ.size() * sizeof(double), cudaMemcpyHostToDevice));
     m.lS = m.lQ + nQ;
     m.lB = reinterpret_cast<int *>(m.lQ + nQ + nS);
@@ -708,8 +740,8 @@ int upload_records(gatt_ctx *c, DevDir &m, int P, int rows = 0)
         cudaFree(m.Rm); m.Rm = nullptr;
         cudaFree(m.Q); m.Q = nullptr;
         m.cap = 0;
-        CU(cudaMalloc(&m.Rm, hRm.size() * sizeof(double)));
-        CU(cudaMalloc(&m.Q, hQ.size() * sizeof(double)));
+        TRY(dev_alloc(c, &m.Rm, hRm.size() * sizeof(double)));
+        TRY(dev_alloc(c, &m.Q, hQ.size() * sizeof(double)));
         m.cap = N;
         invalidate_graphs(c);  // graphs hold the record pointers
     }
@@ -1073,7 +1105,7 @@ int sweep_yz(gatt_ctx *c, const double *in, long long in_bs, const int *sy, cons
         if (r != GATT_ERR_STATE) return r;  // GATT_ERR_STATE: layout refused, two launches
     }
     // two launches: the z sweep beside the y sweep on a third stream
-    const bool fork = c->fork_x && !c->profiling && c->side2;
+    const bool fork = c->fork_x && !c->profiling && z_beside(c);
     if (fork) {
         CU(cudaEventRecord(c->ev_fork2, c->stream));
         CU(cudaStreamWaitEvent(c->side2, c->ev_fork2, 0));
@@ -1339,11 +1371,11 @@ int launch_assemble2d(gatt_ctx *c, StateSet q, StateSet q0, StateSet out, int mo
 }
 
 // launch(d) for every direction, the x direction's launches on the side stream and (3-D) the z
-// direction's on a third one beside the y direction's.
+// direction's on a third one beside the y direction's (apart: they share no scratch).
 template <typename F>
-int each_direction(gatt_ctx *c, F &&launch)
+int each_direction(gatt_ctx *c, F &&launch, bool apart = true)
 {
-    const bool fork = c->fork_x && !c->profiling && c->side && (!c->is3d || c->side2);
+    const bool fork = apart && c->fork_x && !c->profiling && c->side && (!c->is3d || z_beside(c));
     if (!fork) {
         for (int d = 0; d < (c->is3d ? 3 : 2); d++) TRY(launch(d));
         return GATT_OK;
@@ -1534,7 +1566,7 @@ constexpr size_t kBcLevelOps = 48 * 1024 / sizeof(BcOp);
 // Sort the ops into levels (bc.cuh) and upload them: an op's level is one more than the highest
 // level of the earlier ops it conflicts with.  strict: ops that read the same point conflict too
 // (their adjoints add to it).  The first nfree ops are known to be independent.
-int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict, size_t nfree)
+int upload_bc_levels(gatt_ctx *c, gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict, size_t nfree)
 {
     // an op's fields and the box around its points: most pairs differ in these
     struct Around {
@@ -1608,9 +1640,9 @@ int upload_bc_levels(gatt_ctx::BcDev &d, std::vector<HostBcOp> &ops, bool strict
     std::vector<unsigned> lev(begin);
     lev.insert(lev.end(), points.begin(), points.end());
     lev.push_back(0);  // whole 8-byte words
-    CU(cudaMalloc(&d.ops, out.size() * sizeof(BcOp)));
+    TRY(dev_alloc(c, &d.ops, out.size() * sizeof(BcOp)));
     CU(cudaMemcpy(d.ops, out.data(), out.size() * sizeof(BcOp), cudaMemcpyHostToDevice));
-    CU(cudaMalloc(&d.lev, lev.size() * sizeof(unsigned)));
+    TRY(dev_alloc(c, &d.lev, lev.size() * sizeof(unsigned)));
     CU(cudaMemcpy(d.lev, lev.data(), lev.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
     return GATT_OK;
 }
@@ -1652,9 +1684,11 @@ int upload_fixed_points(gatt_ctx *c, const std::vector<FixedBox> &boxes)
                 }
             }
     }
-    CU(cudaMalloc(&c->d_cls, cls.size()));
+    const int rc = dev_alloc(c, &c->d_cls, cls.size());
+    if (rc == GATT_ERR_NOMEM) return GATT_OK;
+    TRY(rc);
     CU(cudaMemcpy(c->d_cls, cls.data(), cls.size(), cudaMemcpyHostToDevice));
-    CU(cudaMalloc(&c->d_clstab, tab.size() * sizeof(FixedClass)));
+    TRY(dev_alloc(c, &c->d_clstab, tab.size() * sizeof(FixedClass)));
     CU(cudaMemcpy(c->d_clstab, tab.data(), tab.size() * sizeof(FixedClass), cudaMemcpyHostToDevice));
     return GATT_OK;
 }
@@ -1907,28 +1941,28 @@ int build_bc_program(gatt_ctx *c)
             ops[2].push_back(ops[0][i]);
             nkept += i < nfixed;
         }
-    TRY(upload_bc_levels(c->d_prog[2], ops[2], false, split[GATT_VAR_R] ? nkept : 0));
-    TRY(upload_bc_levels(c->d_prog[0], ops[0], false, nfree));
-    TRY(upload_bc_levels(c->d_prog[1], ops[1], true, nfree));
+    TRY(upload_bc_levels(c, c->d_prog[2], ops[2], false, split[GATT_VAR_R] ? nkept : 0));
+    TRY(upload_bc_levels(c, c->d_prog[0], ops[0], false, nfree));
+    TRY(upload_bc_levels(c, c->d_prog[1], ops[1], true, nfree));
     c->nops = c->d_prog[0].nops;
     cudaFree(c->d_coef1); c->d_coef1 = nullptr;
     cudaFree(c->d_coef2); c->d_coef2 = nullptr;
     cudaFree(c->d_xs); c->d_xs = nullptr;
     if (!c->coef1.empty()) {
-        CU(cudaMalloc(&c->d_coef1, c->coef1.size() * sizeof(double)));
+        TRY(dev_alloc(c, &c->d_coef1, c->coef1.size() * sizeof(double)));
         CU(cudaMemcpy(c->d_coef1, c->coef1.data(), c->coef1.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
     if (!c->coef2.empty()) {
-        CU(cudaMalloc(&c->d_coef2, c->coef2.size() * sizeof(double)));
+        TRY(dev_alloc(c, &c->d_coef2, c->coef2.size() * sizeof(double)));
         CU(cudaMemcpy(c->d_coef2, c->coef2.data(), c->coef2.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
     if (!c->distx.empty()) {
-        CU(cudaMalloc(&c->d_xs, c->distx.size() * sizeof(double)));
+        TRY(dev_alloc(c, &c->d_xs, c->distx.size() * sizeof(double)));
         CU(cudaMemcpy(c->d_xs, c->distx.data(), c->distx.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
     if (hold_sig != c->hold_sig || (hold_len > 0 && !c->d_hold)) {  // a new hold layout: saved afresh
         cudaFree(c->d_hold); c->d_hold = nullptr;
-        if (hold_len > 0) CU(cudaMalloc(&c->d_hold, sizeof(double) * (size_t)hold_len * c->nb));
+        if (hold_len > 0) TRY(dev_alloc(c, &c->d_hold, sizeof(double) * (size_t)hold_len * c->nb));
         c->hold_len = hold_len;
         c->hold_sig = hold_sig;
         c->hold_saved = false;
@@ -2227,7 +2261,7 @@ int ensure_hist(gatt_ctx *c, int n)
     cudaFree(c->hist);
     cudaFreeHost(c->h_params);
     c->hist = nullptr; c->h_params = nullptr;
-    CU(cudaMalloc(&c->hist, sizeof(double) * 5 * c->nb * (size_t)cap));
+    TRY(dev_alloc(c, &c->hist, sizeof(double) * 5 * c->nb * (size_t)cap));
     CU(cudaMallocHost(&c->h_params, sizeof(StepParams) * (size_t)cap));
     c->hist_cap = cap;
     invalidate_graphs(c);  // graphs hold the history pointer
@@ -2282,7 +2316,7 @@ int run_steps(gatt_ctx *c, int nsteps, double t0, double dt, double *maxChange, 
 
 int alloc_fields(gatt_ctx *c, double **p, int nslots, int members)
 {
-    CU(cudaMalloc(p, sizeof(double) * (size_t)c->npts * nslots * members));
+    TRY(dev_alloc(c, p, sizeof(double) * (size_t)c->npts * nslots * members));
     CU(cudaMemsetAsync(*p, 0, sizeof(double) * (size_t)c->npts * nslots * members, c->stream));
     return GATT_OK;
 }
@@ -2344,19 +2378,19 @@ int arn_alloc(gatt_ctx *c, int m)
         cudaFree(c->arn_zeta);
         c->arn_zeta = nullptr;
         c->arn_m = 0;
-        CU(cudaMalloc(&c->arn_zeta, sizeof(double) * (size_t)c->nb * (m + 1) * len));
+        TRY(dev_alloc(c, &c->arn_zeta, sizeof(double) * (size_t)c->nb * (m + 1) * len));
         cudaFree(c->arn_part);
         c->arn_part = nullptr;
-        CU(cudaMalloc(&c->arn_part, sizeof(double) * (size_t)c->nb * (m + 2) * kRedBlocks));
+        TRY(dev_alloc(c, &c->arn_part, sizeof(double) * (size_t)c->nb * (m + 2) * kRedBlocks));
         cudaFree(c->arn_h);
         c->arn_h = nullptr;
-        CU(cudaMalloc(&c->arn_h, sizeof(double) * (size_t)c->nb * (m + 2)));
+        TRY(dev_alloc(c, &c->arn_h, sizeof(double) * (size_t)c->nb * (m + 2)));
         c->arn_m = m;
     }
-    if (!c->arn_B) CU(cudaMalloc(&c->arn_B, sizeof(double) * (size_t)c->nb * len));
-    if (!c->arn_base) CU(cudaMalloc(&c->arn_base, sizeof(double) * 5 * (size_t)c->npts));
-    if (!c->arn_um) CU(cudaMalloc(&c->arn_um, sizeof(double) * 5 * (size_t)c->npts));
-    if (!c->arn_region) CU(cudaMalloc(&c->arn_region, (size_t)c->npts));
+    if (!c->arn_B) TRY(dev_alloc(c, &c->arn_B, sizeof(double) * (size_t)c->nb * len));
+    if (!c->arn_base) TRY(dev_alloc(c, &c->arn_base, sizeof(double) * 5 * (size_t)c->npts));
+    if (!c->arn_um) TRY(dev_alloc(c, &c->arn_um, sizeof(double) * 5 * (size_t)c->npts));
+    if (!c->arn_region) TRY(dev_alloc(c, &c->arn_region, (size_t)c->npts));
     return GATT_OK;
 }
 
@@ -2575,7 +2609,7 @@ int diff_alloc(gatt_ctx *c, bool adjoint)
         if (diff_sfd(c)) TRY(alloc_zeroed(c, &c->dym, 5));
         return GATT_OK;
     }
-    double **five[] = {&c->a_lam, &c->a_acc, &c->a_arg, &c->a_prev, &c->a_g, &c->a_lq, &c->a_scr[0], &c->a_scr[1], &c->a_scr[2]};
+    double **five[] = {&c->a_lam, &c->a_acc, &c->a_arg, &c->a_prev, &c->a_g, &c->a_lq, &c->a_scr[0]};
     for (double **p : five) TRY(alloc_zeroed(c, p, 5));
     TRY(alloc_zeroed(c, &c->a_ld1, D3_N));
     TRY(alloc_zeroed(c, &c->a_ltau, T3_N));
@@ -2588,35 +2622,51 @@ int diff_alloc(gatt_ctx *c, bool adjoint)
         TRY(alloc_zeroed(c, &c->a_lm, 5));
         TRY(alloc_zeroed(c, &c->a_mscr, 5));
     }
-    // the stage derivatives of a recomputed step, if there is room (81 fields a member); without them
-    // the reverse sweep forms three of the four again
-    if (!c->a_sd1[0] && !c->a_sd_full) {
-        int rc = GATT_OK;
-        for (int s = 0; s < 3 && rc == GATT_OK; s++) {
-            rc = alloc_zeroed(c, &c->a_sd1[s], D3_N);
-            if (rc == GATT_OK) rc = alloc_zeroed(c, &c->a_sd2[s], S3_N);
-        }
-        if (rc == GATT_ERR_NOMEM) {
-            cudaGetLastError();
-            for (int s = 0; s < 3; s++) {
-                cudaFree(c->a_sd1[s]); c->a_sd1[s] = nullptr;
-                cudaFree(c->a_sd2[s]); c->a_sd2[s] = nullptr;
-            }
-            c->a_sd_full = true;
-        } else if (rc != GATT_OK) {
-            return rc;
-        }
-    }
     // five boundary-program tapes per step (after each stage and after the filter / SFD)
     const long long need = 5 * std::max(1LL, c->tape_len) * c->nb;
     if (c->a_tape_cap < need) {
         cudaFree(c->a_tape);
         c->a_tape = nullptr;
         c->a_tape_cap = 0;
-        CU(cudaMalloc(&c->a_tape, sizeof(double) * (size_t)need));
+        TRY(dev_alloc(c, &c->a_tape, sizeof(double) * (size_t)need));
         c->a_tape_cap = need;
     }
     return GATT_OK;
+}
+
+// Sets that make the adjoint faster, once everything it needs is there: a scratch set per direction
+// (the directions' sweeps run side by side) and, for steps, the stage derivatives (81 fields a member;
+// without them the reverse sweep forms three of the four again).  Taken where as much memory stays
+// free; given back when an allocation of the context does not fit (dev_alloc).
+int adjoint_room(gatt_ctx *c, bool steps)
+{
+    if (!c->adj_keep) return GATT_OK;
+    auto take = [&](double **p, int nslots, int sets) -> int {
+        if (*p) return GATT_OK;
+        size_t room = 0, all = 0;
+        CU(cudaMemGetInfo(&room, &all));
+        const size_t bytes = sizeof(double) * (size_t)c->npts * c->nb * nslots;
+        if (room / 2 < bytes * sets) return GATT_ERR_NOMEM;
+        if (cudaMalloc(p, bytes) == cudaSuccess) {
+            CU(cudaMemsetAsync(*p, 0, bytes, c->stream));  // (2-D: the z slots are never written)
+            return GATT_OK;
+        }
+        cudaGetLastError();
+        *p = nullptr;
+        return GATT_ERR_NOMEM;
+    };
+    int rc = GATT_OK;
+    for (int d = 1; d < (c->is3d ? 3 : 2) && rc == GATT_OK; d++) rc = take(&c->a_scr[d], 5, 1);
+    for (int s = 0; s < 3 && steps && rc == GATT_OK; s++) {
+        rc = take(&c->a_sd1[s], D3_N, s ? 1 : 6);  // (all six are about six of the larger)
+        if (rc == GATT_OK) rc = take(&c->a_sd2[s], S3_N, 1);
+    }
+    if (rc == GATT_ERR_NOMEM && c->a_sd1[0] && !c->a_sd2[2])
+        for (int s = 0; s < 3; s++) {
+            cudaFree(c->a_sd1[s]); c->a_sd1[s] = nullptr;
+            cudaFree(c->a_sd2[s]); c->a_sd2[s] = nullptr;
+        }
+    return rc == GATT_ERR_NOMEM ? GATT_OK : rc;
 }
 
 // boundary program on base x and tangent y together, at time t + tfac dt
@@ -2769,9 +2819,10 @@ int sweep_T(gatt_ctx *c, int d, int k0, const double *in, long long in_bs, const
 {
     int sl[16];
     for (int f = 0; f < nf; f++) sl[f] = f;
-    // (a scratch set per direction: the directions' sweeps run side by side)
-    TRY(sweep(c, d, k0, in, in_bs, in_slots, c->a_scr[d], 5 * c->npts, sl, nf, c->nb, 0.0, nullptr, PC_OTHER));
-    return sweep(c, d, k0 + 1, c->a_scr[d], 5 * c->npts, sl, out, out_bs, out_slots, nf, c->nb, 0.0, nullptr, PC_OTHER);
+    // a scratch set per direction where there is room: their sweeps then run side by side
+    double *scr = c->a_scr[d] ? c->a_scr[d] : c->a_scr[0];
+    TRY(sweep(c, d, k0, in, in_bs, in_slots, scr, 5 * c->npts, sl, nf, c->nb, 0.0, nullptr, PC_OTHER));
+    return sweep(c, d, k0 + 1, scr, 5 * c->npts, sl, out, out_bs, out_slots, nf, c->nb, 0.0, nullptr, PC_OTHER);
 }
 
 // G = F'(q)^T a (the adjoint of the RHS at state q, whose first derivatives and second sweeps are
@@ -2780,6 +2831,7 @@ int adj_rhs(gatt_ctx *c, const StateSet &q, const StateSet &a, const StateSet &G
 {
     const int nm = c->nb;
     const long long n = c->npts;
+    const bool apart = c->a_scr[1] && (!c->is3d || c->a_scr[2]);
     TRY(before_launch(c, PC_OTHER));
     k_adj_asm3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(
         c->ph, q, fset(c, d1, D3_N), fset(c, d2, S3_N), a, fset(c, c->a_lq, 5), fset(c, c->a_ld1, D3_N),
@@ -2790,7 +2842,7 @@ int adj_rhs(gatt_ctx *c, const StateSet &q, const StateSet &a, const StateSet &G
     TRY(each_direction(c, [&](int d) {
         const int o4[4] = {4 * d, 4 * d + 1, 4 * d + 2, 4 * d + 3};
         return sweep_T(c, d, 2, c->a_lvt, 4 * n, v4, c->a_s2, 12 * n, o4, 4);
-    }));
+    }, apart));
     TRY(before_launch(c, PC_OTHER));
     k_adj_tau3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(c->ph, q, fset(c, d1, D3_N),
                                                                    fset(c, c->a_ltau, T3_N), fset(c, c->a_s2, 12),
@@ -2801,7 +2853,7 @@ int adj_rhs(gatt_ctx *c, const StateSet &q, const StateSet &a, const StateSet &G
         const int i5[5] = {D3_UX + d, D3_VX + d, D3_WX + d, D3_RX + d, D3_EX + d};
         const int o5[5] = {5 * d, 5 * d + 1, 5 * d + 2, 5 * d + 3, 5 * d + 4};
         return sweep_T(c, d, 2, c->a_ld1, (long long)D3_N * n, i5, c->a_s1, 15 * n, o5, 5);
-    }));
+    }, apart));
     TRY(before_launch(c, PC_OTHER));
     k_adj_q3d<<<dim3(grid_for(c, n), nm), kBlock, 0, c->stream>>>(fset(c, c->a_lq, 5), fset(c, c->a_s1, 15), G, n);
     return after_launch(c);
@@ -2934,6 +2986,7 @@ int rhs_vjp(gatt_ctx *c, const double *q, const double *a, double *lam)
 {
     TRY(check_diff(c, true));
     TRY(diff_alloc(c, true));
+    TRY(adjoint_room(c, false));
     TRY(upload5(c, c->dx[0], q));
     TRY(upload5(c, c->a_arg, a));
     const StateSet X0 = set5(c, c->dx[0]);
@@ -2979,7 +3032,7 @@ int vjp(gatt_ctx *c, int nsteps, double t0, double dt, int every, const double *
         cudaFree(c->a_ckpt);
         c->a_ckpt = nullptr;
         c->a_nckpt = 0;
-        CU(cudaMalloc(&c->a_ckpt, sizeof(double) * st * (nck + 1)));
+        TRY(dev_alloc(c, &c->a_ckpt, sizeof(double) * st * (nck + 1)));
         c->a_nckpt = nck + 1;
         c->a_ckpt_sfd = sfd;
     }
@@ -2987,10 +3040,12 @@ int vjp(gatt_ctx *c, int nsteps, double t0, double dt, int every, const double *
         cudaFree(c->a_seg);
         c->a_seg = nullptr;
         c->a_nseg = 0;
-        CU(cudaMalloc(&c->a_seg, sizeof(double) * st * seg));
+        TRY(dev_alloc(c, &c->a_seg, sizeof(double) * st * seg));
         c->a_nseg = seg;
         c->a_seg_sfd = sfd;
     }
+    TRY(ensure_hist(c, seg));
+    TRY(adjoint_room(c, true));
     auto save = [&](double *dst) -> int {
         TRY(state_to_set(c, state_set(c, 0), dst, true));
         return sfd ? copy_set5(c, dst + s5, c->mean) : GATT_OK;
@@ -2999,7 +3054,6 @@ int vjp(gatt_ctx *c, int nsteps, double t0, double dt, int every, const double *
         TRY(state_to_set(c, state_set(c, 0), const_cast<double *>(src), false));
         return sfd ? copy_set5(c, c->mean, src + s5) : GATT_OK;
     };
-    TRY(ensure_hist(c, seg));
     // forward: checkpoints at steps 0, every, 2*every, ...; slot nck keeps the final state
     for (int k = 0; k < nck; k++) {
         TRY(save(c->a_ckpt + st * k));
@@ -3173,6 +3227,8 @@ int gatt_create(gatt_ctx **out, int nx, int ny, int nz, int nbatch)
         c->fork_x = !(fxs && !strcmp(fxs, "0"));
         const char *fzs = getenv("GATT_FZ_REV");
         c->fz_rev = !(fzs && !strcmp(fzs, "0"));
+        const char *aks = getenv("GATT_ADJ_KEEP");
+        c->adj_keep = !(aks && !strcmp(aks, "0"));
     }
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -3196,7 +3252,6 @@ int gatt_create(gatt_ctx **out, int nx, int ny, int nz, int nbatch)
         if (es != cudaSuccess && rc == GATT_OK) rc = fail(GATT_ERR_CUDA, cudaGetErrorString(es));
     }
     if (rc == GATT_OK) {
-        if (c->is3d) chk(alloc_fields(c, &c->tmp_side2, 1, 1));
         chk(alloc_fields(c, &c->qA, 5, nbatch));
         chk(alloc_fields(c, &c->qB, 5, nbatch));
         chk(alloc_fields(c, &c->delta, 5, nbatch));
@@ -3389,11 +3444,18 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     else TRY(sync_stream(c));
     // (2-D: also for the chained step's sweeps)
     if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_fits(d == 0, N, nRHS, 8))) TRY(upload_line_records(c, m));
+    // z lines that only the global-memory solver takes: a scratch field for the third stream, where
+    // there is room
+    if (d == 2 && (nRHS < 2 || nRHS > kMaxNR || sweep_smem(N, 1, nRHS, m.Wp, false) > kMaxSmem)) {
+        c->long_z = true;
+        const int rc = c->tmp_side2 ? (int)GATT_OK : alloc_fields(c, &c->tmp_side2, 1, 1);
+        if (rc != GATT_OK && rc != GATT_ERR_NOMEM) return rc;
+    }
     m.rpb = rpb;
     m.family = line ? FAM_LINE : rpb ? (want == FAM_LINE ? FAM_PIPE : want) : FAM_TILE;
     m.set = true;
     if (nBlocks > 0) {
-        if (!c->ltype[d]) CU(cudaMalloc(&c->ltype[d], lt.size()));
+        if (!c->ltype[d]) TRY(dev_alloc(c, &c->ltype[d], lt.size()));
         CU(cudaMemcpy(c->ltype[d], lt.data(), lt.size(), cudaMemcpyHostToDevice));
         c->lt_set[d] = true;
         int mx = 0;
@@ -3514,10 +3576,10 @@ int gatt_add_forcing(gatt_ctx *c, int type, const int *ind, int npar, const doub
             return fail(GATT_ERR_BADARG, "forcing box outside the grid");
     if (!c->fsum) {
         c->fblocks = 2 * c->nsm;
-        if (!c->fdone) CU(cudaMalloc(&c->fdone, sizeof(unsigned) * (size_t)c->nb));
+        if (!c->fdone) TRY(dev_alloc(c, &c->fdone, sizeof(unsigned) * (size_t)c->nb));
         CU(cudaMemsetAsync(c->fdone, 0, sizeof(unsigned) * (size_t)c->nb, c->stream));
-        CU(cudaMalloc(&c->fsum, sizeof(double) * (size_t)c->nb * kMaxForcings * 5));
-        CU(cudaMalloc(&c->fpart, sizeof(double) * (size_t)c->nb * kMaxForcings * c->fblocks * 5));
+        TRY(dev_alloc(c, &c->fsum, sizeof(double) * (size_t)c->nb * kMaxForcings * 5));
+        TRY(dev_alloc(c, &c->fpart, sizeof(double) * (size_t)c->nb * kMaxForcings * c->fblocks * 5));
     }
     const int f = c->fc.n++;
     c->fc.type[f] = type;
@@ -3557,7 +3619,7 @@ int gatt_set_sfd(gatt_ctx *c, int type, double Delta, double chiValue, const dou
     c->sfd_delta = Delta;
     invalidate_graphs(c);
     if (type == 0) return GATT_OK;
-    if (!c->chi) CU(cudaMalloc(&c->chi, sizeof(double) * c->npts));
+    if (!c->chi) TRY(dev_alloc(c, &c->chi, sizeof(double) * c->npts));
     if (type == 1) {
         std::vector<double> h(c->npts, chiValue);
         CU(cudaMemcpy(c->chi, h.data(), sizeof(double) * c->npts, cudaMemcpyHostToDevice));
