@@ -242,6 +242,7 @@ struct gatt_ctx {
                             // (GATT_FORK_X=0: everything on one stream)
     bool fz_rev = true;     // last filter direction takes the fields in reverse order (GATT_FZ_REV=0: no)
     bool mc_done = false;   // set when a filter launch ran the max-change epilogue
+    mutable std::set<const void *> smem_allowed;  // kernels whose shared-memory limit it has raised (allow_smem)
     int bc_cluster = 0;     // CTAs per member for the boundary program (0: one CTA, k_bc)
     int bc_cluster_rec = 0, bc_cluster_tl = 0, bc_cluster_adj = 0;  // same, tape / tangent / adjoint
     // per-kernel-class timing (gatt_profile_kernels): events around every launch
@@ -512,19 +513,15 @@ int resident_ctas(const void *k, int threads, size_t smem)
 }
 
 // Let a kernel use up to `most` bytes of dynamic shared memory (and, carve, the whole L1 as shared
-// memory): once per device and kernel, when it is first launched -- setting the attributes of
-// every instantiation for each context took half of its creation.
-int allow_smem(const void *k, size_t most, bool carve = false)
+// memory): when a context first launches it -- setting the attributes of every instantiation took
+// half of a context's creation.  Remembered by the context, as the attribute belongs to its CUDA
+// context: the next one may follow a device reset, or live in another CUDA context of the device.
+int allow_smem(const gatt_ctx *c, const void *k, size_t most, bool carve = false)
 {
-    static std::mutex mu;
-    static std::set<std::pair<int, const void *>> seen;
-    int dev = 0;
-    CU(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    if (seen.count({dev, k})) return GATT_OK;
+    if (c->smem_allowed.count(k)) return GATT_OK;
     CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     if (carve) CU(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    seen.insert({dev, k});
+    c->smem_allowed.insert(k);
     return GATT_OK;
 }
 
@@ -771,7 +768,7 @@ int launch_psweep(gatt_ctx *c, const DevDir &m, int d, SweepArgs &a, int nmember
     }
     const bool cmp = ub && xd && c->x_compact;  // the compact shared-memory layout
     if (!k) return GATT_ERR_STATE;
-    TRY(allow_smem(k, kMaxSmem, true));
+    TRY(allow_smem(c, k, kMaxSmem, true));
     // ring depth: the deepest ring that keeps the most CTAs resident (one stage suffices
     // when a tile's solve outlasts the next tile's copy)
     int nst = 0, per_sm = 0;
@@ -899,7 +896,7 @@ LinePlan line_plan_for(const gatt_ctx *c, const DevDir &m, int d, int nf, int nm
     pl.LL = LL;
     pl.jobs = line_tiles(c, d, LL) * nf * nmem;
     pl.kernel = xd ? line_kernel_x(m.periodic != 0, m.nR, LL) : line_kernel_yz(m.periodic != 0, m.nR, LL);
-    if (allow_smem(pl.kernel, kMaxSmem) != GATT_OK) return best;
+    if (allow_smem(c, pl.kernel, kMaxSmem) != GATT_OK) return best;
     const int warps = (m.lP * LL + 31) / 32;
     const bool S = m.nspecial > 0 && (size_t)m.nspecial * line_band_doubles(m.Wp) * sizeof(double) <= kLineBandBytes;
     for (int v = S ? 0 : 2; v < 4; v++) {
@@ -1036,7 +1033,7 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
         void *args[] = {&a};
         // for every size: the tile of 128 rows in 4 blocks is 48 KB to the byte, past the default
         // limit with the kernel's static variable
-        TRY(allow_smem(k, kMaxSmem));
+        TRY(allow_smem(c, k, kMaxSmem));
         TRY(before_launch(c, cls));
         CU(cudaLaunchKernel(k, grid, dim3(32 * m.P), args, smem, c->stream));
         return after_launch(c);
@@ -1140,7 +1137,7 @@ XyPlan xy_plan(const gatt_ctx *c, int nf, int nmem, int LL)
     p.y = line_plan_for(c, my, 1, nf, nmem, LL);
     if (!p.x.LL || !p.y.LL) return p;
     void *k = line_kernel_xy(mx.periodic != 0, my.periodic != 0, mx.nR, LL);
-    if (!k || allow_smem(k, kMaxSmem) != GATT_OK) return p;
+    if (!k || allow_smem(c, k, kMaxSmem) != GATT_OK) return p;
     p.threads = (std::max(mx.lP, my.lP) * LL + 31) / 32 * 32;
     p.smem = std::max(p.x.smem, p.y.smem);
     p.per_sm = resident_ctas(k, p.threads, p.smem);
@@ -1286,7 +1283,7 @@ int launch_assemble3d_pipe(gatt_ctx *c, const StateSet &q, const StateSet &q0, c
     if (a.use_q0 && !pw_map(c, &maps.m[PW_Q0], q0b, 5, q0.bstride, nmem)) return GATT_ERR_STATE;
     if (a.use_delta && !pw_map(c, &maps.m[PW_DL], dlb, 5, delta.bstride, nmem)) return GATT_ERR_STATE;
     const size_t smem = pw_smem_bytes(a.nst);
-    TRY(allow_smem((const void *)k_assemble3d_pipe, smem));
+    TRY(allow_smem(c, (const void *)k_assemble3d_pipe, smem));
     const int per_sm = resident_ctas((const void *)k_assemble3d_pipe, 2 * kPwC, smem);
     if (per_sm < 1) return GATT_ERR_STATE;
     const long long grid = std::min<long long>(a.njobs, (long long)per_sm * c->nsm);
