@@ -58,7 +58,7 @@ int fail(int code, const std::string &msg)
 
 // Line-solve kernel families: shared-memory tile (any N), register-resident rows loaded
 // from global memory, register-resident rows fed by a TMA ring (persistent CTAs),
-// register-resident rows of lines of any length (up to 1024 rows) through asynchronous copies.
+// register-resident rows of lines of any length (up to line_max_rows) through asynchronous copies.
 enum SweepFamily { FAM_TILE = 0, FAM_REG = 1, FAM_PIPE = 2, FAM_LINE = 3 };
 
 // Matrix kinds per direction: 0 derivative, 1 filter, 2/3 derivative transpose (LHS^T solve,
@@ -571,13 +571,15 @@ int choose_rpb(int d, int N, int Np, int nR, int nTypes, int Wp)
     return psweep_smem_bytes(d == 0, Np, P, nTypes, Wp, 1) <= kMaxSmem ? kRPB : 0;
 }
 
-// Whether k_lsweep takes lines of N rows and band nR, LL lines to a tile.
+// Whether k_lsweep takes lines of N rows and band nR, LL lines to a tile ...
 bool line_fits(bool xd, int N, int nR, int LL)
 {
     const int P = (N + kLineRows - 1) / kLineRows;
-    return nR >= 2 && nR <= kMaxNRreg && P * LL <= line_max_threads(nR) &&
+    return nR >= 2 && nR <= kMaxNRreg && N <= line_max_rows(nR) && P * LL <= line_bound(nR, LL) &&
            line_smem_bytes(xd, N, P, LL, 1, 0, 0, false) <= kMaxSmem;
 }
+// ... or at all (tiles of 4 lines take the longest).
+bool line_takes(bool xd, int N, int nR) { return line_fits(xd, N, nR, 8) || line_fits(xd, N, nR, 4); }
 
 size_t sweep_smem(int N, int P, int nR, int Wp, bool stage = true)
 {
@@ -3134,7 +3136,7 @@ int autotune(gatt_ctx *c, int reps, int *family, int *blocks, double *us)
             if (d >= ndir || !m.set || m.N < 2) continue;
             TuneCand best{m.family, m.rpb, m.P};
             float best_ms = -1.0f;
-            if (!m.lQ && line_fits(d == 0, m.N, m.nR, 8)) rc = upload_line_records(c, m);
+            if (!m.lQ && line_takes(d == 0, m.N, m.nR)) rc = upload_line_records(c, m);
             if (rc != GATT_OK) break;
             for (const TuneCand &t : tune_candidates(m)) {
                 m.family = t.family; m.rpb = t.rpb;
@@ -3424,7 +3426,7 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     int Np = padded_rows(c, d, N, nRHS, periodic);
     int rpb = choose_rpb(d, N, Np, nRHS, nTypes, (W + 3) / 4 * 4);
     const int want = choose_family();
-    const bool line = (want == FAM_LINE || (want == FAM_PIPE && !rpb)) && line_fits(d == 0, N, nRHS, 8) &&
+    const bool line = (want == FAM_LINE || (want == FAM_PIPE && !rpb)) && line_takes(d == 0, N, nRHS) &&
                       line_tiles(c, d, 4) * 16 * c->nb <= INT_MAX / 2;
     const int Npipe = rpb ? Np : N;  // a padded length the pipelined solver does not take is not kept
     if (line) { rpb = 0; Np = N; }  // (its records are its own; the others are the shared-tile solver's)
@@ -3440,7 +3442,7 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     if (!line) TRY(upload_records(c, m, P, rpb ? Np : N));
     else TRY(sync_stream(c));
     // (2-D: also for the chained step's sweeps)
-    if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_fits(d == 0, N, nRHS, 8))) TRY(upload_line_records(c, m));
+    if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_takes(d == 0, N, nRHS))) TRY(upload_line_records(c, m));
     // z lines that only the global-memory solver takes: a scratch field for the third stream, where
     // there is room
     if (d == 2 && (nRHS < 2 || nRHS > kMaxNR || sweep_smem(N, 1, nRHS, m.Wp, false) > kMaxSmem)) {

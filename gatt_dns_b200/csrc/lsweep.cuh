@@ -34,11 +34,15 @@ namespace gatt {
 constexpr int kLineRows = 16;  // rows a thread holds
 constexpr int kLineQ = 6;      // doubles of a compact row record: (fA, fB), (bC, pi), (D, rho)
 
-// Threads a CTA may have: bands of 6 and 7 take up to 128 registers a thread, the others 80.
-__host__ __device__ constexpr int line_max_threads(int nR) { return nR >= 6 ? 512 : 768; }
-// Launch bound of an instantiation: tiles narrower than 32 lines get 96 registers (their CTAs are
-// small; at 80 the solve spills).
+// Threads a CTA may have, the launch bound of an instantiation: 512 for bands of 6 and 7 (128
+// registers a thread), else 768 for tiles of 32 lines (80 registers) and 640 for narrower ones, whose
+// CTAs are small (96).  Spills (bytes stored / loaded, -Xptxas -v): bands of 2 and 3 at most 80/44;
+// band 4, that of the walled fourth-order schemes, the most: 16/16 to 104/100 in tiles of up to 16
+// lines, 116/112 in the x+y sweep of walled lines (156/156 at most), 136/116 to 228/136 with 32 lines
+// and 376/260 to 440/312 in the x+y sweep of 32; band 5 at most 52/52, 212/148 in that sweep.
 __host__ __device__ constexpr int line_bound(int nR, int LL) { return nR >= 6 ? 512 : LL == 32 ? 768 : 640; }
+// Longest line: 96 blocks, 64 for bands of 6 and 7; over 80 blocks tiles of 4 lines only.
+__host__ __device__ constexpr int line_max_rows(int nR) { return nR >= 6 ? 1024 : 1536; }
 
 // Pitch of an x line in shared memory (doubles).
 __host__ __device__ __forceinline__ int line_pitch(int N, int LL)
