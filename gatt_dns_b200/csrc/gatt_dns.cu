@@ -87,6 +87,8 @@ struct DevDir {
     int *lB = nullptr;
     int lP = 0, nspecial = 0;
     double lband[16] = {};
+    bool chainable = false;  // 2-D steps may run it on the any-length solver (chained_2d)
+    bool tuned = false;      // family is gatt_autotune's choice: no rule of size overrides it
 };
 
 struct HostBC {
@@ -1011,8 +1013,8 @@ int sweep(gatt_ctx *c, int d, int kind, const double *in, long long in_bs, const
     // lines of many blocks whose 32-line tiles leave SMs idle (the 300-point y lines of the 800x300
     // grid: 100 tiles of 19 blocks, 13.3 us against 15.3) run as 8-line tiles too
     // (decided by the grid alone: a batch member's arithmetic is that of the member alone; a chain
-    // takes no other solver)
-    const bool few = m.family == FAM_PIPE && m.lQ && m.P >= 16 && (long long)a.ntiles * (c->is3d ? 5 : 4) < c->nsm;
+    // takes no other solver, a tuned set the one that was measured fastest)
+    const bool few = m.family == FAM_PIPE && m.lQ && !m.tuned && m.P >= 16 && (long long)a.ntiles * (c->is3d ? 5 : 4) < c->nsm;
     if (m.family == FAM_LINE || (few && !mc_ref) || (c->chain && m.lQ)) {
         const int r = launch_lsweep(c, m, d, a, nf, nmembers, cls);
         if (r != GATT_ERR_STATE || m.family == FAM_LINE) return r;  // GATT_ERR_STATE: no plan for this launch
@@ -1149,15 +1151,16 @@ XyPlan xy_plan(const gatt_ctx *c, int nf, int nmem, int LL)
 
 // Whether the context's 2-D steps take that launch (and the whole step the chained form):
 // decided by the grid alone, as a batch member's arithmetic must be that of the member alone.
-// Both directions' tiles of one member fit in one round, and neither direction leaves more than
+// Not where GATT_SWEEP asks for another solver; gatt_autotune's choices are for sweeps that are
+// launched by themselves.  Both directions' tiles of one member fit in one round, and neither direction leaves more than
 // a third of the CTA idle (the 800x300 grid: 13 warps of x beside 5 of y would).  On the 128^2
 // cavity a stage is so five launches in a row instead of seven on two streams.
 bool chained_2d(const gatt_ctx *c)
 {
     const DevDir &mx = c->mat[0][0], &my = c->mat[1][0];
-    if (c->is3d || !mx.lQ || !my.lQ || mx.nR != my.nR) return false;
+    if (c->is3d || !mx.chainable || !my.chainable || mx.nR != my.nR) return false;
     for (int d = 0; d < 2; d++)
-        if (c->filt[d] && !c->mat[d][1].lQ) return false;
+        if (c->filt[d] && !c->mat[d][1].chainable) return false;
     if (3 * mx.lP < 2 * my.lP || 3 * my.lP < 2 * mx.lP) return false;
     const XyPlan p = xy_plan(c, 4, 1, 8);
     return p.kernel && p.x.jobs + p.y.jobs <= (long long)p.per_sm * c->nsm;
@@ -3136,6 +3139,7 @@ int autotune(gatt_ctx *c, int reps, int *family, int *blocks, double *us)
             if (d >= ndir || !m.set || m.N < 2) continue;
             TuneCand best{m.family, m.rpb, m.P};
             float best_ms = -1.0f;
+            m.tuned = true;  // every candidate runs on its own solver
             if (!m.lQ && line_takes(d == 0, m.N, m.nR)) rc = upload_line_records(c, m);
             if (rc != GATT_OK) break;
             for (const TuneCand &t : tune_candidates(m)) {
@@ -3442,7 +3446,10 @@ int gatt_set_matrices(gatt_ctx *c, int dir, int kind, int periodic, int nRHS, in
     if (!line) TRY(upload_records(c, m, P, rpb ? Np : N));
     else TRY(sync_stream(c));
     // (2-D: also for the chained step's sweeps)
-    if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_takes(d == 0, N, nRHS))) TRY(upload_line_records(c, m));
+    if (line || (rpb && want != FAM_REG && (P >= 16 || (!c->is3d && kind < 2)) && line_takes(d == 0, N, nRHS))) {
+        TRY(upload_line_records(c, m));
+        m.chainable = !c->is3d && kind < 2;
+    }
     // z lines that only the global-memory solver takes: a scratch field for the third stream, where
     // there is room
     if (d == 2 && (nRHS < 2 || nRHS > kMaxNR || sweep_smem(N, 1, nRHS, m.Wp, false) > kMaxSmem)) {

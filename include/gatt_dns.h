@@ -241,8 +241,10 @@ int gatt_vjp(gatt_ctx *ctx, int nsteps, double t0, double dt, int checkpoint_eve
  * 32 and 64 rows per block -- over `reps` launches of one sweep of 5 (3-D) or 4 (2-D) scratch fields,
  * and keeps the fastest.  Per set (index dir*6 + kind, dir 0..2, kind 0..5), family[] gets
  * 0 shared tile, 1 register (either), 2 TMA-fed register (-1: no matrices), blocks[] the row-block
- * count and us[] the mean microseconds of one launch; any of them may be NULL.  Overwrites
- * the derivative scratch; call it after the matrices and before the first step. */
+ * count and us[] the mean microseconds of one launch; any of them may be NULL.  The choices
+ * hold for sweeps that are launched by themselves: the time steps of small 2-D grids run the
+ * x and y sweeps in one launch of the any-length solver, tuned or not.  Overwrites the
+ * derivative scratch; call it after the matrices and before the first step. */
 int gatt_autotune(gatt_ctx *ctx, int reps, int *family, int *blocks, double *us);
 
 /* Self-test of the pipelined line solver's failure path (no counterpart in the reference):
