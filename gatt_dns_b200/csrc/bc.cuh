@@ -11,9 +11,10 @@
 // field point that they write, or writes one that they read), so the ops of one level are
 // independent whatever their order, and every op finds the values that the reference's order
 // gives it.  The points of a level's ops form one index range spread over all threads; a
-// barrier separates the levels.  One CTA per batch member runs small programs (block barriers),
-// a cluster of up to 16 SMs larger ones (cluster barriers, release/acquire); the widest take one
-// launch per level over the whole GPU.
+// barrier separates the levels.  Programs of up to 16 levels take one launch per level over the whole
+// GPU (k_bc_level).  Deeper ones, the tangent, the recording and the adjoint run in one launch: one CTA
+// per batch member (block barriers) where levels are small, else a cluster of up to 16 SMs (cluster
+// barriers, release/acquire).
 //
 // What bounds it: the chain of levels, about a microsecond each (a barrier, then dependent
 // loads that miss to L2).  The pressure Neumann items and the corners are therefore one op

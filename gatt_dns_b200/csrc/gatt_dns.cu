@@ -56,7 +56,7 @@ int fail(int code, const std::string &msg)
         if (r_ != GATT_OK) return r_; \
     } while (0)
 
-// Line-solve kernel families: shared-memory tile (any N), register-resident rows loaded
+// Line-solve kernel families: shared-memory tile (any N and band), register-resident rows loaded
 // from global memory, register-resident rows fed by a TMA ring (persistent CTAs),
 // register-resident rows of lines of any length (up to line_max_rows) through asynchronous copies.
 enum SweepFamily { FAM_TILE = 0, FAM_REG = 1, FAM_PIPE = 2, FAM_LINE = 3 };
@@ -927,7 +927,10 @@ LinePlan line_plan_for(const gatt_ctx *c, const DevDir &m, int d, int nf, int nm
 // (y lines of the 90x75x54 box: 15.4 us against 18.5 with 16 and 20.8 with 8), fewer for launches
 // that would leave SMs idle, and 8 for lines of 20 blocks and more, whose wide CTAs hold an SM
 // alone (400-point x lines of the plate boundary layer: 118 us against 137 with 16).  4 where
-// 8-line tiles just miss one round (800-point x lines, 152 tiles on 148 SMs: 21.7 us against 28.9).
+// 8-line tiles just miss one round: lines of 500, 650, 800 and 1000 points, 250 to 1100 of them, take
+// up to 2 us less there (650-point x lines, 156 and 200 tiles: 14.7 us against 16.7) and up to 6 us
+// more elsewhere (1000-point y lines, 400 tiles: 33.1 against 29.0); the choice was never more than
+// 1 us, the timer's step, above the better of the two.
 int line_lanes(const gatt_ctx *c, const DevDir &m, int d)
 {
     const char *e = getenv("GATT_LINES");  // 4, 8, 16 or 32 lines a tile, where they fit
@@ -1973,7 +1976,7 @@ int build_bc_program(gatt_ctx *c)
     return GATT_OK;
 }
 
-// The program (form 0 or 1 of d_prog) as the kernels take it, at time t + tfac dt of the step
+// The program (form 0, 1 or 2 of d_prog) as the kernels take it, at time t + tfac dt of the step
 // parameters on the device
 BcProgram bc_program(const gatt_ctx *c, double tfac, int form = 0)
 {

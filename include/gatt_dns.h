@@ -267,8 +267,8 @@ long long gatt_kernel_launches(gatt_ctx *ctx);
 /* Profiling hook (no counterpart in the reference): runs nsteps uncaptured steps with a
  * CUDA event pair around every kernel launch and returns, per kernel class, the mean
  * device time of one launch in ms[GATT_NPROF] and the launches per step in
- * launches[GATT_NPROF].  Advances the state like gatt_run.  gatt_profile_name(i) names
- * class i. */
+ * launches[GATT_NPROF].  The combined x+y sweeps of small 2-D steps count as x sweeps.
+ * Advances the state like gatt_run.  gatt_profile_name(i) names class i. */
 #define GATT_NPROF 17
 int gatt_profile_kernels(gatt_ctx *ctx, double t0, double dt, int nsteps, double *ms, double *launches);
 const char *gatt_profile_name(int cls);
