@@ -2266,10 +2266,11 @@ int ensure_hist(gatt_ctx *c, int n)
     cudaFree(c->hist);
     cudaFreeHost(c->h_params);
     c->hist = nullptr; c->h_params = nullptr;
+    c->hist_cap = 0;       // (until both are there)
+    invalidate_graphs(c);  // graphs hold the history pointer
     TRY(dev_alloc(c, &c->hist, sizeof(double) * 5 * c->nb * (size_t)cap));
     CU(cudaMallocHost(&c->h_params, sizeof(StepParams) * (size_t)cap));
     c->hist_cap = cap;
-    invalidate_graphs(c);  // graphs hold the history pointer
     return GATT_OK;
 }
 

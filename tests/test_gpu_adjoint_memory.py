@@ -101,3 +101,29 @@ def test_z_lines_through_global_memory(cuda_lib, oracle_lib, monkeypatch):
         got, want = g.nseq(f), Oracle(c).nseq(f)
     for k in KEYS:
         assert np.max(np.abs(got[k] - want[k])) < 1e-12 * np.max(np.abs(want[k])), k
+
+
+def test_history_that_does_not_fit(cuda_lib):
+    """A run whose row-a-step history does not fit is refused, and the next one starts from no history."""
+    import torch
+    from gatt_dns_b200 import _lib
+    from gatt_dns_b200.solver import GattDNS
+    c = cs.lid_driven(n=32)
+    f = cs.random_flow(c, seed=5, amp=0.02)
+    dt = 0.25 * c.cfl_dt(f["U"], f["V"], f["W"], 1.0)
+    torch.zeros(1, device="cuda")
+    with GattDNS(c) as g:
+        g.upload(f)
+        want = g.run(3, 0.0, dt)
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        other = torch.empty(free - (256 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            with pytest.raises(_lib.GattError) as e:
+                g.run(1 << 23, 0.0, dt)  # 336 MB of history
+            assert e.value.code == 7     # GATT_ERR_NOMEM
+            g.upload(f)
+            assert np.array_equal(g.run(3, 0.0, dt), want)
+        finally:
+            del other
+            torch.cuda.empty_cache()
